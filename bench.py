@@ -249,16 +249,22 @@ def gemm_peak_tflops(torch, dev, dtype, tf32=False):
     return 2.0 * N ** 3 / best / 1e12
 
 
-def response_flops(case, shape, mixed):
+def response_flops(case, shape, mixed, phases=False):
     """Algorithmic FLOPs of one solve on the block-response path, per launch
     kind.  shape = (B, K, NP, blocks) from the plan.  The aggregate GEMM
     costs 2 NP K per block; the output GEMM 2 B p (K + NP) per block (window
     part 2 B p K, initial-state part 2 B p NP); the carry over blocks 4 NP^2
     per block (up- and down-sweep).  The dominant launch is the output GEMM
-    in FP64 and, in the mixed form, the tensor-core launch that computes the
-    aggregates and the output windows together."""
+    in FP64 and, in the mixed form with sampled inputs, the tensor-core launch
+    that computes the aggregates and the output windows together.  With phases
+    (the mixed form of sinusoid inputs: K phase columns, kernels_expand.cu) the
+    states cost 2 NP (NP + K) per block and the outputs 2 B p (NP + K), all in
+    FP64, and there are no aggregates and no carry."""
     B, K, NP, blocks = shape
     p = case.p
+    if phases:
+        out, states = 2.0 * B * p * (NP + K) * blocks, 2.0 * NP * (NP + K) * blocks
+        return {"dominant": out, "solve": out + states}
     agg, win, state, carry = 2.0 * NP * K * blocks, 2.0 * B * p * K * blocks, 2.0 * B * p * NP * blocks, \
         4.0 * NP * NP * blocks
     dominant = (agg + win) if mixed else (win + state)
@@ -785,11 +791,13 @@ def run_ours(args):
     if rank == 0:
         peaks, peaks_kind = measured_peaks()
         used_mixed = main["precision_used"] == pb.MIXED
-        fl = response_flops(case, main["response_shape"], used_mixed) if main["path"] == 3 else None
-        stage = "aggregates+windows" if used_mixed else "outputs"
+        phases = "states" in main["stages_ms"]  # sinusoid inputs as phases: all FP64
+        on_tc = used_mixed and not phases
+        fl = response_flops(case, main["response_shape"], used_mixed, phases) if main["path"] == 3 else None
+        stage = "aggregates+windows" if on_tc else "outputs"
         dom_ms = main["stages_ms"].get(stage)
         tf32_run = None
-        if used_mixed:
+        if on_tc:
             # dense TF32 is half the bf16 rate; 3xTF32 spends three tensor
             # products per algorithmic product
             peak = peaks["bf16_tflops"] / 2.0 / 3.0
@@ -803,11 +811,12 @@ def run_ours(args):
         achieved = fl["dominant"] / (dom_ms / 1e3) / 1e12 if (fl and dom_ms) else None
         roofline = {"bound": "tensor",
                     "kernel": ("k_resp_tc: 3xTF32 tcgen05 GEMMs of the block aggregates and output windows"
-                               if used_mixed else "k_level_tiled: FP64 DMMA output GEMM y = W [window; X_b]"),
+                               if on_tc else "k_expand_out: FP64 DMMA outputs y = W [X_b; phases of b]" if phases
+                               else "k_level_tiled: FP64 DMMA output GEMM y = W [window; X_b]"),
                     "stage": stage, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                     "frac": (achieved / peak) if achieved else None, "peak_source": peak_src,
                     "algorithmic_flops_per_launch": fl["dominant"] if fl else None,
-                    "traffic": DOMINANT_TRAFFIC.get((case.T, used_mixed)),
+                    "traffic": None if phases else DOMINANT_TRAFFIC.get((case.T, used_mixed)),
                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch (profiles/)",
                     "stages_ms": main["stages_ms"],
                     "whole_solve_tflops": fl["solve"] / (main["ms_per_step"] / 1e3) / 1e12 if fl else None}
@@ -830,7 +839,7 @@ def run_ours(args):
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": main["ms_per_step"], "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,
-            "dtype": "tf32x3+f64" if used_mixed else "f64", "data": "synthetic (seeded system and input)",
+            "dtype": "tf32x3+f64" if on_tc else "f64", "data": "synthetic (seeded system and input)",
             "config": bench_config(args, world),
             "precision_used": "mixed" if used_mixed else "fp64",
             "path": {1: "level-synchronous", 2: "blocked, in-block sweeps",

@@ -200,7 +200,13 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
             throw Error(kInvalidArgument, "the blocked path supports scan dimensions up to 64");
         if (opt.path != kPathLevel && can_block) path_ = kPathBlocked;
     }
-    if (path_ == kPathBlocked) {
+    if (path_ == kPathBlocked && choose_expand(opt)) {
+        Np_ = ext_.sh.NP;
+        shape_.R = ext_.sh.R;
+        shape_.B = ext_.sh.B;
+        nblocks_ = ext_.sh.nblocks;
+        levels_ = 1;  // only Phi itself: the expansion has its own powers
+    } else if (path_ == kPathBlocked) {
         Np_ = shape_.NP;
         ntiles_ = (nScan_ + shape_.S - 1) / shape_.S;
         nblocks_ = ntiles_ * (shape_.S / shape_.B);
@@ -314,6 +320,7 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
     // (each cudaMallocAsync costs a few microseconds even from a warm pool)
     std::vector<std::pair<double**, long>> want;
     double* st = nullptr;
+    double* dPar = nullptr;  // expansion: the input's amplitudes, angular frequencies, phases
     long npow = std::max(levels_, 1);
     want.emplace_back(&dPow_, npow * (long)Np_ * Np_);
     want.emplace_back(&dBbar_, (long)n * W * std::max(mB, 1));
@@ -346,6 +353,14 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
             want.emplace_back(&dMs_, nScan_ * (long)Np_ * Np_);
             want.emplace_back(&dXs_, nScan_ * (long)Np_);
         }
+    } else if (ex_) {
+        const ExpandShape& e = ext_.sh;
+        want.emplace_back(&ext_.E, (long)e.pow_levels * e.NP * e.Kc);
+        want.emplace_back(&ext_.T, std::max(1L, e.table_rows() * e.Kc));
+        want.emplace_back(&ext_.W, (long)e.rows() * e.Kc);
+        want.emplace_back(&dPar, std::max(1L, 3L * e.H / 2));
+        want.emplace_back(&dZ_, e.nblocks * e.Kc);
+        want.emplace_back(&dCext_, (long)p_ * Np_);
     } else {
         want.emplace_back(&dG_, nblocks_ * (long)Np_);
         want.emplace_back(&dWork_, std::max(blocked_items_scratch(shape_, nblocks_),
@@ -375,15 +390,16 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
     }
     // the response leaf reads whole windows: the last block's window runs
     // past the samples into a zero padding
-    const long pad = (mu_ > 0 && !gen_ && br_) ? (2L * shape_.B + 8) * mu_ + 2 : 0;
+    const bool sampled = mu_ > 0 && !gen_ && !ex_;
+    const long pad = (sampled && br_) ? (2L * shape_.B + 8) * mu_ + 2 : 0;
     // the mixed response GEMMs read the samples as TF32 planes (their TMA
     // boxes run up to 15 samples past a window); FP64 samples are then only
     // the scratch a user input function fills before the split
-    const bool planes = mu_ > 0 && !gen_ && br_tc_;
+    const bool planes = sampled && br_tc_;
     const long nf = nU_ * (long)mu_ + pad + 16;
     double* dh = nullptr;
     double* dl = nullptr;
-    if (mu_ > 0 && !gen_) {
+    if (sampled) {
         if (!planes || input_->kind != InputEntry::kSinusoid) want.emplace_back(&dU_, nU_ * (long)mu_ + pad);
         if (planes) {
             want.emplace_back(&dh, (nf + 1) / 2);
@@ -409,7 +425,7 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         h2d(dCext_, Cext.data(), sizeof(double) * Cext.size());
     }
     phase("output rows", false);
-    if (mu_ > 0 && !gen_) {
+    if (sampled) {
         // every execute writes all nU x mu samples: only the padding is zeroed
         if (dU_ && pad) PARODE_CUDA(cudaMemsetAsync(dU_ + nU_ * mu_, 0, sizeof(double) * (size_t)pad, stream_));
         const size_t used = (size_t)nU_ * mu_;  // rewritten by every execute
@@ -511,6 +527,33 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
     }
     h2d(dX0_, X0.data(), sizeof(double) * Np_);
     phase("copies+start-up", true);
+    if (ex_) {
+        ext_.solver = solver;
+        ext_.n = n;
+        ext_.mu = mu_;
+        ext_.terms = mu_ > 0 ? input_->K : 0;
+        ext_.zeroB = sys.zeroB || mu_ == 0;
+        ext_.zeroD = sys.zeroD || mu_ == 0;
+        ext_.dt = u_dt_;
+        ext_.Phi = dPow_;
+        ext_.Bbar = dBbar_;
+        ext_.Cext = dCext_;
+        ext_.D = dD_;
+        ext_.par = dPar;
+        if (mu_ > 0) {
+            // the parameters of the system's channels, the angular frequency rounded as the samplers round it
+            const size_t q = (size_t)mu_ * input_->K;
+            std::vector<double> par(3 * q);
+            for (size_t k = 0; k < q; ++k) {
+                par[k] = input_->a[k];
+                par[q + k] = 6.283185307179586476925286766559 * input_->f[k];
+                par[2 * q + k] = input_->phi[k];
+            }
+            h2d(dPar, par.data(), sizeof(double) * par.size());
+        }
+        launch_expand_tables(ext_, stream_);
+        phase("expansion tables", true);
+    }
     if (br_) {
         // the carry's powers P_1 .. P_levels (Phi^(2^l)) depend on Phi alone:
         // formed once here, on the side stream beside W (both only read level 0)
@@ -842,11 +885,47 @@ void Plan::response_shape(long long info[4]) const
         batch_->response_shape(0, info);
         return;
     }
+    if (ex_ && mu_ > 0) {
+        info[0] = ext_.sh.B;
+        info[1] = ext_.sh.H;
+        info[2] = ext_.sh.NP;
+        info[3] = ext_.sh.nblocks;
+        return;
+    }
     if (!br_) return;
     info[0] = shape_.B;
     info[1] = brK_;
     info[2] = Np_;
     info[3] = (nScan_ + shape_.B - 1) / shape_.B;
+}
+
+bool Plan::choose_expand(const PlanOptions& opt)
+{
+    // A solve without inputs in any form; with sinusoid inputs in the mixed
+    // and TF32 forms at the scan dimensions those forms cover (their sample
+    // planes took the nominal phase steps that the expansion takes; the FP64
+    // form samples at the rounded times and keeps its samples).  User input
+    // functions, time shards and the fault hook of the tensor-core kernel
+    // take the sample windows.  An input with too few channels is refused
+    // where the samples are filled, as before.
+    // A path forced to either leaf of kernels_br.cu / the in-block sweeps takes
+    // that leaf.
+    if ((opt.path != kPathAuto && opt.path != kPathBlocked) || opt.shards > 1 || opt.shard != 0 || opt.fault_withhold)
+        return false;
+    const bool free_response = mu_ == 0;
+    const bool phases = mu_ > 0 && opt.precision != kFP64 && Ns_ > 8 && input_->kind == InputEntry::kSinusoid &&
+                        input_->m >= mu_;
+    if (!free_response && !phases) return false;
+    // Long blocks cost only table rows; 64 steps leave enough blocks to fill
+    // the chip from 4096 steps on.  A forced or measured length wins.
+    int R = phases ? opt.force_log2_block : 0;
+    if (R < 2 && phases) R = tuned_log2_block(tune_class(solver_, Ns_, mu_, p_, nScan_, opt.precision));
+    if (R < 2 || R > 7) R = nScan_ >= 4096 ? 6 : 4;
+    while (R > 2 && (1L << R) / 2 >= nScan_) --R;
+    if (!expand_shape(Ns_, mu_, mu_ > 0 ? input_->K : 0, p_, nScan_, R, &ext_.sh)) return false;
+    ex_ = true;
+    if (opt.precision != kFP64 && Ns_ > 8) precision_used_ = phases && opt.precision == kTF32 ? kTF32 : kMixed;
+    return true;
 }
 
 void Plan::execute_body(double* y, cudaStream_t s)
@@ -1079,6 +1158,11 @@ int Plan::response_head(cudaStream_t s)
     int launches = 0;
     marks_.clear();
     mark("start", s);
+    if (ex_) {
+        launches = launch_expand_states(ext_, dX0_, dZ_, u_base_, (solver_ == kRK4 ? 2L : 1L) * shape_.B, s);
+        mark("states", s);
+        return launches;
+    }
     fill_inputs(s);
     ++launches;
     mark("inputs", s);
@@ -1105,6 +1189,10 @@ void Plan::response_outputs(double* Y, long c0, long c1, cudaStream_t s)
 {
     // the outputs of blocks [c0, c1) with their carried states, written
     // straight into y (rows (j, o) of block b are contiguous there)
+    if (ex_) {
+        launch_expand_out(ext_, dZ_, Y + (solver_ == kRK4 ? 0L : 3L * p_), c0, c1, nScan_ * (long)p_, sms_, s);
+        return;
+    }
     if (br_tc_) {
         state_part(Y, c0, c1, s);  // y = windows + C Phi^j X_b (FP64)
         return;
@@ -1133,7 +1221,7 @@ void Plan::execute_response(double* Y, cudaStream_t s)
 void Plan::solve_to_host(double* yd, float* yf)
 {
     void* y = yf ? (void*)yf : (void*)yd;
-    if (!y || batch_ || shards_ > 1 || path_ != kPathBlocked || !br_ || profiling_ || nblocks_ < 8) {
+    if (!y || batch_ || shards_ > 1 || path_ != kPathBlocked || !(br_ || ex_) || profiling_ || nblocks_ < 8) {
         execute(nullptr, nullptr);
         if (yf)
             get_output_f32(nullptr, yf);
@@ -1290,7 +1378,7 @@ void Plan::shard_down(const double* dGathered, double* Y, cudaStream_t s)
 
 void Plan::execute_blocked(double* Y, cudaStream_t s)
 {
-    if (br_) {
+    if (br_ || ex_) {
         execute_response(Y, s);
         return;
     }

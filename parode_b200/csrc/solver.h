@@ -7,6 +7,7 @@
 #pragma once
 
 #include "blocked.h"
+#include "expand.h"
 #include "host_math.h"
 #include "inputs.h"
 #include "kernels.h"
@@ -98,10 +99,11 @@ public:
     int device() const { return device_; }
     cudaStream_t stream() const { return stream_; }
     const double* device_output() const;
-    // kPathLevel, kPathBlocked (in-block sweep leaf) or kPathBlockedResponse
-    int path() const { return br_ ? (int)kPathBlockedResponse : path_; }
-    // Response leaf: block length, window columns, padded scan dimension,
-    // blocks (zeros when not that path)
+    // kPathLevel, kPathBlocked (in-block sweep leaf, or the expansion of a free
+    // response) or kPathBlockedResponse (sample windows or sinusoid phases)
+    int path() const { return br_ || (ex_ && mu_ > 0) ? (int)kPathBlockedResponse : path_; }
+    // Response leaf: block length, window (or phase) columns, padded scan
+    // dimension, blocks (zeros when not that path)
     void response_shape(long long info[4]) const;
     int precision_used() const { return precision_used_; }
 
@@ -133,6 +135,7 @@ private:
     void execute_blocked(double* Y, cudaStream_t s);
     void execute_response(double* Y, cudaStream_t s);
     void execute_general(double* Y, cudaStream_t s);
+    bool choose_expand(const PlanOptions& opt);
     int carry(cudaStream_t s);
     LevelArgs response_agg_args() const;
     LevelArgs response_out_args(double* Y) const;
@@ -170,6 +173,11 @@ private:
     bool br_ = false;           // leaf = block response GEMM (kernels_br.cu)
     int brK_ = 0, brKpad_ = 0;  // window columns (padded to even)
     double* dW_ = nullptr;      // response matrix, (B p + NP) x (brKpad_ + NP)
+    // block states by radix expansion (kernels_expand.cu): no inputs, or
+    // sinusoid inputs in the mixed and TF32 forms
+    bool ex_ = false;
+    ExpandTables ext_;
+    double* dZ_ = nullptr;      // augmented block states, nblocks x Kc
     double* dMs_ = nullptr;     // general path: T copies of Phi (Ns x Ns each)
     double* dXs_ = nullptr;     // general path: the states x_k (T x Ns)
     // mixed form of the response leaf: aggregates and output windows on the
