@@ -21,6 +21,7 @@ namespace {
 constexpr size_t kAlign = 256;
 constexpr size_t kSmemOptIn = 232448 - 1024;
 constexpr int kTcConfig = 100;  // grouped launch of the tensor-core (3xTF32) level contraction
+constexpr int kNarrowConfig = 101;  // grouped launch of k_expand_narrow
 
 size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
 
@@ -206,6 +207,60 @@ BatchPlan::BatchPlan(int device, std::vector<BatchSpec> specs, InputRegistry* in
     }
 }
 
+bool BatchPlan::choose_expand(Sys& q, const PlanOptions& opt)
+{
+    // No inputs (any form), or sinusoid inputs in the mixed form, whatever
+    // their term count up to the width the kernels take: the samplers' cost
+    // grows with the terms too.  Measured, one mixed system against the sample
+    // windows: RK4 n = 96, m = p = 12, 60,000 steps 0.060 against 0.308 ms with
+    // 3 terms a channel, 0.181 against 0.869 with 40 (960 phase columns); ABM
+    // n = 64, m = p = 8, 0.071 against 0.418 and 0.127 against 0.889.  A forced
+    // path keeps its leaf.  (A single plan's rule is Plan::choose_expand; scan
+    // dimensions above 64 and wide inputs come here.)
+    if (opt.path != kPathAuto && opt.path != kPathBlocked) return false;
+    const bool phases = q.mu > 0 && opt.precision == kMixed && q.input->kind == InputEntry::kSinusoid;
+    if (q.mu > 0 && !phases) return false;
+    const int np = (int)round_up(q.Ns, 8);
+    const long hq = phases ? (long)q.mu * q.input->K : 0;
+    if (np > 1024 || hq > kExpandMaxPairs) return false;
+    const int kc = (int)round_up(np + 2 * hq, 8);
+    int R = expand_log2_block(np, kc, q.p, q.nScan, opt.executions);
+    if (phases) {
+        int Rt = opt.force_log2_block;
+        if (Rt < 2) Rt = tuned_log2_block(tune_class(q.solver, q.Ns, q.mu, q.p, q.nScan, opt.precision));
+        if (Rt >= 2 && Rt <= 7) {
+            while (Rt > 2 && (1L << Rt) / 2 >= q.nScan) --Rt;
+            R = Rt;
+        }
+    }
+    q.ex = true;
+    q.Np = np;
+    q.K = phases ? q.input->K : 0;
+    q.lev0 = R;
+    q.Bk = 1 << R;
+    q.nblocks = (q.nScan + q.Bk - 1) / q.Bk;
+    q.levels = ilog2(next_pow2(q.nblocks));
+    q.pow_levels = std::max(1, q.levels > 0 ? R + q.levels : R);
+    ExpandJob& j = q.exj;
+    j.solver = q.solver;
+    j.n = q.n;
+    j.mu = q.mu;
+    j.terms = q.K;
+    j.p = q.p;
+    j.NP = np;
+    j.H = (int)(2 * hq);
+    j.Kc = kc;
+    j.R = R;
+    j.pow_levels = q.pow_levels;
+    j.zeroB = q.zeroB || q.mu == 0;
+    j.zeroD = q.zeroD || q.mu == 0;
+    j.nblocks = q.nblocks;
+    j.stride = (q.solver == kRK4 ? 2L : 1L) * q.Bk;
+    j.base = q.u_base;
+    j.dt = q.u_dt;
+    return true;
+}
+
 void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const PlanOptions& opt)
 {
     if (specs.empty()) throw Error(kInvalidArgument, "empty batch");
@@ -274,6 +329,11 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         }
         BlockedShape sh;
         const bool can_block = blocked_shape(q.Ns, std::max(q.mu, 1), 0, &sh);
+        if (choose_expand(q, opt)) {
+            ex_.push_back(i);
+            q.precision = (opt.precision == kMixed && (q.mu > 0 || !can_block)) ? kMixed : kFP64;
+            continue;
+        }
         // block-response leaf for systems with inputs when it costs less than
         // the level-synchronous sweeps (4 Np^2 per step) or, for scan
         // dimensions <= 64, half the in-block sweeps
@@ -407,7 +467,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             const int mB = specs[i].sys.zeroB ? 0 : q.m;
             doff[i].phi = D.take(sizeof(double) * (size_t)q.n * q.Ns);
             doff[i].bbar = D.take(sizeof(double) * (size_t)q.n * q.W * std::max(mB, 1));
-            doff[i].bbarT = (!q.blocked && !q.resp) ? D.take(sizeof(double) * (size_t)std::max(q.W * mB, 1) * q.n) : 0;
+            doff[i].bbarT = q.level_sync() ? D.take(sizeof(double) * (size_t)std::max(q.W * mB, 1) * q.n) : 0;
         }
         if (fault_alloc_now()) throw Error(kNotEnoughResources, "batch discretisation buffer (injected)");
         cudaError_t e = cudaMallocAsync(&disc_, std::max<size_t>(D.bytes, 8), stream_);
@@ -462,7 +522,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             const int mB = s.zeroB ? 0 : s.m;
             doff[i].phi = D.take(sizeof(double) * (size_t)q.n * q.Ns);
             doff[i].bbar = D.take(sizeof(double) * (size_t)q.n * q.W * std::max(mB, 1));
-            doff[i].bbarT = (!q.blocked && !q.resp) ? D.take(sizeof(double) * (size_t)std::max(q.W * mB, 1) * q.n) : 0;
+            doff[i].bbarT = q.level_sync() ? D.take(sizeof(double) * (size_t)std::max(q.W * mB, 1) * q.n) : 0;
             doff[i].work = D.take(sizeof(double) * (size_t)discretise_work_doubles(q.n, mB));
         }
         if (fault_alloc_now()) throw Error(kNotEnoughResources, "batch discretisation buffer (injected)");
@@ -518,7 +578,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
     struct Off {
         size_t c, d, cext, x0, sin, ypre;
         size_t cT, dT;  // level-synchronous systems: transposed copies (coalesced per-row kernels)
-        size_t P, U, Y, V, G, CP, Ps, W, Psa, Psw;
+        size_t P, U, Y, V, G, CP, Ps, W, Psa, Psw, rot;
     };
     std::vector<Off> off(N);
     for (int i = 0; i < N; ++i) {
@@ -528,7 +588,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         o.c = L.take(sizeof(double) * (s.zeroC ? 1 : (size_t)q.p * q.n));
         o.d = L.take(sizeof(double) * (s.zeroD ? 1 : (size_t)q.p * s.m));
         o.x0 = L.take(sizeof(double) * (size_t)q.Np);
-        o.cext = (q.blocked || q.resp) ? L.take(sizeof(double) * (size_t)q.p * q.Np) : 0;
+        o.cext = !q.level_sync() ? L.take(sizeof(double) * (size_t)q.p * q.Np) : 0;
         o.sin = 0;
         if (q.mu > 0 && q.input->kind == InputEntry::kSinusoid) {
             q.K = q.input->K;
@@ -536,7 +596,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         }
         o.ypre = q.solver == kABM ? L.take(sizeof(double) * 3 * (size_t)q.p) : 0;
         o.cT = o.dT = 0;
-        if (!q.blocked && !q.resp) {
+        if (q.level_sync()) {
             o.cT = L.take(sizeof(double) * (size_t)q.n * q.p);
             o.dT = L.take(sizeof(double) * (size_t)std::max(s.m, 1) * q.p);
         }
@@ -557,7 +617,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         std::fill(x0, x0 + q.Np, 0.0);
         if (q.solver == kRK4)
             for (int r = 0; r < q.n; ++r) x0[r] = s.x0[r];  // ABM: the start-up below
-        if (q.blocked || q.resp) {
+        if (!q.level_sync()) {
             double* cext = slot(o.cext);
             std::fill(cext, cext + (size_t)q.p * q.Np, 0.0);
             const int xoff = q.solver == kRK4 ? 0 : 3 * q.n;
@@ -577,7 +637,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             std::memcpy(prm + na, e->f.data(), sizeof(double) * na);
             std::memcpy(prm + 2 * na, e->phi.data(), sizeof(double) * na);
         }
-        if (!q.blocked && !q.resp) {
+        if (q.level_sync()) {
             double* ct = slot(o.cT);
             double* dt = slot(o.dT);
             std::fill(ct, ct + (size_t)q.n * q.p, 0.0);
@@ -659,6 +719,15 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             o.P = L.take(sizeof(double) * (size_t)(bk.sh.R + 1) * q.Np * q.Np);
             o.G = L.take(sizeof(double) * (size_t)q.ntiles * (bk.sh.S / bk.sh.B) * q.Np);
             o.CP = L.take(sizeof(double) * (size_t)bk.sh.B * q.p * q.Np);
+        } else if (q.ex) {
+            const ExpandJob& j = q.exj;
+            o.P = L.take(sizeof(double) * (size_t)q.pow_levels * j.NP * j.Kc);
+            o.V = L.take(sizeof(double) * (size_t)q.nblocks * j.Kc);
+            o.rot = L.take(sizeof(double) * (size_t)q.pow_levels * std::max(j.H, 1));
+            const size_t at1 = L.bytes;
+            o.W = L.take(sizeof(double) * (size_t)q.Bk * q.p * j.Kc);
+            kind_bytes[1] += L.bytes - at1;
+            kind_bytes[0] -= L.bytes - at1;
         } else {
             o.P = L.take(sizeof(double) * (size_t)std::max(q.pow_levels, 1) * q.Np * q.Np);
             o.V = L.take(sizeof(double) * (size_t)(q.Tp + 1) * q.Np);  // slot -1 holds the initial state
@@ -687,7 +756,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         // window runs past the samples into a zero padding
         const size_t upad = q.resp ? (size_t)(2 * q.Bk + 8) * q.mu + 2 : 0;
         const size_t at3 = L.bytes;
-        o.U = q.mu > 0 ? L.take(sizeof(double) * ((size_t)q.nU * q.mu + upad)) : 0;
+        o.U = q.mu > 0 && !q.ex ? L.take(sizeof(double) * ((size_t)q.nU * q.mu + upad)) : 0;
         const size_t at4 = L.bytes;
         o.Y = L.take(sizeof(double) * (size_t)q.nOut * q.p);
         kind_bytes[0] += at3 - at0;
@@ -717,7 +786,8 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         long lev_entries = 0;
         for (int i : ls_) lev_entries += 4L * std::max(sys_[i].levels, 1);
         for (int i : rs_) lev_entries += 4L * std::max(sys_[i].pow_levels, 1) + 8;
-        job_bytes = nb * (sizeof(LeafArgs) + 3 * sizeof(double*) + 4 * kAlign) +
+        for (int i : ex_) lev_entries += 3L * sys_[i].pow_levels + 4;
+        job_bytes = ex_.size() * sizeof(ExpandJob) + nb * (sizeof(LeafArgs) + 3 * sizeof(double*) + 4 * kAlign) +
                     (size_t)items_ub * sizeof(BatchItem) + buckets_.size() * 8 * kAlign +
                     (size_t)N * (sizeof(SampleJob) + sizeof(ForcingJob) + sizeof(OutputJob) + 2 * sizeof(CopyJob) + sizeof(PhiJob)) +
                     8 * kAlign + (size_t)lev_entries * (2 * sizeof(LevelArgs) + sizeof(long) + 128) +
@@ -734,7 +804,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         PARODE_CUDA(cudaDeviceGetDefaultMemPool(&pool, device_));
         uint64_t keep = 0;
         PARODE_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-        uint64_t want = (uint64_t)arena_bytes_ + (rs_.empty() ? 0 : ((uint64_t)5 << 29));
+        uint64_t want = (uint64_t)arena_bytes_ + (rs_.empty() && ex_.empty() ? 0 : ((uint64_t)5 << 29));
         if (keep < want) PARODE_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &want));
     }
     {
@@ -759,8 +829,11 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         q.D = dp(o.d);
         q.X0 = dp(o.x0);
         q.Y = dp(o.Y);
-        q.U = q.mu > 0 ? dp(o.U) : nullptr;
-        if (q.blocked) {
+        q.U = q.mu > 0 && !q.ex ? dp(o.U) : nullptr;
+        if (q.ex) {
+            q.Cext = dp(o.cext);
+            q.Wm = dp(o.W);
+        } else if (q.blocked) {
             q.G = dp(o.G);
             q.CP = dp(o.CP);
             q.Cext = dp(o.cext);
@@ -777,6 +850,23 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             }
         }
         if (q.mu > 0 && q.input->kind == InputEntry::kSinusoid) q.sin = dp(o.sin);
+        if (q.ex) {
+            ExpandJob& j = q.exj;
+            if (q.mu > 0) {
+                const size_t na = q.input->a.size();
+                j.amp = q.sin;
+                j.freq = q.sin + na;
+                j.phi = q.sin + 2 * na;
+            }
+            j.Bbar = q.Bbar;
+            j.Cext = q.Cext;
+            j.D = q.D;
+            j.X0 = q.X0;
+            j.E = q.P;
+            j.W = q.Wm;
+            j.Z = dp(o.V);
+            j.rot = dp(o.rot);
+        }
     }
 
     phase("arena", true);
@@ -858,7 +948,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         std::vector<SampleJob> sj;
         for (int i = 0; i < N; ++i) {
             const Sys& q = sys_[i];
-            if (q.mu <= 0) continue;
+            if (q.mu <= 0 || q.ex) continue;
             if (q.input->kind != InputEntry::kSinusoid) {
                 user_inputs_.push_back(i);
                 continue;
@@ -886,7 +976,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
     // levels; response systems: their GEMMs, seed and block-scan levels
     std::vector<int> lv = ls_;
     lv.insert(lv.end(), rs_.begin(), rs_.end());
-    if (!lv.empty()) {
+    if (!lv.empty() || !ex_.empty()) {
         std::vector<ForcingJob> fj;
         std::vector<OutputJob> oj;
         std::vector<CopyJob> cj;
@@ -1259,6 +1349,79 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             rs_tc_.push_back(make_tc(tcg));
             add_level(rs_state_, state, -1);
         }
+        // radix expansion: the squaring steps (set-up), the doubling levels, the outputs
+        if (!ex_.empty()) {
+            std::vector<ExpandJob> jobs;
+            int lmax = 0;
+            for (int i : ex_) {
+                const Sys& q = sys_[i];
+                const ExpandJob& j = q.exj;
+                const long pairs = (j.Kc - j.NP) / 2;
+                jobs.push_back(j);
+                lmax = std::max(lmax, q.levels);
+                exSteps_ = std::max(exSteps_, std::max(q.pow_levels - 1, j.R));
+                exMaxHq_ = std::max(exMaxHq_, j.H / 2);
+                exMaxInit_ = std::max(exMaxInit_, j.NP * pairs + (long)j.p * j.Kc + (long)q.pow_levels * j.H / 2);
+                exMaxRot_ = std::max(exMaxRot_, (j.NP + ((long)j.p << j.R) / 2) * j.Kc / 2);
+                exMaxFeed_ = std::max(exMaxFeed_, (long)(j.H / 2) << j.R);
+                exMaxPhases_ = std::max(exMaxPhases_, std::max<long>(j.NP, q.nblocks * pairs));
+            }
+            dEx_ = reinterpret_cast<ExpandJob*>(base + jput(jobs.data(), sizeof(ExpandJob) * jobs.size()));
+            for (int l = 0; l < exSteps_; ++l) {
+                ex_power_at_.push_back(ex_power_.size());
+                std::vector<std::pair<int, LevelArgs>> ents;
+                for (int i : ex_) {
+                    LevelArgs two[2];
+                    const int c = expand_power_args(sys_[i].exj, l, two);
+                    for (int k = 0; k < c; ++k) ents.push_back({i, two[k]});
+                }
+                add_level(ex_power_, ents, -1);
+            }
+            ex_power_at_.push_back(ex_power_.size());
+            for (int l = 0; l < lmax; ++l) {
+                // few columns go to the narrow kernel; so do up to 512 when the
+                // level's 64 x 64 tiles would leave SMs idle (one large system,
+                // NP = 512, 64 columns: 8 tiles, 19 us, against 128 narrow CTAs)
+                std::vector<std::pair<int, LevelArgs>> wide;
+                std::vector<LevelArgs> narrow;
+                long tiles = 0;
+                for (int i : ex_) {
+                    if (l >= sys_[i].levels) continue;
+                    const LevelArgs a = expand_level_args(sys_[i].exj, l);
+                    tiles += level_tiles(level_config(a), a);
+                    if (a.ncols <= 32) narrow.push_back(a);
+                    else wide.push_back({i, a});
+                }
+                if (tiles < sms_) {
+                    std::vector<std::pair<int, LevelArgs>> rest;
+                    for (auto& e : wide) {
+                        if (e.second.ncols <= 512) narrow.push_back(e.second);
+                        else rest.push_back(e);
+                    }
+                    wide.swap(rest);
+                }
+                add_level(ex_level_, wide, -1);
+                if (!narrow.empty()) {
+                    GroupedLaunch gl;
+                    gl.cfg.id = kNarrowConfig;
+                    gl.nent = (int)narrow.size();
+                    std::vector<long> start;
+                    for (const LevelArgs& a : narrow) {
+                        start.push_back(gl.tiles);
+                        gl.tiles += expand_narrow_tiles(a);
+                    }
+                    gl.args = reinterpret_cast<LevelArgs*>(base + jput(narrow.data(), sizeof(LevelArgs) * narrow.size()));
+                    gl.start = reinterpret_cast<long*>(base + jput(start.data(), sizeof(long) * start.size()));
+                    ex_level_.push_back(gl);
+                }
+            }
+            std::vector<std::pair<int, LevelArgs>> outs;
+            for (int i : ex_) {
+                const Sys& q = sys_[i];
+                outs.push_back({i, expand_out_args(q.exj, q.Y + (q.solver == kRK4 ? 0L : 3L * q.p), q.nScan * (long)q.p)});
+            }
+            add_level(ex_out_, outs, -1);
+        }
         nZero_ = (int)zero.size();
         if (nZero_ > 0) dZero_ = reinterpret_cast<CopyJob*>(base + jput(zero.data(), sizeof(CopyJob) * zero.size()));
     }
@@ -1315,6 +1478,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         pj.n = q.n;
         pj.Np = q.Np;
         pj.solver = q.solver;
+        pj.ld = q.ex ? q.exj.Kc : 0;
         phi_jobs.push_back(pj);
         max_phi = std::max(max_phi, (long)q.Np * q.Np);
         if (q.solver == kABM) {
@@ -1355,6 +1519,15 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
     // formed here with Phi, once per batch, like the rest of the discretisation
     for (const Bucket& bk : buckets_) launch_batch_stage(0, bk.sh, bk.launch, stream_);
     for (const GroupedLaunch& g : ls_power_) launch_grouped(g, stream_);
+    if (!ex_.empty()) {
+        const int ne = (int)ex_.size();
+        launch_expand_init(dEx_, ne, exMaxHq_, exMaxInit_, stream_);
+        for (int l = 0; l < exSteps_; ++l) {
+            launch_expand_rot(dEx_, ne, l, exMaxRot_, stream_);
+            for (size_t k = ex_power_at_[l]; k < ex_power_at_[l + 1]; ++k) launch_grouped(ex_power_[k], stream_);
+        }
+        launch_expand_feed(dEx_, ne, exMaxFeed_, stream_);
+    }
     phase("power-tables", true);
     build_responses();
     phase("responses", true);
@@ -1378,9 +1551,9 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
     }
     if (opt.log)
         std::fprintf(stderr,
-                     "ParODE batch set-up (%d systems, %zu response, %zu level, %zu buckets, %.2f GB: tables+scan %.2f, "
+                     "ParODE batch set-up (%d systems, %zu expansion, %zu response, %zu level, %zu buckets, %.2f GB: tables+scan %.2f, "
                      "W %.2f, W split %.2f, samples %.2f, outputs %.2f):%s\n",
-                     N, rs_.size(), ls_.size(), buckets_.size(), arena_bytes_ / 1e9, kind_bytes[0] / 1e9,
+                     N, ex_.size(), rs_.size(), ls_.size(), buckets_.size(), arena_bytes_ / 1e9, kind_bytes[0] / 1e9,
                      kind_bytes[1] / 1e9, kind_bytes[2] / 1e9, kind_bytes[3] / 1e9, kind_bytes[4] / 1e9, phases.c_str());
 }
 
@@ -1667,6 +1840,13 @@ void BatchPlan::enqueue(cudaStream_t s)
             ++launches;
         }
     }
+    if (!ex_.empty()) {
+        // on the caller's stream, beside the forked sets
+        launch_expand_phases(dEx_, (int)ex_.size(), exMaxPhases_, s);
+        for (const GroupedLaunch& g : ex_level_) launch_grouped(g, s);
+        for (const GroupedLaunch& g : ex_out_) launch_grouped(g, s);
+        launches += 1 + (int)(ex_level_.size() + ex_out_.size());
+    }
     // join
     for (int k = 0; k < f; ++k) {
         PARODE_CUDA(cudaEventRecord(events_[k + 1], forks_[k]));
@@ -1677,7 +1857,8 @@ void BatchPlan::enqueue(cudaStream_t s)
 
 void BatchPlan::launch_grouped(const GroupedLaunch& g, cudaStream_t s)
 {
-    if (g.cfg.id == kTcConfig) launch_level_tc(g.args, g.start, g.nent, g.cta, g.ctas, dStatus_, s);
+    if (g.cfg.id == kNarrowConfig) launch_expand_narrow(g.args, g.start, g.nent, g.tiles, s);
+    else if (g.cfg.id == kTcConfig) launch_level_tc(g.args, g.start, g.nent, g.cta, g.ctas, dStatus_, s);
     else launch_affine_level_grouped(g.cfg, g.args, g.start, g.nent, g.tiles, g.smem, s);
 }
 

@@ -7,6 +7,9 @@
 //  - scan dimension <= 64: the blocked path per padded dimension NP, batched
 //    (one tables launch, one persistent leaf launch over work items of all
 //    systems, one chain launch, one fix-up launch per NP);
+//  - without inputs, and in the mixed form with sinusoid inputs (whose phases
+//    then take the place of samples): the block states by doublings and the
+//    outputs from them, one grouped GEMM per level (kernels_expand.cu);
 //  - larger scan dimensions: the level-synchronous path with one grouped
 //    contraction launch per level and tiling configuration over all systems;
 //  - systems with inputs where it costs less: the block-response leaf (one
@@ -18,6 +21,7 @@
 #pragma once
 
 #include "blocked.h"
+#include "expand.h"
 #include "host_math.h"
 #include "inputs.h"
 #include "kernels.h"
@@ -79,17 +83,20 @@ public:
     int precision_used(int i) const { return sys_[i].precision; }
     int path(int i) const
     {
-        return sys_[i].resp ? kPathBlockedResponse : sys_[i].blocked ? kPathBlocked : kPathLevel;
+        const Sys& q = sys_[i];
+        if (q.ex) return q.mu > 0 ? kPathBlockedResponse : q.Ns <= 64 ? kPathBlocked : kPathLevel;
+        return q.resp ? kPathBlockedResponse : q.blocked ? kPathBlocked : kPathLevel;
     }
     // Response leaf geometry of system i: block length, window columns,
     // padded scan dimension, blocks (zeros on other paths).
     void response_shape(int i, long long info[4]) const
     {
         const Sys& q = sys_[i];
-        info[0] = q.resp ? q.Bk : 0;
-        info[1] = q.resp ? q.Kw : 0;
-        info[2] = q.resp ? q.Np : 0;
-        info[3] = q.resp ? q.nblocks : 0;
+        const bool on = q.resp || (q.ex && q.mu > 0);
+        info[0] = on ? q.Bk : 0;
+        info[1] = q.ex ? 2L * q.mu * q.K : q.resp ? q.Kw : 0;
+        info[2] = on ? q.Np : 0;
+        info[3] = on ? q.nblocks : 0;
     }
     // Sum over systems of n * outputs (state*steps of one execute).
     double state_steps() const;
@@ -104,6 +111,8 @@ private:
         int lev0 = 0;             // power-table level of scan level 0 (log2 of the block length)
         int pow_levels = 0;       // power-table levels P_0 .. P_{pow_levels - 1}
         bool blocked = false;
+        bool ex = false;          // radix expansion (kernels_expand.cu): no inputs, or mixed with sinusoids
+        ExpandJob exj;
         bool resp = false;        // block-response leaf
         int Bk = 0, Kw = 0, Kpad = 0;  // response: block length, window columns (padded to even)
         long nblocks = 0;
@@ -125,6 +134,7 @@ private:
         int K = 0;
         bool zeroB = true, zeroC = true, zeroD = true;
         long ntiles = 0;
+        bool level_sync() const { return !blocked && !resp && !ex; }
     };
     struct Bucket {
         BlockedShape sh;
@@ -182,6 +192,13 @@ private:
     std::vector<Bucket> buckets_;
     std::vector<int> ls_;  // level-synchronous systems
     std::vector<int> rs_;  // block-response systems (their block scan joins the level launches)
+    std::vector<int> ex_;  // systems by radix expansion
+    std::vector<GroupedLaunch> ex_power_, ex_level_, ex_out_;  // ex_power_: all steps, ex_power_at_[l] launches up to step l
+    std::vector<size_t> ex_power_at_;
+    ExpandJob* dEx_ = nullptr;
+    int exMaxHq_ = 0, exSteps_ = 0;
+    long exMaxInit_ = 1, exMaxRot_ = 1, exMaxFeed_ = 1, exMaxPhases_ = 1;
+    bool choose_expand(Sys& q, const PlanOptions& opt);
     std::vector<GroupedLaunch> ls_power_, ls_up_, ls_down_;
     std::vector<GroupedLaunch> rs_agg_, rs_out_;  // response GEMMs: block aggregates, outputs
     std::vector<GroupedLaunch> rs_tc_, rs_state_;  // mixed: tensor-core aggregates + windows; FP64 state part

@@ -340,6 +340,7 @@ struct PhiJob {
     double* dst = nullptr;
     const double* src = nullptr;
     int n = 0, Np = 0, solver = 0;
+    int ld = 0;  // dst's row pitch (0: Np)
 };
 void launch_phi_batch(const PhiJob* dJobs, int njobs, long max_elems, cudaStream_t s);
 // max_elems: the largest element count of a job (sizes the x dimension); for

@@ -34,6 +34,7 @@
 #include "device_common.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace parode {
 
@@ -406,6 +407,193 @@ __global__ void __launch_bounds__(OutCfg<KS>::threads, 1)
     }
 }
 
+// ---- batches -----------------------------------------------------------------
+// blockIdx.y = job; the x dimension strides over its elements.
+
+constexpr double kTwoPi = 6.283185307179586476925286766559;
+
+// S_1 into E(1)'s phase columns (pads zero), W's first p rows [Cext | 0], and
+// the rotation table.
+__global__ void __launch_bounds__(kThreads) k_expand_init_batch(const ExpandJob* __restrict__ jobs)
+{
+    extern __shared__ double trig[];  // sin, cos of w dt s per (pair, slot)
+    const ExpandJob j = jobs[blockIdx.y];
+    const int HQ = j.H / 2, pairs = (j.Kc - j.NP) / 2, rk4 = j.solver == 0, Wd = rk4 ? 3 : 5;
+    const int coff = rk4 ? 0 : 3 * j.n;
+    for (int e = threadIdx.x; e < HQ * Wd; e += kThreads) {
+        const int q = e / Wd, sl = e - q * Wd;
+        sincos(__dmul_rn(__dmul_rn(kTwoPi, j.freq[q]), j.dt) * sl, &trig[2 * e], &trig[2 * e + 1]);
+    }
+    __syncthreads();
+    const long n0 = (long)j.NP * pairs, n1 = (long)j.p * j.Kc, n2 = (long)j.pow_levels * HQ;
+    for (long e = (long)blockIdx.x * kThreads + threadIdx.x; e < n0 + n1 + n2; e += (long)gridDim.x * kThreads) {
+        if (e < n0) {
+            const int r = (int)(e / pairs), q = (int)(e - (long)r * pairs);
+            double vs = 0.0, vc = 0.0;
+            if (q < HQ && !j.zeroB && r >= coff && r < coff + j.n)
+                for (int sl = 0; sl < Wd; ++sl) {
+                    const double b = j.Bbar[(long)(r - coff) * Wd * j.mu + sl * j.mu + q / j.terms] * j.amp[q];
+                    vs = fma(b, trig[2 * (q * Wd + sl) + 1], vs);
+                    vc = fma(b, trig[2 * (q * Wd + sl)], vc);
+                }
+            *reinterpret_cast<double2*>(j.E + (long)r * j.Kc + j.NP + 2 * q) = make_double2(vs, vc);
+        } else if (e < n0 + n1) {
+            const long u = e - n0;
+            const int o = (int)(u / j.Kc), c = (int)(u - (long)o * j.Kc);
+            j.W[u] = c < j.NP ? j.Cext[(long)o * j.NP + c] : 0.0;
+        } else {
+            const long u = e - n0 - n1;
+            const int l = (int)(u / HQ), q = (int)(u - (long)l * HQ);
+            const double step = __dmul_rn(__dmul_rn(kTwoPi, j.freq[q]), j.dt) * (rk4 ? 2 : 1);
+            sincos(ldexp(step, l), &j.rot[2 * u], &j.rot[2 * u + 1]);
+        }
+    }
+}
+
+// The rotation parts [0 | S R] of step l, which its GEMMs then add to.
+__global__ void __launch_bounds__(kThreads) k_expand_rot_batch(const ExpandJob* __restrict__ jobs, int l)
+{
+    const ExpandJob j = jobs[blockIdx.y];
+    const int half = j.Kc / 2, HQ = j.H / 2;
+    const long erows = l + 1 < j.pow_levels ? j.NP : 0, wrows = l < j.R ? ((long)1 << l) * j.p : 0;
+    const double* rot = j.rot + (long)l * j.H;
+    for (long e = (long)blockIdx.x * kThreads + threadIdx.x; e < (erows + wrows) * half;
+         e += (long)gridDim.x * kThreads) {
+        const long r = e / half;
+        const int c = 2 * (int)(e - r * half), q = (c - j.NP) / 2;
+        const double* src = r < erows ? j.E + ((long)l * j.NP + r) * j.Kc : j.W + (r - erows) * j.Kc;
+        double* dst = r < erows ? j.E + ((long)(l + 1) * j.NP + r) * j.Kc : j.W + (r - erows + wrows) * j.Kc;
+        double2 v = make_double2(0.0, 0.0);
+        if (c >= j.NP && q < HQ) {
+            const double s0 = src[c], s1 = src[c + 1], si = rot[2 * q], co = rot[2 * q + 1];
+            v = make_double2(s0 * co - s1 * si, s0 * si + s1 * co);
+        }
+        *reinterpret_cast<double2*>(dst + c) = v;
+    }
+}
+
+// D u of the block's steps into W: step i reads sample 2 i (RK4) or i + 3 (ABM).
+__global__ void __launch_bounds__(kThreads) k_expand_feed_batch(const ExpandJob* __restrict__ jobs)
+{
+    const ExpandJob j = jobs[blockIdx.y];
+    if (j.zeroD) return;
+    const int HQ = j.H / 2;
+    for (long e = (long)blockIdx.x * kThreads + threadIdx.x; e < ((long)HQ << j.R); e += (long)gridDim.x * kThreads) {
+        const long i = e / HQ;
+        const int q = (int)(e - i * HQ);
+        double si, co;
+        sincos(__dmul_rn(__dmul_rn(kTwoPi, j.freq[q]), j.dt) * (double)(j.solver == 0 ? 2 * i : i + 3), &si, &co);
+        for (int o = 0; o < j.p; ++o) {
+            const double d = j.D[(long)o * j.mu + q / j.terms] * j.amp[q];
+            double* w = j.W + (i * j.p + o) * j.Kc + j.NP + 2 * q;
+            w[0] += d * co;
+            w[1] += d * si;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_expand_phases_batch(const ExpandJob* __restrict__ jobs)
+{
+    const ExpandJob j = jobs[blockIdx.y];
+    const int pairs = (j.Kc - j.NP) / 2, HQ = j.H / 2;
+    const long total = j.nblocks * pairs;
+    const long e0 = (long)blockIdx.x * kThreads + threadIdx.x, step = (long)gridDim.x * kThreads;
+    for (long e = e0; e < j.NP; e += step) j.Z[e] = j.X0[e];
+    for (long e = e0; e < total; e += step) {
+        const long b = e / pairs;
+        const int q = (int)(e - b * pairs);
+        double si = 0.0, co = 0.0;
+        if (q < HQ) {
+            const double ts = sample_time(j.base, j.dt, b * j.stride);
+            sincos(__dadd_rn(__dmul_rn(__dmul_rn(kTwoPi, j.freq[q]), ts), j.phi[q]), &si, &co);
+        }
+        *reinterpret_cast<double2*>(j.Z + b * j.Kc + j.NP + 2 * q) = make_double2(si, co);
+    }
+}
+
+// dst(g, r) = sum_k P[r][k] src(g, k): CTA = 8 rows x 32 columns g, its four
+// warps a quarter of K each (fragments straight from L2, two K values per
+// load), the quarters summed in order.  Latency-bound, so a warp has the
+// loads of kBatch K chunks in flight before their products.  A level of one
+// system with NP = 512, Kc = 608 and up to 32 columns is 64 CTAs instead of 8
+// of the 64 x 64 tiles (19 us, mostly padding).
+constexpr int kNarrowThreads = 128, kNarrowCols = 32;
+
+template <int CT>
+__device__ __forceinline__ void narrow_mma(const double* pr, const double* const (&z)[4], int k0, int k1,
+                                           double (&acc)[4][2])
+{
+    constexpr int kBatch = CT == 1 ? 8 : CT == 2 ? 6 : 4;
+    for (int k = k0; k < k1; k += kBatch) {
+        double2 e[kBatch], v[kBatch][CT];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int kk = 8 * min(k + u, k1 - 1);  // chunks past the end load the last one and are not used
+            e[u] = *reinterpret_cast<const double2*>(pr + kk);
+#pragma unroll
+            for (int c = 0; c < CT; ++c) v[u][c] = *reinterpret_cast<const double2*>(z[c] + kk);
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+            for (int c = 0; c < CT; ++c) {
+                if (k + u >= k1) continue;
+                dmma_m8n8k4(acc[c][0], acc[c][1], v[u][c].x, e[u].x);
+                dmma_m8n8k4(acc[c][0], acc[c][1], v[u][c].y, e[u].y);
+            }
+    }
+}
+
+__global__ void __launch_bounds__(kNarrowThreads) k_expand_narrow(const LevelArgs* __restrict__ args,
+                                                                  const long* __restrict__ start, int nent)
+{
+    __shared__ double2 red[4][4][32];
+    const long t = blockIdx.x;
+    int lo = 0, hi = nent - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (start[mid] <= t) lo = mid;
+        else hi = mid - 1;
+    }
+    const LevelArgs& a = args[lo];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
+    const int rt = a.M / 8;
+    const long u = t - start[lo], c0 = (u / rt) * kNarrowCols;
+    const int r0 = (int)(u % rt) * 8;
+    const int cols = (int)min((long)kNarrowCols, a.ncols - c0), ct = (cols + 7) / 8;
+    const int n8 = a.K / 8, k0 = n8 * warp / 4, k1 = n8 * (warp + 1) / 4;
+    const double* pr = a.P + (long)(r0 + g) * a.ldp + 2 * tq;
+    const double* z[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) z[c] = a.src + (c0 + (8 * c + g < cols ? 8 * c + g : 0)) * a.src_gs + 2 * tq;
+    double acc[4][2] = {};
+    switch (ct) {
+    case 1: narrow_mma<1>(pr, z, k0, k1, acc); break;
+    case 2: narrow_mma<2>(pr, z, k0, k1, acc); break;
+    case 3: narrow_mma<3>(pr, z, k0, k1, acc); break;
+    default: narrow_mma<4>(pr, z, k0, k1, acc); break;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) red[warp][c][lane] = make_double2(acc[c][0], acc[c][1]);
+    __syncthreads();
+    if (8 * warp + g < cols) {  // this warp stores column tile `warp`
+        double2 v = red[0][warp][lane];
+#pragma unroll
+        for (int w = 1; w < 4; ++w) {
+            v.x += red[w][warp][lane].x;
+            v.y += red[w][warp][lane].y;
+        }
+        *reinterpret_cast<double2*>(a.dst + (c0 + 8 * warp + g) * a.dst_gs + r0 + 2 * tq) = v;
+    }
+}
+
+// x extent of a batched launch: a few CTAs a job, about 2048 in all when the jobs are few.
+unsigned batch_x(long max_elems, int njobs)
+{
+    const long want = std::max<long>(4, (2048 + njobs - 1) / njobs);
+    return (unsigned)std::max<long>(1, std::min<long>((max_elems + kThreads - 1) / kThreads, want));
+}
+
 template <int KS>
 void level_t(const ExpandTables& t, const double* T, double* Z, int imax, long d, cudaStream_t s)
 {
@@ -540,6 +728,128 @@ void launch_expand_out(const ExpandTables& t, const double* Z, double* Y, long c
 {
     if (c1 <= c0) return;
     by_width(t.sh.Kc, [&](auto ks) { out_t<decltype(ks)::value>(t, Z, Y, c0, c1, limit, sms, s); });
+}
+
+int expand_log2_block(int NP, int Kc, int p, long nScan, double executions)
+{
+    int best = 3;
+    double best_cost = -1.0;
+    for (int R = 3; R <= 7; ++R) {
+        const double B = (double)(1 << R);
+        if (R > 3 && B / 2 >= (double)nScan) break;
+        if (R > 3 && 8.0 * B * p * Kc > 256e6) break;
+        const double build = executions > 0 ? 2.0 * B * p * NP * Kc / ((double)nScan * executions) : 0.0;
+        const double cost = 2.0 * NP * Kc / B + build;
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best = R;
+        }
+    }
+    return best;
+}
+
+void launch_expand_init(const ExpandJob* dJobs, int njobs, int max_hq, long max_elems, cudaStream_t s)
+{
+    const size_t smem = sizeof(double) * 2 * 5 * (size_t)std::max(max_hq, 1);
+    PARODE_CUDA(cudaFuncSetAttribute(k_expand_init_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_expand_init_batch<<<dim3(batch_x(max_elems, njobs), (unsigned)njobs), kThreads, smem, s>>>(dJobs);
+    PARODE_CUDA(cudaGetLastError());
+}
+
+void launch_expand_rot(const ExpandJob* dJobs, int njobs, int l, long max_elems, cudaStream_t s)
+{
+    k_expand_rot_batch<<<dim3(batch_x(max_elems, njobs), (unsigned)njobs), kThreads, 0, s>>>(dJobs, l);
+    PARODE_CUDA(cudaGetLastError());
+}
+
+void launch_expand_feed(const ExpandJob* dJobs, int njobs, long max_elems, cudaStream_t s)
+{
+    k_expand_feed_batch<<<dim3(batch_x(max_elems, njobs), (unsigned)njobs), kThreads, 0, s>>>(dJobs);
+    PARODE_CUDA(cudaGetLastError());
+}
+
+int expand_power_args(const ExpandJob& j, int l, LevelArgs out[2])
+{
+    int c = 0;
+    const double* El = j.E + (long)l * j.NP * j.Kc;
+    LevelArgs a;  // [Phi^(2^l) as rows] x E(2^l), onto the rotation part
+    a.P = El;
+    a.ldp = j.Kc;
+    a.Np = j.NP;
+    a.M = j.NP;
+    a.K = j.NP;
+    a.ncols = j.Kc;
+    a.src = El;
+    a.src_gs = 1;
+    a.src_ks = j.Kc;
+    a.acc_gs = a.dst_gs = 1;
+    a.acc_is = a.dst_is = j.Kc;
+    if (l + 1 < j.pow_levels) {
+        a.dst = j.E + (long)(l + 1) * j.NP * j.Kc;
+        a.acc = a.dst;
+        out[c++] = a;
+    }
+    if (l < j.R) {
+        a.P = j.W;
+        a.M = j.p << l;
+        a.dst = j.W + ((long)j.p << l) * j.Kc;
+        a.acc = a.dst;
+        out[c++] = a;
+    }
+    return c;
+}
+
+void launch_expand_phases(const ExpandJob* dJobs, int njobs, long max_elems, cudaStream_t s)
+{
+    k_expand_phases_batch<<<dim3(batch_x(max_elems, njobs), (unsigned)njobs), kThreads, 0, s>>>(dJobs);
+    PARODE_CUDA(cudaGetLastError());
+}
+
+LevelArgs expand_level_args(const ExpandJob& j, int l)
+{
+    const long d = 1L << l;
+    LevelArgs a;
+    a.P = j.E + (long)(j.R + l) * j.NP * j.Kc;
+    a.ldp = j.Kc;
+    a.Np = j.NP;
+    a.M = j.NP;
+    a.K = j.Kc;
+    a.ncols = std::min(d, j.nblocks - d);
+    a.src = j.Z;
+    a.src_gs = j.Kc;
+    a.src_ks = 1;
+    a.dst = j.Z + d * j.Kc;
+    a.dst_gs = j.Kc;
+    a.dst_is = 1;
+    return a;
+}
+
+LevelArgs expand_out_args(const ExpandJob& j, double* Y, long limit)
+{
+    LevelArgs a;
+    a.P = j.W;
+    a.ldp = j.Kc;
+    a.Np = j.NP;
+    a.M = j.p << j.R;
+    a.K = j.Kc;
+    a.ncols = j.nblocks;
+    a.src = j.Z;
+    a.src_gs = j.Kc;
+    a.src_ks = 1;
+    a.dst = Y;
+    a.dst_gs = a.M;
+    a.dst_is = 1;
+    a.dst_limit = limit;
+    return a;
+}
+
+long expand_narrow_tiles(const LevelArgs& a) { return (long)(a.M / 8) * ((a.ncols + kNarrowCols - 1) / kNarrowCols); }
+
+void launch_expand_narrow(const LevelArgs* dArgs, const long* dStart, int nent, long tiles, cudaStream_t s)
+{
+    if (tiles <= 0) return;
+    k_expand_narrow<<<(unsigned)tiles, kNarrowThreads, 0, s>>>(dArgs, dStart, nent);
+    PARODE_CUDA(cudaGetLastError());
 }
 
 }  // namespace parode

@@ -525,7 +525,7 @@ __global__ void k_phi_batch(const PhiJob* __restrict__ jobs)
         } else if (r < 4 * n && c < 4 * n) {
             v = J.src[(long)(r - 3 * n) * (4 * n) + c];
         }
-        J.dst[e] = v;
+        J.dst[J.ld ? (long)r * J.ld + c : e] = v;
     }
 }
 

@@ -60,6 +60,18 @@ size_t estimate_request_bytes(const BatchSpec& b, int precision)
         if (precision == kMixed) bytes += (double)level_split_bytes((int)Np) * levels;
         bytes += 8.0 * (double)levels * 1024;                                 // launch descriptors
     }
+    if (mu == 0 || (precision == kMixed && b.input && b.input->kind == InputEntry::kSinusoid)) {
+        // the radix expansion (batch.cpp choose_expand): powers, output table,
+        // block states, rotations and launch descriptors instead of the samples
+        // and the scan; the larger estimate of the two counts
+        const int np = (int)round_up(Ns, 8);
+        const double kc = (double)round_up(np + (mu > 0 ? 2L * mu * b.input->K : 0), 8);
+        const int R = expand_log2_block(np, (int)kc, p, nScan, 1.0);
+        const double blocks = (double)((nScan + (1L << R) - 1) >> R), pw = std::max(ilog2(nScan) + 1, R);
+        const double ex = 8.0 * (pw * np * kc + (double)(p << R) * kc + blocks * kc + pw * kc + (double)nOut * p) +
+                          8.0 * pw * 1024;
+        bytes = std::max(bytes, ex);
+    }
     return (size_t)(bytes * 1.05) + (1u << 20);
 }
 

@@ -161,7 +161,15 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         throw Error(kInvalidArgument, "the general scan supports scan dimensions up to 64");
     if ((opt.shards > 1 || opt.shard != 0) && (Ns_ > 64 || opt.path == kPathGeneral || opt.path == kPathLevel))
         throw Error(kInvalidArgument, "a time shard runs on the block-response path (scan dimension <= 64, inputs)");
-    if (Ns_ > 64 && opt.path != kPathBlocked && opt.path != kPathBlockedSweep) {
+    // sinusoid inputs whose phases are too wide for the single-plan expansion
+    // take the batch engine's (RK4 n = 64, m = 8, 10 terms, 2^18 steps mixed:
+    // 0.26 ms with the sample windows)
+    const bool wide = Ns_ > 8 && Ns_ <= 64 && opt.path == kPathAuto && opt.precision == kMixed && opt.shards <= 1 &&
+                      opt.shard == 0 && !opt.fault_withhold && mu_ > 0 && input_->kind == InputEntry::kSinusoid &&
+                      input_->m >= mu_ && (long)mu_ * input_->K <= kExpandMaxPairs &&
+                      blocked_shape(Ns_, mu_, solver, &shape_) &&
+                      !expand_shape(Ns_, mu_, input_->K, p_, nScan_, 6, &ext_.sh);
+    if ((Ns_ > 64 && opt.path != kPathBlocked && opt.path != kPathBlockedSweep) || wide) {
         // scan dimensions above 64: the batch engine's one-system form (the
         // response leaf or the level-synchronous scan, tensor-core levels in
         // the mixed form)

@@ -138,3 +138,57 @@ def test_input_with_too_few_channels_is_refused(pb):
     with pytest.raises(pb.ParODEError) as e:
         pb.simulate(c.A, c.B, c.C, c.D, c.x0, u, c.t0, c.t_end, c.h, solver=0, precision=pb.MIXED)
     assert e.value.code == -8
+
+
+BATCH = [  # solver, n, m, p, T, terms, B, C, D (the batch's doublings; any scan dimension)
+    (0, 1, 1, 1, 1, 1, True, True, True), (0, 8, 2, 3, 700, 3, True, True, True), (0, 65, 5, 4, 64 * 33, 3, True, True, True),
+    (0, 96, 12, 12, 9001, 2, True, True, False), (0, 200, 3, 7, 2500, 5, True, False, True), (1, 1, 1, 1, 4, 1, True, True, True),
+    (1, 17, 2, 2, 39_146, 3, True, True, True), (1, 40, 5, 5, 5003, 3, False, True, True), (1, 100, 2, 1, 1031, 4, True, True, True),
+    (0, 30, 0, 30, 3333, 0, False, False, False), (0, 90, 0, 5, 20_000, 0, False, True, False),
+    (1, 33, 0, 33, 4100, 0, False, False, False),
+]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_batch_expansion(pb, precision):
+    """Mixed: every system by the expansion; FP64: those without inputs."""
+    specs, refs = [], []
+    for k, (solver, n, m, p, T, terms, B, Cm, D) in enumerate(BATCH):
+        if precision == 0 and m:
+            continue
+        c = wl.small(17000 + 31 * k, solver, n, max(m, 1), p, T, h=1e-3)
+        s = wl.sinusoid(wl.Rng(17500 + k), max(m, 1), max(terms, 1))
+        u = pb.register_sinusoid(s.a, s.f, s.phi)
+        specs.append({"A": c.A, "B": c.B if B else None, "C": c.C if Cm else None, "D": c.D if D else None, "x0": c.x0,
+                      "u": u, "t0": c.t0, "t_end": c.t_end, "h": c.h, "solver": solver})
+        inp = oracle.Input.sinusoid(s.a, s.f, s.phi) if m else oracle.Input.zero()
+        refs.append((m, oracle.simulate_affine(oracle.System(c.A, specs[-1]["B"], specs[-1]["C"], specs[-1]["D"], c.x0),
+                                               inp, solver, c.t0, c.t_end, c.h)))
+    b = pb.Batch(specs, precision=precision)
+    for _ in range(3):  # eager, captured, replayed
+        b.execute()
+    for i, (m, ref) in enumerate(refs):
+        _, y = b.output(i)
+        assert y.shape == ref.shape
+        err = oracle.rel_err(y, ref)
+        assert err <= (TOL_PHASES if m else TOL_FREE), (i, specs[i]["solver"], specs[i]["A"].shape, err)
+        assert b.path(i) == (3 if m else 2 if specs[i]["A"].shape[0] * (4 if specs[i]["solver"] else 1) <= 64 else 1)
+    b.close()
+
+
+@pytest.mark.parametrize("solver,n,m,T,terms", [(0, 72, 9, 100, 3), (1, 128, 16, 64 * 600 + 5, 3), (0, 520, 2, 1500, 3),
+                                                (0, 64, 8, 9000, 7), (1, 16, 10, 3001, 40)])
+def test_large_plan_runs_doublings(pb, solver, n, m, T, terms):
+    """One system above scan dimension 64, or with more phases than the
+    single-plan kernels take: few tiles a level, so most levels take the
+    narrow kernel, the others the 64 x 64 tiles."""
+    c = wl.small(18000 + n, solver, n, m, 3, T, h=5e-4)
+    s = wl.sinusoid(wl.Rng(18500 + n), m, terms)
+    u = pb.register_sinusoid(s.a, s.f, s.phi)
+    plan = _plan(pb, c, u, pb.MIXED)
+    assert plan.precision == pb.MIXED and plan.response_shape[1] == 2 * terms * m
+    y = _device_y(plan, 0)
+    plan.close()
+    ref = oracle.simulate_affine(oracle.System(c.A, c.B, c.C, c.D, c.x0), oracle.Input.sinusoid(s.a, s.f, s.phi),
+                                 solver, c.t0, c.t_end, c.h)
+    assert oracle.rel_err(y, ref) <= TOL_PHASES
