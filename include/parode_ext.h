@@ -264,16 +264,15 @@ void ParODE_AffineScanDevice(const double* dPhi, const double* dGamma, const dou
 /* General affine scan over per-step maps on device data: x_0 = dX0 (NULL:
  * zero), x_{k+1} = dM[k] x_k + dV[k] (dV NULL: zero), dX[k] = x_k for
  * k < count; dM count x ns x ns, dV and dX count x ns, row-major FP64, device
- * memory of the current device; ns in [1, 64].  Every pair of every up-sweep
- * level is composed, matrices and vectors, as the reference's MM / MVV scan
- * kernels do (Kernels/MMKernelScanUpsweep.cl:13-56,
- * Kernels/MVVKernelScanUpsweep.cl:14-50, MVVKernelScanDownsweep.cl:14-50), so
- * the maps may differ from step to step (a time-varying system).  precision:
- * PARODE_PRECISION_FP64 (FP64 tensor cores) or PARODE_PRECISION_MIXED (the
- * matrix products in 3xTF32 on tcgen05 for ns in 17..64, the vectors in FP64).
- * Enqueued on `stream` (NULL: the legacy default stream); returns once the
- * scan is done.  Scratch (count rounded up to a power of two, times
- * ns^2 + ns doubles with ns rounded up to 8, 16, 32 or 64) comes from the
+ * memory of the current device; ns in [1, 64].  The maps may differ from step
+ * to step (a time-varying system): the scan composes them, matrices and
+ * vectors, as the reference's MM / MVV scan kernels do
+ * (Kernels/MMKernelScanUpsweep.cl:13-56, Kernels/MVVKernelScanUpsweep.cl:14-50,
+ * MVVKernelScanDownsweep.cl:14-50), chunk by chunk.  precision:
+ * PARODE_PRECISION_FP64 or PARODE_PRECISION_MIXED; the arithmetic is FP64
+ * (FP64 tensor cores) in both.  dX may be dV.  Enqueued on `stream` (NULL: the
+ * legacy default stream); returns once the scan is done.  Scratch (about
+ * count / 15 times ns^2 + 2 ns doubles with ns rounded up to 8) comes from the
  * device's stream-ordered pool. */
 void ParODE_AffineScanGeneral(const double* dM, const double* dV, const double* dX0, int ns, long long count,
                               int precision, double* dX, void* stream, int nErr[]);

@@ -946,24 +946,8 @@ void ParODE_AffineScanGeneral(const double* dM, const double* dV, const double* 
         if (precision != PARODE_PRECISION_FP64 && precision != PARODE_PRECISION_MIXED)
             throw Error(kInvalidArgument, "unknown precision");
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        int* status = nullptr;
-        if (fault_alloc_now()) throw Error(kNotEnoughResources, "device allocation failed (injected)");
-        if (cudaMallocAsync(reinterpret_cast<void**>(&status), sizeof(int), s) != cudaSuccess) {
-            cudaGetLastError();
-            throw Error(kNotEnoughResources, "device allocation failed");
-        }
-        int host_status = 0;
-        try {
-            PARODE_CUDA(cudaMemsetAsync(status, 0, sizeof(int), s));
-            general_scan(dM, dV, dX0, ns, (long)count, precision, dX, status, s);
-            PARODE_CUDA(cudaMemcpyAsync(&host_status, status, sizeof(int), cudaMemcpyDeviceToHost, s));
-            PARODE_CUDA(cudaStreamSynchronize(s));
-        } catch (...) {
-            cudaFreeAsync(status, s);
-            throw;
-        }
-        PARODE_CUDA(cudaFreeAsync(status, s));
-        if (host_status != 0) throw Error(kDeviceError, "a device-side wait gave up (tensor-core completion not observed)");
+        general_scan(dM, dV, dX0, ns, (long)count, precision, dX, s);
+        PARODE_CUDA(cudaStreamSynchronize(s));
     });
     if (nErr) nErr[0] = rc;
 }

@@ -1,63 +1,104 @@
 // general.cpp -- host driver of the general affine scan (general.h).
 //
 // The reference's scan driver (Sources/GPUFixedStepIterative.cpp:236-398)
-// with its matrix products kept: a level-synchronous up-sweep that composes
-// the pairs of each level (matrices and vectors), then a down-sweep that
-// passes the prefixes down through the left subtrees' compositions, in place.
-// Pairs whose span starts past the last map are skipped (the padding up to
-// the next power of two is never read for an output).
+// with its matrix products kept, over chunks instead of levels of pairs
+// (kernels_general.cu).
 #include "general.h"
 
 #include "common.h"
 #include "kernels.h"
 
 #include <algorithm>
+#include <vector>
 
 namespace parode {
 
+namespace {
+
+// Maps per chunk: 16, up to 64 at the lowest level while that still leaves a
+// chunk for each of 16 warps per SM (a chunk's maps are composed one after
+// another, so short chunks cost upper-level work and long ones parallelism).
+int chunk_length(long count)
+{
+    int L = 16;
+    while (L < 64 && count / (2 * L) >= 148L * 24) L *= 2;
+    return L;
+}
+
+// The device's stream-ordered pool keeps a scan's scratch mapped for the next
+// one (as a plan's buffers): mapped anew, 10 MB cost 0.5 ms a call.
+void keep_scratch(size_t bytes)
+{
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    PARODE_CUDA(cudaGetDevice(&dev));
+    PARODE_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
+    uint64_t keep = 0, want = 2 * (uint64_t)bytes + ((uint64_t)64 << 20);
+    PARODE_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    if (keep < want) PARODE_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &want));
+}
+
+}  // namespace
+
+size_t general_scan_bytes(int ns, long count)
+{
+    const long Tp = next_pow2(std::max<long>(count, 1));
+    const long NP = general_padded_dim(ns);
+    return sizeof(double) * (size_t)(Tp * NP * NP + (Tp + 1) * NP);
+}
+
 void general_scan(const double* M, const double* V, const double* x0, int ns, long count, int precision,
-                  double* X, int* status, cudaStream_t s)
+                  double* X, cudaStream_t s)
 {
     if (!M || !X) throw Error(kInvalidArgument, "general scan: M and X must be device pointers");
     if (ns < 1 || ns > 64) throw Error(kInvalidArgument, "general scan: scan dimension must be in [1, 64]");
     if (count < 1) throw Error(kInvalidArgument, "general scan: count must be >= 1");
     if (precision != kFP64 && precision != kMixed) throw Error(kInvalidArgument, "unknown precision");
-    int dev = 0, sms = 148;
-    PARODE_CUDA(cudaGetDevice(&dev));
-    PARODE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int NP = general_padded_dim(ns);
-    const long Tp = next_pow2(count);
+    const int NP = (int)round_up(ns, 8);
+    // level 0: the caller's maps; level l + 1: the compositions of level l's
+    // chunks (all but the last, whose composition no state needs)
+    std::vector<ScanLevel> lev(1);
+    lev[0] = ScanLevel{M, V, X, ns, count, chunk_length(count)};
+    size_t doubles = 0;
+    std::vector<size_t> at;
+    while (lev.back().count > lev.back().L) {
+        const ScanLevel& b = lev.back();
+        ScanLevel u;
+        u.ns = NP;
+        u.count = (b.count + b.L - 1) / b.L;
+        u.L = chunk_length(u.count);
+        at.push_back(doubles);
+        doubles += (size_t)u.count * NP * (NP + 2);
+        lev.push_back(u);
+    }
     double* buf = nullptr;
     if (fault_alloc_now()) throw Error(kNotEnoughResources, "general scan: device allocation failed (injected)");
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&buf), general_scan_bytes(ns, count), s);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        throw Error(kNotEnoughResources, "general scan: device allocation failed");
+    if (doubles) {
+        keep_scratch(sizeof(double) * doubles);
+        cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&buf), sizeof(double) * doubles, s);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            throw Error(kNotEnoughResources, "general scan: device allocation failed");
+        }
     }
-    double* Mp = buf;
-    double* Vp = Mp + Tp * (long)NP * NP;  // slot -1
-    double* V1 = Vp + NP;                  // slot 0
     try {
-        launch_general_in(Mp, Vp, M, V, x0, ns, NP, count, Tp, sms, s);
-        const int levels = ilog2(Tp);
-        for (int l = 0; l < levels; ++l) {
-            const long d = 1L << l;
-            // mixed form: the top four levels compose in FP64, as the mixed
-            // level-synchronous scan keeps its high powers (few pairs, and
-            // their products carry the whole horizon)
-            const int prec = l < levels - 4 ? precision : (int)kFP64;
-            launch_compose(NP, prec, Mp, V1, d, sweep_columns(count, Tp, d), sms, status, s);
+        for (size_t l = 1; l < lev.size(); ++l) {
+            ScanLevel& u = lev[l];
+            double* m = buf + at[l - 1];
+            u.M = m;
+            u.V = m + (size_t)u.count * NP * NP;
+            u.X = m + (size_t)u.count * NP * (NP + 1);
+            launch_scan_up(lev[l - 1], NP, u.count - 1, m, m + (size_t)u.count * NP * NP, s);
         }
-        for (int l = levels - 1; l >= 0; --l) {
-            const long d = 1L << l;
-            launch_down_general(NP, Mp, V1, d, sweep_columns(count, Tp, d), sms, s);
+        for (size_t l = lev.size(); l-- > 0;) {
+            const bool top = l + 1 == lev.size();
+            launch_scan_down(lev[l], NP, top ? x0 : lev[l + 1].X, top ? ns : NP, s);
         }
-        launch_general_out(X, Vp, ns, NP, count, sms, s);
     } catch (...) {
-        cudaFreeAsync(buf, s);
+        if (buf) cudaFreeAsync(buf, s);
         throw;
     }
-    PARODE_CUDA(cudaFreeAsync(buf, s));
+    if (buf) PARODE_CUDA(cudaFreeAsync(buf, s));
 }
 
 }  // namespace parode

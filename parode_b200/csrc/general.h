@@ -1,5 +1,5 @@
 // general.h -- the general affine scan over per-step maps (kernels_general.cu,
-// kernels_general_tc.cu, general.cpp).
+// general.cpp).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -8,34 +8,34 @@
 
 namespace parode {
 
-// Padded scan dimension of the general scan (8, 16, 32 or 64).
+// Padded scan dimension of a plan's general path (8, 16, 32 or 64) and the
+// device bytes by which that path judges whether a solve is too large.
 int general_padded_dim(int ns);
-// Device bytes of its scan buffers for `count` maps.
 size_t general_scan_bytes(int ns, long count);
 
-// Caller arrays into / out of the padded in-place layout (general.h).
-void launch_general_in(double* Mp, double* Vp, const double* M, const double* V, const double* x0, int ns, int NP,
-                       long count, long Tp, int sms, cudaStream_t s);
-void launch_general_out(double* X, const double* Vp, int ns, int NP, long count, int sms, cudaStream_t s);
 // Ms[k] = Phi (NP x NP) for k < count.
 void launch_distribute(double* Ms, const double* Phi, int NP, long count, int sms, cudaStream_t s);
 
-// Up-sweep level with distance d over npairs pairs: V1[k] += M[k] V1[k-d],
-// M[k] <- M[k] M[k-d] for k = q 2d + 2d - 1 (V1 = slot 0).  precision kMixed
-// runs the products on tcgen05 (3xTF32) where compose_tc_supported(NP).
-void launch_compose(int NP, int precision, double* M, double* V1, long d, long npairs, int sms, int* status,
-                    cudaStream_t s);
-bool compose_tc_supported(int NP);
-void launch_compose_tc(int NP, double* M, double* V1, long d, long npairs, int sms, int* status, cudaStream_t s);
-// Down-sweep level: V1[L] += M[L] V1[p], L = q 2d + d - 1, p = q 2d - 1.
-void launch_down_general(int NP, const double* M, double* V1, long d, long npairs, int sms, cudaStream_t s);
+// One level of the chunked scan: count maps M[k] (ns x ns) with V[k] (ns, or
+// null), in chunks of L, and the states X[k] (ns) entering them.
+struct ScanLevel {
+    const double* M = nullptr;
+    const double* V = nullptr;
+    double* X = nullptr;
+    int ns = 0;
+    long count = 0;
+    int L = 16;
+};
+// The compositions of the first nch chunks: Mo (NP x NP each) and Vo (NP), NP = ns rounded up to 8.
+void launch_scan_up(const ScanLevel& l, int NP, long nch, double* Mo, double* Vo, cudaStream_t s);
+// X of every chunk from the states entering the chunks (pitch ss; null: zero).
+void launch_scan_down(const ScanLevel& l, int NP, const double* starts, int ss, cudaStream_t s);
 
 // The whole scan on device data: x_0 = x0 (nullptr: 0), x_{k+1} = M_k x_k +
 // V_k (V nullptr: 0), X[k] = x_k for k < count; M count x ns x ns, V and X
-// count x ns, row-major FP64.  Scratch from the stream-ordered pool; returns
-// after enqueueing (status: device word the tensor-core kernel sets on a
-// time-out, nullptr for the FP64 form).
+// count x ns (X may be V), row-major FP64.  FP64 in either precision form.
+// Scratch from the stream-ordered pool; returns after enqueueing.
 void general_scan(const double* M, const double* V, const double* x0, int ns, long count, int precision,
-                  double* X, int* status, cudaStream_t s);
+                  double* X, cudaStream_t s);
 
 }  // namespace parode

@@ -199,7 +199,7 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
     if (opt.path == kPathGeneral) {
         path_ = kPathGeneral;
         Np_ = general_padded_dim(Ns_);
-        precision_used_ = (opt.precision != kFP64 && compose_tc_supported(Np_)) ? kMixed : kFP64;
+        precision_used_ = (opt.precision != kFP64 && Np_ >= 32) ? kMixed : kFP64;  // FP64 arithmetic in both forms
         const double bytes = (double)nScan_ * Np_ * Np_ * 8.0 + (double)general_scan_bytes(Np_, nScan_);
         if (bytes > 24e9) throw Error(kNotEnoughResources, "the general scan holds a copy of Phi per step");
     } else {
@@ -1066,7 +1066,7 @@ void Plan::execute_general(double* Y, cudaStream_t s)
     launch_distribute(dMs_, dPow_, Np_, nScan_, sms_, s);
     launches += 2;
     mark("maps", s);
-    general_scan(dMs_, V1, dX0_, Np_, nScan_, precision_used_, dXs_, dStatus_, s);
+    general_scan(dMs_, V1, dX0_, Np_, nScan_, precision_used_, dXs_, s);
     launches += 2 * ilog2(Tp_) + 2;
     mark("scan", s);
     if (solver_ == kRK4) {
