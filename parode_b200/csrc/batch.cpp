@@ -946,6 +946,10 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
     // input samples
     {
         std::vector<SampleJob> sj;
+        long samples = 0;
+        for (const Sys& q : sys_)
+            if (q.mu > 0 && !q.ex && q.input->kind == InputEntry::kSinusoid) samples += q.nU * q.mu;
+        const int run = sample_run(samples);
         for (int i = 0; i < N; ++i) {
             const Sys& q = sys_[i];
             if (q.mu <= 0 || q.ex) continue;
@@ -964,7 +968,8 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             j.base = q.u_base;
             j.dt = q.u_dt;
             j.count = q.nU;
-            maxSample_ = std::max(maxSample_, (q.nU + kSampleRun - 1) / kSampleRun * q.mu);  // threads: runs x channels
+            j.run = run;
+            maxSample_ = std::max(maxSample_, (q.nU + run - 1) / run * q.mu);  // threads: runs x channels
             maxTerms_ = std::max(maxTerms_, q.K);
             sj.push_back(j);
         }

@@ -98,8 +98,7 @@ __device__ __forceinline__ double sample_time(double base, double dt, long j)
     return __dadd_rn(base, __dmul_rn(dt, (double)j));
 }
 
-// Samples j0 .. j0 + L - 1 (those below count) of channel i of the sum-of-
-// sinusoid input, into out[(j - j0) * stride]: the values sinusoid_value
+// Samples j0 .. j0 + n - 1 of channel i of the sum-of-sinusoid input, into out[(j - j0) * stride]: the values sinusoid_value
 // gives, at a fraction of its cost.  Every argument is rounded exactly as
 // sinusoid_value rounds it; each term starts from sincos at j0 and advances
 // by the rotation through the difference d of consecutive arguments.  d is
@@ -115,7 +114,7 @@ __device__ __forceinline__ double sample_time(double base, double dt, long j)
 // side by side as independent chains and are summed in sinusoid_value's
 // order; inputs with more than 4 terms per channel take sinusoid_value per
 // sample.
-template <int L, int KT, class Out>
+template <int KT, class Out>
 __device__ __forceinline__ void sinusoid_run_terms(const double* a, const double* f, const double* phi, int i,
                                                    double base, double dt, long j0, int n, const Out& out,
                                                    long joff)
@@ -165,7 +164,7 @@ __device__ __forceinline__ void sinusoid_run_terms(const double* a, const double
 // the amplitude at the benchmark's times): for the TF32 sample planes, whose
 // own rounding is 2^-22, not for the FP64 samples.  5 FP64 operations per
 // term and sample instead of ~14.
-template <int L, int KT, class Out>
+template <int KT, class Out>
 __device__ __forceinline__ void sinusoid_rot_terms(const double* a, const double* f, const double* phi, int i,
                                                    double base, double dt, long j0, int n, const Out& out, long joff)
 {
@@ -195,16 +194,14 @@ __device__ __forceinline__ void sinusoid_rot_terms(const double* a, const double
     }
 }
 
-template <int L, int KMAX, class Out>
+template <int KMAX, class Out>
 __device__ __forceinline__ void sinusoid_rot(const double* a, const double* f, const double* phi, int K, int i,
-                                             double base, double dt, long j0, long count, const Out& out, long joff)
+                                             double base, double dt, long j0, int n, const Out& out, long joff)
 {
-    const long rest = count - j0;
-    const int n = rest < L ? (int)rest : L;
-    if (K == 1) sinusoid_rot_terms<L, 1>(a, f, phi, i, base, dt, j0, n, out, joff);
-    else if (KMAX >= 2 && K == 2) sinusoid_rot_terms<L, (KMAX >= 2 ? 2 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
-    else if (KMAX >= 3 && K == 3) sinusoid_rot_terms<L, (KMAX >= 3 ? 3 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
-    else if (KMAX >= 4 && K == 4) sinusoid_rot_terms<L, (KMAX >= 4 ? 4 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
+    if (K == 1) sinusoid_rot_terms<1>(a, f, phi, i, base, dt, j0, n, out, joff);
+    else if (KMAX >= 2 && K == 2) sinusoid_rot_terms<(KMAX >= 2 ? 2 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
+    else if (KMAX >= 3 && K == 3) sinusoid_rot_terms<(KMAX >= 3 ? 3 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
+    else if (KMAX >= 4 && K == 4) sinusoid_rot_terms<(KMAX >= 4 ? 4 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
     else
         for (int j = 0; j < n; ++j) out(j, sinusoid_value(a, f, phi, K, i, sample_time(base, dt, joff + j0 + j)));
 }
@@ -213,21 +210,19 @@ __device__ __forceinline__ void sinusoid_rot(const double* a, const double* f, c
 // registers follow the largest variant it contains.  Sample j of the run is
 // written at out(j) and taken at the time of sample joff + j0 + j (joff: the
 // index of the buffer's first sample on the whole horizon).
-template <int L, int KMAX, class Out>
+template <int KMAX, class Out>
 __device__ __forceinline__ void sinusoid_run(const double* a, const double* f, const double* phi, int K, int i,
-                                             double base, double dt, long j0, long count, const Out& out,
+                                             double base, double dt, long j0, int n, const Out& out,
                                              long joff = 0)
 {
-    const long rest = count - j0;
-    const int n = rest < L ? (int)rest : L;
     if (K == 1) {
-        sinusoid_run_terms<L, 1>(a, f, phi, i, base, dt, j0, n, out, joff);
+        sinusoid_run_terms<1>(a, f, phi, i, base, dt, j0, n, out, joff);
     } else if (KMAX >= 2 && K == 2) {
-        sinusoid_run_terms<L, (KMAX >= 2 ? 2 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
+        sinusoid_run_terms<(KMAX >= 2 ? 2 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
     } else if (KMAX >= 3 && K == 3) {
-        sinusoid_run_terms<L, (KMAX >= 3 ? 3 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
+        sinusoid_run_terms<(KMAX >= 3 ? 3 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
     } else if (KMAX >= 4 && K == 4) {
-        sinusoid_run_terms<L, (KMAX >= 4 ? 4 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
+        sinusoid_run_terms<(KMAX >= 4 ? 4 : 1)>(a, f, phi, i, base, dt, j0, n, out, joff);
     } else {
         for (int j = 0; j < n; ++j) out(j, sinusoid_value(a, f, phi, K, i, sample_time(base, dt, joff + j0 + j)));
     }

@@ -7,9 +7,17 @@
 
 namespace parode {
 
-// Samples per thread of the input-sampling kernels: one thread advances one
-// channel over a run of this many consecutive samples.
-constexpr int kSampleRun = 64;
+// Samples per thread of the input-sampling kernels (one thread advances one
+// channel over a run of consecutive samples), for `total` samples in all
+// channels: 64, which spreads the two sincos that start each term of a run
+// over many rotations, down to 8 where longer runs would leave the chip to a
+// few serial chains (16,386 samples: 16 us by runs of 64).
+inline int sample_run(long total)
+{
+    int run = 64;
+    while (run > 8 && total / run < 148L * 1024) run /= 2;
+    return run;
+}
 
 // Column addressing of the batched affine-level contraction:
 //   result(g, i) = sum_k P[i][k] * src(g, k) (+ acc(g, i))
@@ -310,6 +318,7 @@ struct SampleJob {
     const double *a = nullptr, *f = nullptr, *phi = nullptr;
     double base = 0, dt = 0;
     long count = 0;
+    int run = 64;  // samples per thread
 };
 struct ForcingJob {
     double* V = nullptr;
@@ -344,7 +353,7 @@ struct PhiJob {
 };
 void launch_phi_batch(const PhiJob* dJobs, int njobs, long max_elems, cudaStream_t s);
 // max_elems: the largest element count of a job (sizes the x dimension); for
-// the samples, runs of 32 samples x channels (one thread each).
+// the samples, runs of the jobs' length x channels (one thread each).
 // max_terms: the largest term count of the jobs' inputs
 void launch_samples_batch(const SampleJob* dJobs, int njobs, long max_elems, int max_terms, cudaStream_t s);
 void launch_forcing_batch(const ForcingJob* dJobs, int njobs, long max_elems, cudaStream_t s);

@@ -338,34 +338,34 @@ __global__ void k_swap_grouped(const LevelArgs* __restrict__ args)
     swap_body(a);
 }
 
-// One thread per (run of kSampleRun samples, channel); channels fastest.
+// One thread per (run of `run` samples, channel); channels fastest.
 template <int KMAX>
 __global__ void k_sinusoid_samples(double* U, int m, int K, const double* a, const double* f, const double* phi,
-                                   double base, double dt, long count, long joff)
+                                   double base, double dt, long count, long joff, int run)
 {
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long runs = (count + kSampleRun - 1) / kSampleRun;
+    const long runs = (count + run - 1) / run;
     if (e >= runs * m) return;
     const long r = e / m;
     const int i = (int)(e - r * m);
-    const long j0 = r * kSampleRun;
-    sinusoid_run<kSampleRun, KMAX>(a, f, phi, K, i, base, dt, j0, count, SampleOut64{U + j0 * m + i, m}, joff);
+    const long j0 = r * run;
+    sinusoid_run<KMAX>(a, f, phi, K, i, base, dt, j0, (int)min((long)run, count - j0), SampleOut64{U + j0 * m + i, m}, joff);
 }
 
 // The same samples as TF32 hi / lo planes (the tensor-core GEMMs' operands),
 // by the plain rotation (sinusoid_rot: the planes' own rounding is 2^-22).
 template <int KMAX>
 __global__ void k_sinusoid_planes(float* hi, float* lo, int m, int K, const double* a, const double* f,
-                                  const double* phi, double base, double dt, long count, long joff)
+                                  const double* phi, double base, double dt, long count, long joff, int run)
 {
     grid_dep_trigger();  // the response GEMMs may set up meanwhile (they wait for these samples)
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long runs = (count + kSampleRun - 1) / kSampleRun;
+    const long runs = (count + run - 1) / run;
     if (e >= runs * m) return;
     const long r = e / m;
     const int i = (int)(e - r * m);
-    const long j0 = r * kSampleRun;
-    sinusoid_rot<kSampleRun, KMAX>(a, f, phi, K, i, base, dt, j0, count,
+    const long j0 = r * run;
+    sinusoid_rot<KMAX>(a, f, phi, K, i, base, dt, j0, (int)min((long)run, count - j0),
                                    SampleOutSplit{hi + j0 * m + i, lo ? lo + j0 * m + i : nullptr, m}, joff);
 }
 
@@ -441,14 +441,14 @@ template <int KMAX>
 __global__ void k_samples_batch(const SampleJob* __restrict__ jobs)
 {
     const SampleJob J = jobs[blockIdx.y];
-    const long runs = (J.count + kSampleRun - 1) / kSampleRun;
+    const long runs = (J.count + J.run - 1) / J.run;
     const long total = runs * J.m;
     for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
         const long r = e / J.m;
         const int i = (int)(e - r * J.m);
-        const long j0 = r * kSampleRun;
-        sinusoid_run<kSampleRun, KMAX>(J.a, J.f, J.phi, J.K, i, J.base, J.dt, j0, J.count,
-                                       SampleOut64{J.U + j0 * J.m + i, J.m});
+        const long j0 = r * J.run;
+        sinusoid_run<KMAX>(J.a, J.f, J.phi, J.K, i, J.base, J.dt, j0, (int)min((long)J.run, J.count - j0),
+                           SampleOut64{J.U + j0 * J.m + i, J.m});
     }
 }
 
@@ -621,13 +621,14 @@ void launch_sinusoid_samples(double* U, int m, int K, const double* a, const dou
                              double base, double dt, long count, cudaStream_t s, long joff)
 {
     if (count <= 0 || m <= 0) return;
-    const long total = (count + kSampleRun - 1) / kSampleRun * m;
+    const int run = sample_run(count * m);
+    const long total = (count + run - 1) / run * m;
     const unsigned g = (unsigned)blocks_for(total, 256);
     switch (sample_kmax(K)) {
-    case 1: k_sinusoid_samples<1><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff); break;
-    case 2: k_sinusoid_samples<2><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff); break;
-    case 3: k_sinusoid_samples<3><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff); break;
-    default: k_sinusoid_samples<4><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff); break;
+    case 1: k_sinusoid_samples<1><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff, run); break;
+    case 2: k_sinusoid_samples<2><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff, run); break;
+    case 3: k_sinusoid_samples<3><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff, run); break;
+    default: k_sinusoid_samples<4><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff, run); break;
     }
     PARODE_CUDA(cudaGetLastError());
 }
@@ -636,13 +637,14 @@ void launch_sinusoid_planes(float* hi, float* lo, int m, int K, const double* a,
                             double base, double dt, long count, cudaStream_t s, long joff)
 {
     if (count <= 0 || m <= 0) return;
-    const long total = (count + kSampleRun - 1) / kSampleRun * m;
+    const int run = sample_run(count * m);
+    const long total = (count + run - 1) / run * m;
     const unsigned g = (unsigned)blocks_for(total, 256);
     switch (sample_kmax(K)) {
-    case 1: k_sinusoid_planes<1><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff); break;
-    case 2: k_sinusoid_planes<2><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff); break;
-    case 3: k_sinusoid_planes<3><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff); break;
-    default: k_sinusoid_planes<4><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff); break;
+    case 1: k_sinusoid_planes<1><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff, run); break;
+    case 2: k_sinusoid_planes<2><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff, run); break;
+    case 3: k_sinusoid_planes<3><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff, run); break;
+    default: k_sinusoid_planes<4><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff, run); break;
     }
     PARODE_CUDA(cudaGetLastError());
 }

@@ -167,7 +167,6 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
     const bool wide = Ns_ > 8 && Ns_ <= 64 && opt.path == kPathAuto && opt.precision == kMixed && opt.shards <= 1 &&
                       opt.shard == 0 && !opt.fault_withhold && mu_ > 0 && input_->kind == InputEntry::kSinusoid &&
                       input_->m >= mu_ && (long)mu_ * input_->K <= kExpandMaxPairs &&
-                      blocked_shape(Ns_, mu_, solver, &shape_) &&
                       !expand_shape(Ns_, mu_, input_->K, p_, nScan_, 6, &ext_.sh);
     if ((Ns_ > 64 && opt.path != kPathBlocked && opt.path != kPathBlockedSweep) || wide) {
         // scan dimensions above 64: the batch engine's one-system form (the
@@ -203,7 +202,9 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         const double bytes = (double)nScan_ * Np_ * Np_ * 8.0 + (double)general_scan_bytes(Np_, nScan_);
         if (bytes > 24e9) throw Error(kNotEnoughResources, "the general scan holds a copy of Phi per step");
     } else {
-        const bool can_block = blocked_shape(Ns_, mu_, solver, &shape_);
+        // (the response leaf does not hold the samples on chip as the sweeps
+        // do: any number of inputs)
+        const bool can_block = blocked_shape(Ns_, opt.path == kPathBlockedSweep ? mu_ : std::min(mu_, 1), solver, &shape_);
         if (opt.path >= kPathBlocked && !can_block)
             throw Error(kInvalidArgument, "the blocked path supports scan dimensions up to 64");
         if (opt.path != kPathLevel && can_block) path_ = kPathBlocked;
@@ -230,38 +231,36 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         // FP64 sin evaluations would compete with the scan for issue slots)
         gen_ = false;
         stage_bytes_ = blocked_leaf_stage_bytes(shape_, sys.n, mu_, p_, solver);
-        // the leaf as GEMMs with the block response matrix (kernels_br.cu)
-        // when that costs fewer flops than the in-block sweeps: about
-        // 2 (B p + NP) K / B per step against 4 NP^2.  The mixed form runs the
-        // aggregate and output-window products on the tensor cores (3xTF32)
-        // and keeps the initial-state part of the outputs in FP64.
+        // sampled inputs: the leaf as GEMMs with the block response matrix
+        // (kernels_br.cu), unless the in-block sweeps are forced.  Blocks of 16
+        // steps are at or near the best length of every scan dimension measured
+        // (8 states, 4096 steps FP64: 43 us with 16, 47 with 32, 86 with the
+        // sweeps; 32 states, 3e5 steps mixed, user input: 84 us with 16, 96 with
+        // 64, 340 with the sweeps); 8 steps where a short horizon leaves few
+        // blocks of a 64-state RK4 system (20,000 steps FP64: 76 against 88 us).
+        // The mixed form runs the aggregate and output-window products on the
+        // tensor cores (3xTF32) and keeps the initial-state part of the outputs
+        // in FP64; at scan dimensions up to 8 it stays in FP64, as ever.
         if (mu_ > 0 && opt.path != kPathBlockedSweep) {
-            const int K = response_window(solver, shape_.B, mu_);
-            const double resp = 2.0 * ((double)shape_.B * p_ + Np_) * K / shape_.B;
-            const double sweeps = 4.0 * Np_ * Np_;
-            if (opt.path == kPathBlockedResponse || resp < 0.5 * sweeps) {
-                br_ = true;
-                br_tc_ = opt.precision != kFP64;
-                one_pass_ = opt.precision == kTF32;
-                if (br_tc_) precision_used_ = one_pass_ ? kTF32 : kMixed;
-                // a block length forced by the caller or measured for this
-                // class of systems (tuner.h) replaces the shape's default
-                int Rt = opt.force_log2_block;
-                if (Rt < 2) Rt = tuned_log2_block(tune_class(solver, Ns_, mu_, p_, nScan_, opt.precision));
-                if (Rt >= 2 && Rt <= 7) {
-                    while (Rt > 2 && (1L << Rt) / 2 >= nScan_) --Rt;
-                    shape_.R = Rt;
-                    shape_.B = 1 << Rt;
-                }
-                const int Kb = response_window(solver, shape_.B, mu_);
-                brK_ = Kb;
-                brKpad_ = (Kb + 1) & ~1;
-                nblocks_ = (nScan_ + shape_.B - 1) / shape_.B;
-                // the chunked carry over blocks reads P_R .. P_{R + 4 h + 3}
-                levels_ = shape_.R + chunk_carry_table_levels(nblocks_);
-            }
+            br_ = true;
+            br_tc_ = opt.precision != kFP64 && (shape_.NP > 8 || opt.path == kPathBlockedResponse);
+            one_pass_ = br_tc_ && opt.precision == kTF32;
+            if (br_tc_) precision_used_ = one_pass_ ? kTF32 : kMixed;
+            // a block length forced by the caller or measured for this class of
+            // systems (tuner.h) replaces the default
+            int Rt = opt.force_log2_block;
+            if (Rt < 2) Rt = tuned_log2_block(tune_class(solver, Ns_, mu_, p_, nScan_, opt.precision));
+            if (Rt < 2 || Rt > 7) Rt = solver == kRK4 && shape_.NP == 64 && nScan_ < 32768 ? 3 : 4;
+            while (Rt > 2 && (1L << Rt) / 2 >= nScan_) --Rt;
+            shape_.R = Rt;
+            shape_.B = 1 << Rt;
+            brK_ = response_window(solver, shape_.B, mu_);
+            brKpad_ = (brK_ + 1) & ~1;
+            nblocks_ = (nScan_ + shape_.B - 1) / shape_.B;
+            // the chunked carry over blocks reads P_R .. P_{R + 4 h + 3}
+            levels_ = shape_.R + chunk_carry_table_levels(nblocks_);
         }
-        // otherwise the mixed form runs the in-block sweeps on the tensor
+        // with the sweeps the mixed form runs them on the tensor
         // cores (3xTF32) when the shape allows it, with the longest tile that
         // fits its shared-memory layout; otherwise the solve stays in FP64
         if (opt.precision != kFP64 && !br_) {
@@ -1228,8 +1227,12 @@ void Plan::execute_response(double* Y, cudaStream_t s)
 
 void Plan::solve_to_host(double* yd, float* yf)
 {
+    // ranges pay once y is long enough for its copy to matter against four
+    // launches and four copies (8 MB: 0.15 ms over the link; 2 MB of floats to
+    // pageable memory took 0.24 ms in four copies, 0.15 in one)
+    constexpr double kRangeBytes = 8e6;
     void* y = yf ? (void*)yf : (void*)yd;
-    if (!y || batch_ || shards_ > 1 || path_ != kPathBlocked || !(br_ || ex_) || profiling_ || nblocks_ < 8) {
+    if (!y || (yf ? 4.0 : 8.0) * (double)nOut_ * p_ < kRangeBytes || batch_ || shards_ > 1 || path_ != kPathBlocked || !(br_ || ex_) || profiling_ || nblocks_ < 8) {
         execute(nullptr, nullptr);
         if (yf)
             get_output_f32(nullptr, yf);
@@ -1285,6 +1288,13 @@ void Plan::solve_to_host(double* yd, float* yf)
     launches_ = launches;
     last_y_ = dY_;
     PARODE_CUDA(cudaStreamSynchronize(s));
+    check_status();
+}
+
+void Plan::check_status()
+{
+    // only the tensor-core kernels of the mixed forms have waits that can give up
+    if (!br_tc_ && !(path_ == kPathBlocked && !br_ && !ex_ && precision_used_ == kMixed)) return;
     int status = 0;
     PARODE_CUDA(cudaMemcpy(&status, dStatus_, sizeof(int), cudaMemcpyDeviceToHost));
     if (status != 0) throw Error(kDeviceError, "a device-side wait gave up (tensor-core completion not observed)");
@@ -1496,9 +1506,7 @@ void Plan::get_output_f32(float* t, float* y)
     }
     if (t) time_vector_f(solver_, t0_, tEnd_, h_, t);
     PARODE_CUDA(cudaStreamSynchronize(stream_));
-    int status = 0;
-    PARODE_CUDA(cudaMemcpy(&status, dStatus_, sizeof(int), cudaMemcpyDeviceToHost));
-    if (status != 0) throw Error(kDeviceError, "a device-side wait gave up (tensor-core completion not observed)");
+    check_status();
 }
 
 void Plan::get_output(double* t, double* y)
@@ -1532,9 +1540,7 @@ void Plan::get_output(double* t, double* y)
         time_vector(solver_, t0_, tEnd_, h_, t);
     }
     PARODE_CUDA(cudaStreamSynchronize(stream_));
-    int status = 0;
-    PARODE_CUDA(cudaMemcpy(&status, dStatus_, sizeof(int), cudaMemcpyDeviceToHost));
-    if (status != 0) throw Error(kDeviceError, "a device-side wait gave up (tensor-core completion not observed)");
+    check_status();
 }
 
 }  // namespace parode

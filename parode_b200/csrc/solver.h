@@ -142,6 +142,7 @@ private:
     int response_head(cudaStream_t s);  // inputs, aggregates, carry; returns the launches
     void response_outputs(double* Y, long c0, long c1, cudaStream_t s);  // blocks [c0, c1)
     void state_part(double* Y, long c0, long c1, cudaStream_t s);
+    void check_status();  // after a synchronise: throws when a device-side wait gave up
     void setup_shard(const PlanOptions& opt);
     void fill_inputs(cudaStream_t s);
 
