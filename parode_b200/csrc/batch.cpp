@@ -1337,6 +1337,9 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             b.K1 = q.Kpad;
             b.src2 = q.V;
             b.src2_gs = q.Np;
+            b.tri_p = q.p;  // y_j reads samples up to 2 j (RK4), j + 3 (ABM)
+            b.tri_base = (q.solver == kRK4 ? 1 : 4) * q.mu;
+            b.tri_step = (q.solver == kRK4 ? 2 : 1) * q.mu;
             b.ncols = q.nblocks;
             b.src_cols = 0;
             b.dst = q.Y + (q.solver == kRK4 ? 0L : 3L * q.p);

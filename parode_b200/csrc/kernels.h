@@ -55,6 +55,10 @@ struct LevelArgs {
     int K1 = 0;
     const double* src2 = nullptr;
     long src2_gs = 0;
+    // Tiled kernel, K1 > 0: row r reads only the first tri_base + (r / tri_p)
+    // tri_step contraction indices below K1 (tri_p > 0; P is zero in the rest:
+    // a step's output reads no later sample of its block).
+    int tri_p = 0, tri_base = 0, tri_step = 0;
     // Tiled kernel: columns g >= src_cols (> 0) read a zero source, so their
     // results are acc or 0 (a zero padding written by the same launch).
     long src_cols = 0;
@@ -86,6 +90,12 @@ struct RespArgs {
 // tiled GEMM).
 bool launch_state_out(int NP, const double* W, long ld, int M, const double* X, const double* acc, double* Y, long gs,
                       long nblocks, long limit, int sms, cudaStream_t s);
+
+// The FP64 outputs of the block-response leaf for one system (the arguments
+// of launch_gemm_tiled, kernels_resp_f64.cu).  Returns false, launching
+// nothing, where a slice of W does not fit in shared memory or an operand is
+// not on 16-byte boundaries (the caller then uses the tiled GEMM).
+bool launch_resp_f64(const LevelArgs& a, int sms, cudaStream_t s);
 
 long resp_tc_tiles(const RespArgs& a);
 std::vector<long> resp_tc_ranges(const std::vector<RespArgs>& ents, int ctas);

@@ -136,84 +136,146 @@ __device__ void affine_level_body(const LevelArgs& a, long tile, int CW, int KS,
 // The result must not alias the source (the down-sweep swaps first).
 // kTileKC: the source columns are K-contiguous (src_ks == 1, the sweeps);
 // otherwise N-contiguous (src_gs == 1, the power-table squaring).
+// K-contiguous, products 2 c + u of a K chunk of 8 take the K indices
+// 8 c + 2 t + u (A and B alike), so a lane's fragments are 16-byte loads, two
+// products each; the 16-byte chunks of odd rows are stored XOR 4 (conflict-free
+// without padding).  N-contiguous, the K order stays 8 c + 4 u + t: squared in
+// the other order, the powers of ABM companion matrices lost up to a factor of
+// 14 in accuracy (outputs 2e-15 -> 3e-14).  The 4 warps of a row half sit on
+// the 4 sub-partitions, so a half whose rows read fewer K (tri_p) leaves none
+// idle.  Fragments are loaded a chunk ahead and the copies' addresses set up
+// once per tile: the 2^20-step RK4 aggregates (2.2 GFLOP, a floor of 60 us)
+// took 90 us without, 82 with; ABM outputs of K = 608 (5.1 GFLOP) 182 and 172.
 // ---------------------------------------------------------------------------
 
 constexpr int kTM = 64, kTN = 64, kTK = 32, kTStages = 3;
-constexpr int kLdA = kTK + 4;   // A tile [64 rows][36]: rows g and g+4 of a fragment in distinct bank halves
-constexpr int kLdBk = kTK + 4;  // B tile, K-contiguous: [64 cols][36]
-constexpr int kLdBn = kTN + 4;  // B tile, N-contiguous: [32 k][68]
-constexpr int kStageA = kTM * kLdA;
-constexpr int kStageB = (kTN * kLdBk > kTK * kLdBn) ? kTN * kLdBk : kTK * kLdBn;
+constexpr int kLdBn = kTN + 4;  // B tile, N-contiguous: [32 k][68]: rows t apart by 4 t mod 16 doubles
+constexpr int kStageA = kTM * kTK;
+constexpr int kStageB = (kTN * kTK > kTK * kLdBn) ? kTN * kTK : kTK * kLdBn;
 constexpr size_t kTiledSmem = (size_t)kTStages * (kStageA + kStageB) * sizeof(double);
 
-__device__ __forceinline__ void cp_async16(double* dst, const double* src, bool valid)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-    const int bytes = valid ? 16 : 0;  // 0: the 16 bytes are zero-filled and src is not read
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(src), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-template <bool kKC>
-__device__ void tiled_load(const LevelArgs& a, int m0, long n0, int k0, double* sA, double* sB)
+// Volatile, as the products are: a fragment's load stays where it is written.
+__device__ __forceinline__ double2 lds128(unsigned at)
 {
-    const int tid = threadIdx.x;
-    const int rows = level_rows(a), K = level_k(a);  // K even: a 2-double chunk is wholly in or out
-    const long scols = a.src_cols > 0 ? a.src_cols : a.ncols;
-    // A: 64 rows x 32 doubles = 1024 chunks of 16 bytes
+    double2 v;
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "r"(at) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ double lds64(unsigned at)
+{
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1];\n" : "=d"(v) : "r"(at) : "memory");
+    return v;
+}
+
+// Offset (doubles) of 16-byte chunk c of row r in a K-contiguous tile.
+__device__ __forceinline__ int tile_at(int r, int c) { return r * kTK + ((c ^ ((r & 1) << 2)) << 1); }
+
+// A thread's part of a slice's copies: 16-byte chunk tid & 15 of the A rows
+// (tid >> 4) + 16 q and, K-contiguous, of the same B columns; N-contiguous,
+// columns 2 (tid & 31) of the K rows (tid >> 5) + 8 q.  Set up once per tile.
+template <bool kKC>
+struct TiledLoad {
+    const double *pa, *pb, *pb2;
+    long lda16, ldb;   // pointer steps per q
+    unsigned sa, sb;   // shared byte offsets of q = 0 in a stage
+    unsigned okA, okB; // q's rows / columns inside the matrices
+    int K, K1, kc;     // kc: the thread's K index in a slice (A; K-contiguous B)
+
+    __device__ TiledLoad(const LevelArgs& a, int m0, long n0)
+    {
+        const int tid = threadIdx.x, rows = level_rows(a);
+        const long scols = a.src_cols > 0 ? a.src_cols : a.ncols;
+        const int r = tid >> 4;
+        K = level_k(a);  // even: a 2-double chunk is wholly in or out
+        K1 = a.K1;
+        kc = (tid & 15) * 2;
+        okA = okB = 0;
+        pa = a.P + (long)(m0 + r) * a.ldp + kc;
+        lda16 = 16 * a.ldp;
+        sa = 8 * tile_at(r, tid & 15);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int c = tid + q * 256;
-        const int r = c >> 4, kc = (c & 15) * 2;
-        const bool ok = (m0 + r < rows) && (k0 + kc < K);
-        const double* src = ok ? a.P + (long)(m0 + r) * a.ldp + k0 + kc : a.P;
-        cp_async16(sA + r * kLdA + kc, src, ok);
-    }
-    if (kKC) {
-        // B: 64 columns x 32 doubles of K, each column contiguous in K
+        for (int q = 0; q < 4; ++q)
+            if (m0 + r + 16 * q < rows) okA |= 1u << q;
+        pb2 = nullptr;
+        if (kKC) {
+            pb = a.src + (n0 + r) * a.src_gs + kc;
+            if (K1 > 0) pb2 = a.src2 + (n0 + r) * a.src2_gs + kc - K1;
+            ldb = 16 * a.src_gs;
+            sb = sa;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int c = tid + q * 256;
-            const int col = c >> 4, kc = (c & 15) * 2;
-            const long g = n0 + col;
-            const int k = k0 + kc;
-            const bool ok = (g < scols) && (k < K);
-            const double* src = !ok ? a.src
-                                    : (a.K1 > 0 && k >= a.K1) ? a.src2 + g * a.src2_gs + (k - a.K1)
-                                                              : a.src + g * a.src_gs + k;
-            cp_async16(sB + col * kLdBk + kc, src, ok);
+            for (int q = 0; q < 4; ++q)
+                if (n0 + r + 16 * q < scols) okB |= 1u << q;
+        } else {
+            const int kr = tid >> 5, nc = (tid & 31) * 2;
+            pb = a.src + (long)kr * a.src_ks + n0 + nc;
+            ldb = 8 * a.src_ks;
+            sb = 8 * (kr * kLdBn + nc);
+            if (n0 + nc < scols) okB = 15;
         }
-    } else {
-        // B: 32 rows of K x 64 columns, each row contiguous in N
+    }
+    // slice k0 .. k0 + 31 into the stage at shared addresses A, B
+    __device__ __forceinline__ void operator()(const LevelArgs& a, int k0, unsigned A, unsigned B) const
+    {
+        const bool kin = k0 + kc < K;
+        const double* p = pa + k0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int c = tid + q * 256;
-            const int kr = c >> 5, nc = (c & 31) * 2;
-            const long g = n0 + nc;
-            const bool ok = (g < scols) && (k0 + kr < K);
-            const double* src = ok ? a.src + (long)(k0 + kr) * a.src_ks + g : a.src;
-            cp_async16(sB + kr * kLdBn + nc, src, ok);
+        for (int q = 0; q < 4; ++q) copy(A + sa + q * 16 * kTK * 8, p + q * lda16, kin && (okA >> q & 1), a.P);
+        if (kKC) {
+            const bool two = K1 > 0 && k0 + kc >= K1;
+            const double* b = (two ? pb2 : pb) + k0;
+            const long step = two ? 16 * a.src2_gs : ldb;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) copy(B + sb + q * 16 * kTK * 8, b + q * step, kin && (okB >> q & 1), a.src);
+        } else {
+            const double* b = pb + (long)k0 * a.src_ks;
+            const int kr = threadIdx.x >> 5;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                copy(B + sb + q * 8 * kLdBn * 8, b + q * ldb, k0 + kr + 8 * q < K && (okB >> q & 1), a.src);
         }
     }
+    // 16 bytes, or zeros (nothing read)
+    __device__ __forceinline__ static void copy(unsigned dst, const double* src, bool in, const double* any)
+    {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(in ? src : any), "r"(in ? 16 : 0)
+                     : "memory");
+    }
+};
+
+// Contraction indices below K1 that rows up to r read.
+__device__ __forceinline__ int tri_limit(const LevelArgs& a, int r)
+{
+    const int rows = level_rows(a);
+    if (a.tri_p <= 0) return a.K1;
+    return min(a.K1, a.tri_base + (min(r, rows - 1) / a.tri_p) * a.tri_step);
 }
 
 template <bool kKC>
 __device__ void tiled_level_body(const LevelArgs& a, long tile, double* smem)
 {
-    const int rows = level_rows(a);
+    const int rows = level_rows(a), K = level_k(a);
     const int mt = (rows + kTM - 1) / kTM;
     const int m0 = (int)(tile % mt) * kTM;
     const long n0 = (tile / mt) * kTN;
-    double* sA = smem;
-    double* sB = smem + kTStages * kStageA;
+    const unsigned sA = (unsigned)__cvta_generic_to_shared(smem), sB = sA + 8 * kTStages * kStageA;
+    const TiledLoad<kKC> fetch(a, m0, n0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wm = warp & 1, wn = warp >> 1;
+    const int wm = warp >> 2, wn = warp & 3;
     const int gq = lane >> 2, tq = lane & 3;
     // a tile wholly beyond the source columns only writes acc (or zeros)
     const long scols = a.src_cols > 0 ? a.src_cols : a.ncols;
-    const int nk = n0 >= scols ? 0 : (level_k(a) + kTK - 1) / kTK;
+    const int all = n0 >= scols ? 0 : (K + kTK - 1) / kTK;
+    // slices [0, n1) and [s2, all): those between hold only zeros of these rows
+    const int n1 = min(all, (tri_limit(a, m0 + kTM - 1) + kTK - 1) / kTK), s2 = max(n1, min(all, a.K1 / kTK));
+    const int nk = n1 + all - s2;
+    const int wlim = tri_limit(a, m0 + wm * 32 + 31);  // this warp's rows
+    auto slice = [&](int i) { return (i < n1 ? i : s2 + i - n1) * kTK; };
 
     double acc[4][2][2];
 #pragma unroll
@@ -223,34 +285,65 @@ __device__ void tiled_level_body(const LevelArgs& a, long tile, double* smem)
 
 #pragma unroll
     for (int s = 0; s < kTStages - 1; ++s) {
-        if (s < nk) tiled_load<kKC>(a, m0, n0, s * kTK, sA + s * kStageA, sB + s * kStageB);
+        if (s < nk) fetch(a, slice(s), sA + 8 * s * kStageA, sB + 8 * s * kStageB);
         cp_async_commit();
     }
+    int st = 0;
     for (int kt = 0; kt < nk; ++kt) {
         cp_async_wait<kTStages - 2>();
         __syncthreads();
         {
-            const int nx = kt + kTStages - 1;
-            const int st = nx % kTStages;
-            if (nx < nk) tiled_load<kKC>(a, m0, n0, nx * kTK, sA + st * kStageA, sB + st * kStageB);
+            const int nx = kt + kTStages - 1, sx = st == 0 ? kTStages - 1 : st - 1;
+            if (nx < nk) fetch(a, slice(nx), sA + 8 * sx * kStageA, sB + 8 * sx * kStageB);
             cp_async_commit();
         }
-        const double* A = sA + (kt % kTStages) * kStageA;
-        const double* B = sB + (kt % kTStages) * kStageB;
-#pragma unroll
-        for (int kk = 0; kk < kTK; kk += 4) {
-            double af[4], bf[2];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) af[i] = A[(wm * 32 + i * 8 + gq) * kLdA + kk + tq];
+        const unsigned As = sA + 8 * st * kStageA, Bs = sB + 8 * st * kStageB;
+        st = st + 1 == kTStages ? 0 : st + 1;
+        const int k0 = slice(kt);
+        auto at64 = [&](unsigned base, int r, int k) { return lds64(base + 8 * (tile_at(r, k >> 1) + (k & 1))); };
+        auto load = [&](int c, double2 (&af)[4], double2 (&bf)[2]) {
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int col = wn * 16 + j * 8 + gq;
-                bf[j] = kKC ? B[col * kLdBk + kk + tq] : B[(kk + tq) * kLdBn + col];
+                if (kKC) bf[j] = lds128(Bs + 8 * tile_at(col, 4 * c + tq));
+                else bf[j] = make_double2(lds64(Bs + 8 * ((8 * c + tq) * kLdBn + col)), lds64(Bs + 8 * ((8 * c + 4 + tq) * kLdBn + col)));
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = wm * 32 + i * 8 + gq;
+                if (kKC) af[i] = lds128(As + 8 * tile_at(r, 4 * c + tq));
+                else af[i] = make_double2(at64(As, r, 8 * c + tq), at64(As, r, 8 * c + 4 + tq));
+            }
+        };
+        auto products = [&](const double2 (&af)[4], const double2 (&bf)[2]) {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 2; ++j) dmma_m8n8k4(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+                for (int j = 0; j < 2; ++j) dmma_m8n8k4(acc[i][j][0], acc[i][j][1], af[i].x, bf[j].x);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) dmma_m8n8k4(acc[i][j][0], acc[i][j][1], af[i].y, bf[j].y);
+        };
+        double2 a0[4], b0[2], a1[4], b1[2];
+        if (k0 + kTK <= K && (k0 + kTK <= wlim || k0 >= a.K1)) {
+            // fragments one chunk ahead of their products
+            load(0, a0, b0);
+            load(1, a1, b1);
+            products(a0, b0);
+            load(2, a0, b0);
+            products(a1, b1);
+            load(3, a1, b1);
+            products(a0, b0);
+            products(a1, b1);
+        } else {  // the last slice, or one that these rows read in part or not at all
+            for (int c = 0; c < kTK / 8; ++c) {
+                const int k = k0 + 8 * c;
+                if (k < K && (k < wlim || k + 8 > a.K1)) {
+                    load(c, a0, b0);
+                    products(a0, b0);
+                }
+            }
         }
     }
     cp_async_wait<0>();

@@ -1120,6 +1120,10 @@ LevelArgs Plan::response_out_args(double* Y) const
     h.K1 = brKpad_;
     h.src2 = dG_;
     h.src2_gs = Np_;
+    // y_j reads samples up to 2 j (RK4), j + 3 (ABM)
+    h.tri_p = p_;
+    h.tri_base = (solver_ == kRK4 ? 1 : 4) * mu_;
+    h.tri_step = (solver_ == kRK4 ? 2 : 1) * mu_;
     h.dst = Y + ybase * p_;
     h.dst_gs = (long)shape_.B * p_;
     h.dst_limit = nScan_ * p_;
@@ -1210,7 +1214,7 @@ void Plan::response_outputs(double* Y, long c0, long c1, cudaStream_t s)
     h.dst += c0 * h.dst_gs;
     h.dst_limit -= c0 * h.dst_gs;
     h.ncols = c1 - c0;
-    launch_gemm_tiled(h, s);
+    if (!launch_resp_f64(h, sms_, s)) launch_gemm_tiled(h, s);
 }
 
 void Plan::execute_response(double* Y, cudaStream_t s)
