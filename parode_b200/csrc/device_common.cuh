@@ -98,6 +98,75 @@ __device__ __forceinline__ double sample_time(double base, double dt, long j)
     return __dadd_rn(base, __dmul_rn(dt, (double)j));
 }
 
+// A run of samples by Reinsch's recurrence, for nominal steps |dl| <= 1 and
+// arguments below 1e7 (else false, nothing written): S_j = amp sin(a0 + j dl)
+// advances as D <- D - 4 sin^2(dl / 2) S, S <- S + D, two FP64 operations a
+// term; the argument is formed rounded, as sinusoid_value rounds it, and its
+// difference e from a0 + j dl (the roundings of t_j and of the argument, below
+// 1e-8) enters to first order as amp cos(a0 + j dl) e, whose cosine comes from
+// a rotation in FP32 (its relative error of 1e-5 is 1e-13 of e's bound; the
+// neglected e^2 / 2 is below 1e-16).  7 FP64 operations a term instead of
+// sinusoid_run_terms' 14: the sampler is bound by the FP64 pipe.
+template <int KT, class Out>
+__device__ __forceinline__ bool sinusoid_run_reinsch(const double* a, const double* f, const double* phi, int i,
+                                                     double base, double dt, long j0, int n, const Out& out, long joff)
+{
+    const double two_pi = 6.283185307179586476925286766559;
+    double w[KT], ph[KT], a0[KT], dl[KT];
+    const double tl = sample_time(base, dt, joff + j0 + n);
+    bool fit = true;
+#pragma unroll
+    for (int q = 0; q < KT; ++q) {
+        w[q] = __dmul_rn(two_pi, f[i * KT + q]);
+        ph[q] = phi[i * KT + q];
+        a0[q] = __dadd_rn(__dmul_rn(w[q], sample_time(base, dt, joff + j0)), ph[q]);
+        dl[q] = __dmul_rn(w[q], dt);
+        fit = fit && fabs(dl[q]) <= 1.0 && fabs(a0[q]) < 1e7 && fabs(w[q] * tl) < 1e7;
+    }
+    if (!fit) return false;
+    double S[KT], D[KT], kap[KT];
+    float s32[KT], c32[KT], sd[KT], cd[KT];
+#pragma unroll
+    for (int q = 0; q < KT; ++q) {
+        const double amp = a[i * KT + q];
+        double si, co, sh, ch;
+        sincos(a0[q], &si, &co);
+        sincos(0.5 * dl[q], &sh, &ch);
+        kap[q] = 4.0 * sh * sh;
+        S[q] = amp * si;
+        D[q] = 2.0 * amp * sh * (co * ch - si * sh);  // S_1 - S_0
+        s32[q] = (float)S[q];
+        c32[q] = (float)(amp * co);
+        sd[q] = (float)(2.0 * sh * ch);
+        cd[q] = (float)(1.0 - 2.0 * sh * sh);
+    }
+    double v = 0.0;
+#pragma unroll
+    for (int q = 0; q < KT; ++q) v += S[q];
+    if (n > 0) out(0, v);
+    double jd = 0.0, idx = (double)(joff + j0);
+    for (int j = 1; j < n; ++j) {
+        jd += 1.0;
+        const double t = __dadd_rn(base, __dmul_rn(dt, idx + jd));  // sample_time, the index exact in FP64
+        float corr = 0.f;
+        v = 0.0;
+#pragma unroll
+        for (int q = 0; q < KT; ++q) {
+            const double arg = __dadd_rn(__dmul_rn(w[q], t), ph[q]);
+            const float e = (float)fma(-jd, dl[q], arg - a0[q]);
+            S[q] += D[q];
+            D[q] = fma(-kap[q], S[q], D[q]);
+            const float cn = fmaf(c32[q], cd[q], -(s32[q] * sd[q]));
+            s32[q] = fmaf(s32[q], cd[q], c32[q] * sd[q]);
+            c32[q] = cn;
+            corr = fmaf(cn, e, corr);
+            v += S[q];
+        }
+        out(j, v + (double)corr);
+    }
+    return true;
+}
+
 // Samples j0 .. j0 + n - 1 of channel i of the sum-of-sinusoid input, into out[(j - j0) * stride]: the values sinusoid_value
 // gives, at a fraction of its cost.  Every argument is rounded exactly as
 // sinusoid_value rounds it; each term starts from sincos at j0 and advances
@@ -119,6 +188,7 @@ __device__ __forceinline__ void sinusoid_run_terms(const double* a, const double
                                                    double base, double dt, long j0, int n, const Out& out,
                                                    long joff)
 {
+    if (sinusoid_run_reinsch<KT>(a, f, phi, i, base, dt, j0, n, out, joff)) return;
     const double two_pi = 6.283185307179586476925286766559;
     double w[KT], ph[KT], amp[KT], prev[KT], s[KT], c[KT], dl[KT], sdl[KT], cdl[KT];
     double v = 0.0;
