@@ -1058,9 +1058,10 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             long tiles = 0, swap_elems = 0;
             size_t smem = 0;
         };
+        enum class Narrow { kNone, kTiled, kAll };  // the entries the narrow kernel may take: none, Np > 64, all
         struct PreparedLevel {
             std::vector<PreparedGroup> groups;
-            std::vector<LevelArgs> tc;
+            std::vector<LevelArgs> tc, narrow;
             std::vector<unsigned char> maps;
             std::vector<long> tc_start, tc_ranges;
             long tc_tiles = 0;
@@ -1088,11 +1089,23 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             P.tc_ctas = (int)std::min<long>(sms_, P.tc_tiles);
             P.tc_ranges = level_tc_ranges(P.tc, P.tc_ctas);
         };
-        auto prepare = [&](const std::vector<std::pair<int, LevelArgs>>& ents, int l) {
-            // group by (config id, CW); entries keep the original form for the
+        auto prepare = [&](const std::vector<std::pair<int, LevelArgs>>& ents, int l, Narrow narrow) {
+            // group by config id; entries keep the original form for the
             // swap of a tiled down-sweep and the stored form for the contraction
             PreparedLevel P;
-            std::vector<std::pair<int, int>> keys;
+            std::vector<int> keys;
+            // up to 32 columns, a narrow CTA's own width, go to the narrow
+            // kernel; up to 512 when the level's tiles would leave SMs idle (one
+            // large system, NP = 512, 64 columns: 8 tiles of 64 x 64, 19 us,
+            // against 128 narrow CTAs)
+            auto may_narrow = [&](const LevelArgs& a) {
+                return (narrow == Narrow::kAll || (narrow == Narrow::kTiled && a.Np > 64)) && a.ncols > 0 &&
+                       a.src_ks == 1 && a.dst_is == 1 && !a.cpy && a.K1 == 0 && a.dst_limit < 0 && a.src_cols == 0;
+            };
+            long ntiles = 0;
+            for (const auto& e : ents)
+                if (may_narrow(e.second)) ntiles += level_tiles(level_config(e.second), e.second);
+            const long cap = ntiles < sms_ ? 512 : 32;
             // mixed form: levels below the top four of a system run on the
             // tensor cores (3xTF32); the top four, where high powers of Phi
             // amplify rounding, stay FP64
@@ -1112,11 +1125,14 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
                     continue;
                 }
                 LevelConfig c = level_config(e.second);
-                std::pair<int, int> key(c.id, c.CW);
+                if (may_narrow(e.second) && e.second.ncols <= cap) {
+                    P.narrow.push_back(e.second);
+                    continue;
+                }
                 size_t g = 0;
-                while (g < keys.size() && keys[g] != key) ++g;
+                while (g < keys.size() && keys[g] != c.id) ++g;
                 if (g == keys.size()) {
-                    keys.push_back(key);
+                    keys.push_back(c.id);
                     P.groups.emplace_back();
                     P.groups.back().cfg = c;
                 }
@@ -1125,8 +1141,13 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
                 if (c.id >= 5 && e.second.cpy) G.swaps.push_back(e.second);
             }
             for (PreparedGroup& G : P.groups) {
+                if (G.cfg.id == 5 || G.cfg.id == 6) {
+                    long tiles = 0;
+                    for (const LevelArgs& a : G.stored) tiles += level_tiles(G.cfg, a);
+                    if (level_few_tiles(tiles)) G.cfg = level_small(G.cfg);
+                }
                 for (const LevelArgs& a : G.stored) {
-                    LevelConfig c = level_config(a);
+                    const LevelConfig c = G.cfg.id >= 5 ? G.cfg : level_config(a);
                     G.start.push_back(G.tiles);
                     G.tiles += level_tiles(c, a);
                     G.smem = std::max(G.smem, c.smem);
@@ -1165,11 +1186,24 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
                 }
                 out.push_back(gl);
             }
+            if (!P.narrow.empty()) {
+                GroupedLaunch gl;
+                gl.cfg.id = kNarrowConfig;
+                gl.nent = (int)P.narrow.size();
+                std::vector<long> start;
+                for (const LevelArgs& a : P.narrow) {
+                    start.push_back(gl.tiles);
+                    gl.tiles += expand_narrow_tiles(a);
+                }
+                gl.args = reinterpret_cast<LevelArgs*>(base + jput(P.narrow.data(), sizeof(LevelArgs) * P.narrow.size()));
+                gl.start = reinterpret_cast<long*>(base + jput(start.data(), sizeof(long) * start.size()));
+                out.push_back(gl);
+            }
             if (!P.tc.empty()) out.push_back(emit_tc(P));
         };
         auto add_level = [&](std::vector<GroupedLaunch>& out, const std::vector<std::pair<int, LevelArgs>>& ents,
-                             int l) {
-            PreparedLevel P = prepare(ents, l);
+                             Narrow narrow) {
+            PreparedLevel P = prepare(ents, -1, narrow);
             emit(out, P);
         };
         auto make_tc = [&](std::vector<LevelArgs>& tc) {
@@ -1248,7 +1282,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
                 }
                 ents.push_back({i, a});
             }
-            T.P = prepare(ents, T.tc_level);
+            T.P = prepare(ents, T.tc_level, T.kind == 0 ? Narrow::kNone : Narrow::kTiled);
         });
         phase("jobs/levels prepared", false);
         for (LevelTask& T : tasks) emit(*T.out, T.P);
@@ -1350,12 +1384,12 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
                 throw Error(kInvalidArgument, "response GEMM shapes must be even");
         }
         if (!agg.empty()) {
-            add_level(rs_agg_, agg, -1);
-            add_level(rs_out_, out, -1);
+            add_level(rs_agg_, agg, Narrow::kNone);
+            add_level(rs_out_, out, Narrow::kNone);
         }
         if (!tcg.empty()) {
             rs_tc_.push_back(make_tc(tcg));
-            add_level(rs_state_, state, -1);
+            add_level(rs_state_, state, Narrow::kNone);
         }
         // radix expansion: the squaring steps (set-up), the doubling levels, the outputs
         if (!ex_.empty()) {
@@ -1383,52 +1417,21 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
                     const int c = expand_power_args(sys_[i].exj, l, two);
                     for (int k = 0; k < c; ++k) ents.push_back({i, two[k]});
                 }
-                add_level(ex_power_, ents, -1);
+                add_level(ex_power_, ents, Narrow::kNone);
             }
             ex_power_at_.push_back(ex_power_.size());
             for (int l = 0; l < lmax; ++l) {
-                // few columns go to the narrow kernel; so do up to 512 when the
-                // level's 64 x 64 tiles would leave SMs idle (one large system,
-                // NP = 512, 64 columns: 8 tiles, 19 us, against 128 narrow CTAs)
-                std::vector<std::pair<int, LevelArgs>> wide;
-                std::vector<LevelArgs> narrow;
-                long tiles = 0;
-                for (int i : ex_) {
-                    if (l >= sys_[i].levels) continue;
-                    const LevelArgs a = expand_level_args(sys_[i].exj, l);
-                    tiles += level_tiles(level_config(a), a);
-                    if (a.ncols <= 32) narrow.push_back(a);
-                    else wide.push_back({i, a});
-                }
-                if (tiles < sms_) {
-                    std::vector<std::pair<int, LevelArgs>> rest;
-                    for (auto& e : wide) {
-                        if (e.second.ncols <= 512) narrow.push_back(e.second);
-                        else rest.push_back(e);
-                    }
-                    wide.swap(rest);
-                }
-                add_level(ex_level_, wide, -1);
-                if (!narrow.empty()) {
-                    GroupedLaunch gl;
-                    gl.cfg.id = kNarrowConfig;
-                    gl.nent = (int)narrow.size();
-                    std::vector<long> start;
-                    for (const LevelArgs& a : narrow) {
-                        start.push_back(gl.tiles);
-                        gl.tiles += expand_narrow_tiles(a);
-                    }
-                    gl.args = reinterpret_cast<LevelArgs*>(base + jput(narrow.data(), sizeof(LevelArgs) * narrow.size()));
-                    gl.start = reinterpret_cast<long*>(base + jput(start.data(), sizeof(long) * start.size()));
-                    ex_level_.push_back(gl);
-                }
+                std::vector<std::pair<int, LevelArgs>> ents;
+                for (int i : ex_)
+                    if (l < sys_[i].levels) ents.push_back({i, expand_level_args(sys_[i].exj, l)});
+                add_level(ex_level_, ents, Narrow::kAll);
             }
             std::vector<std::pair<int, LevelArgs>> outs;
             for (int i : ex_) {
                 const Sys& q = sys_[i];
                 outs.push_back({i, expand_out_args(q.exj, q.Y + (q.solver == kRK4 ? 0L : 3L * q.p), q.nScan * (long)q.p)});
             }
-            add_level(ex_out_, outs, -1);
+            add_level(ex_out_, outs, Narrow::kNone);
         }
         nZero_ = (int)zero.size();
         if (nZero_ > 0) dZero_ = reinterpret_cast<CopyJob*>(base + jput(zero.data(), sizeof(CopyJob) * zero.size()));
@@ -1526,7 +1529,22 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
     // mixed form, the splits of the tensor-core operands depend on Phi alone:
     // formed here with Phi, once per batch, like the rest of the discretisation
     for (const Bucket& bk : buckets_) launch_batch_stage(0, bk.sh, bk.launch, stream_);
-    for (const GroupedLaunch& g : ls_power_) launch_grouped(g, stream_);
+    const int nforks = (int)buckets_.size() + (lv.empty() ? 0 : 1);
+    two_chains_ = false;
+    {
+        // the small systems' launches (one CTA owns all rows) and the large ones'
+        bool small = false, large = false;
+        for (const auto* list : {&ls_power_, &ls_up_, &ls_down_})
+            for (const GroupedLaunch& g : *list) (g.cfg.id == 0 ? small : large) = true;
+        two_chains_ = small && large;
+    }
+    forks_.resize(nforks + two_chains_, nullptr);
+    events_.resize(forks_.size() + 1 + two_chains_, nullptr);
+    for (auto& e : events_) PARODE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    launch_chains(stream_, {&ls_power_}, [&] {
+        // after the large chain's launches: its kernels run meanwhile (a stream takes about 50 us)
+        for (auto& f : forks_) PARODE_CUDA(cudaStreamCreateWithFlags(&f, cudaStreamNonBlocking));
+    });
     if (!ex_.empty()) {
         const int ne = (int)ex_.size();
         launch_expand_init(dEx_, ne, exMaxHq_, exMaxInit_, stream_);
@@ -1541,11 +1559,6 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
     phase("responses", true);
     for (int k = 0; k < nSplit_; k += 65535)
         launch_level_split(dSplit_ + k, std::min(65535, nSplit_ - k), maxSplitElems_, stream_);
-    const int nforks = (int)buckets_.size() + (lv.empty() ? 0 : 1);
-    forks_.resize(nforks, nullptr);
-    for (auto& f : forks_) PARODE_CUDA(cudaStreamCreateWithFlags(&f, cudaStreamNonBlocking));
-    events_.resize(nforks + 1, nullptr);
-    for (auto& e : events_) PARODE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     // no wait for the device here: executes are ordered after the set-up by
     // ready_, and the host images stay alive with the plan
     PARODE_CUDA(cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming));
@@ -1665,6 +1678,11 @@ void BatchPlan::build_responses()
             long tiles = 0;
             for (const LevelArgs& a : ents) {
                 if (level_config(a).id != st.cfg.id) throw Error(kDeviceError, "response tables: mixed tilings");
+                tiles += level_tiles(st.cfg, a);
+            }
+            if (level_few_tiles(tiles)) st.cfg = level_small(st.cfg);
+            tiles = 0;
+            for (const LevelArgs& a : ents) {
                 start.push_back(tiles);
                 tiles += level_tiles(st.cfg, a);
             }
@@ -1821,20 +1839,9 @@ void BatchPlan::enqueue(cudaStream_t s)
                 ++launches;
             }
         }
-        for (const GroupedLaunch& g : ls_up_) {
-            launch_grouped(g, fs);
-            ++launches;
-        }
+        // slot 0, the initial state, is read by the down-sweep only
         launch_copy_batch(dSeed_, nSeed_, maxSeed_, fs);
-        ++launches;
-        for (const GroupedLaunch& g : ls_down_) {
-            if (g.nswap > 0) {
-                launch_swap_grouped(g.swaps, g.nswap, g.swap_elems, fs);
-                ++launches;
-            }
-            launch_grouped(g, fs);
-            ++launches;
-        }
+        launches += 1 + launch_chains(fs, {&ls_up_, &ls_down_}, [] {});
         if (nls > 0) {
             launch_output_batch(dOutput_, nls, maxOutput_, fs);
             ++launches;
@@ -1861,6 +1868,40 @@ void BatchPlan::enqueue(cudaStream_t s)
         PARODE_CUDA(cudaStreamWaitEvent(s, events_[k + 1], 0));
     }
     launches_ = launches;
+}
+
+// Level launches, each list's in order.  Small systems (NP <= 64) and large ones
+// share none and neither chain's launches fill the chip: the small chain runs on
+// a stream of its own beside the large one, joined into s.  `before_small` runs
+// between the two chains' launches.
+int BatchPlan::launch_chains(cudaStream_t s, std::initializer_list<const std::vector<GroupedLaunch>*> lists,
+                             const std::function<void()>& before_small)
+{
+    int launches = 0;
+    auto run = [&](bool small, cudaStream_t cs) {
+        for (const auto* list : lists)
+            for (const GroupedLaunch& g : *list) {
+                if (two_chains_ && small != (g.cfg.id == 0)) continue;
+                if (g.nswap > 0) {
+                    launch_swap_grouped(g.swaps, g.nswap, g.swap_elems, cs);
+                    ++launches;
+                }
+                launch_grouped(g, cs);
+                ++launches;
+            }
+    };
+    if (two_chains_) PARODE_CUDA(cudaEventRecord(events_.back(), s));
+    run(false, s);
+    before_small();
+    if (two_chains_) {
+        cudaStream_t small = forks_.back();
+        cudaEvent_t join = events_[events_.size() - 2];
+        PARODE_CUDA(cudaStreamWaitEvent(small, events_.back(), 0));
+        run(true, small);
+        PARODE_CUDA(cudaEventRecord(join, small));
+        PARODE_CUDA(cudaStreamWaitEvent(s, join, 0));
+    }
+    return launches;
 }
 
 void BatchPlan::launch_grouped(const GroupedLaunch& g, cudaStream_t s)

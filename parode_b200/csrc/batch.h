@@ -29,6 +29,7 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <memory>
 #include <vector>
 
@@ -160,6 +161,8 @@ private:
     };
 
     void launch_grouped(const GroupedLaunch& g, cudaStream_t s);
+    int launch_chains(cudaStream_t s, std::initializer_list<const std::vector<GroupedLaunch>*> lists,
+                      const std::function<void()>& before_small);
     void build(std::vector<BatchSpec> specs, InputRegistry* inputs, const PlanOptions& opt);
     void release();  // idempotent: what the plan holds on the device goes back
     void build_responses();
@@ -178,6 +181,7 @@ private:
     cudaStream_t stream_ = nullptr;
     std::vector<cudaStream_t> forks_;
     std::vector<cudaEvent_t> events_;
+    bool two_chains_ = false;  // forks_.back() and the last two events belong to the small systems' chain
     // set-up finished on stream_ (an execute on another stream waits for it)
     cudaEvent_t ready_ = nullptr;
     // host images of the set-up copies, kept until the plan is destroyed so

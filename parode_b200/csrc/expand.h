@@ -102,8 +102,8 @@ void launch_expand_phases(const ExpandJob* dJobs, int njobs, long max_elems, cud
 LevelArgs expand_level_args(const ExpandJob& j, int l);
 LevelArgs expand_out_args(const ExpandJob& j, double* Y, long limit);
 
-// dst = P src for a few columns (K-contiguous, M and K multiples of 8, no
-// acc): 8 rows x 32 columns per CTA with K split over its warps, where the
+// dst = P src (+ acc, which may be dst) for a few columns (K-contiguous, rows
+// and K multiples of 8): 8 rows x 32 columns per CTA with K split over its warps, where the
 // 64 x 64 tiles would mostly multiply padding.
 long expand_narrow_tiles(const LevelArgs& a);
 void launch_expand_narrow(const LevelArgs* dArgs, const long* dStart, int nent, long tiles, cudaStream_t s);

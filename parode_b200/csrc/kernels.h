@@ -276,9 +276,10 @@ int launches_per_level();
 // ---------------------------------------------------------------------------
 
 // Tiling of the level contraction: entries of one grouped launch must share
-// the config id (and CW).  Ids 0..4: one CTA owns all Np rows of NC columns
-// (Np <= 64 here); ids 5/6: 64 x 64 tiles with cp.async staging (Np > 64;
-// 5: K-contiguous source columns, 6: N-contiguous, the power table).
+// the config id.  Ids 0..4: one CTA owns all Np rows of NC columns (Np <= 64
+// here: id 0, each entry with its own CW); ids 5/6: 64 x 64 tiles with cp.async
+// staging (Np > 64; 5: K-contiguous source columns, 6: N-contiguous, the power
+// table); 7/8: the same in 32 x 32 tiles (level_small).
 struct LevelConfig {
     int id = 0;     // template configuration
     int CW = 1;     // column warps
@@ -291,6 +292,12 @@ LevelConfig level_config(const LevelArgs& a);
 // the down-sweep, whose swap launch_swap_grouped performs beforehand).
 LevelArgs level_grouped_args(const LevelArgs& a);
 long level_tiles(const LevelConfig& c, const LevelArgs& stored);
+// A launch of this many 64 x 64 tiles takes 32 x 32 ones.  K = 512, us of the
+// 64 and the 32 form: 26.7 and 12.3 at 32 tiles, 26.7 and 24.6 at 128, 45 and 39
+// at 224, 82 and 73 at 512, 119 and 107 at 768; 139 both at 1024, 272 and 274 at
+// 2048 (K = 96: 59.4 and 61.5).
+inline bool level_few_tiles(long tiles64) { return tiles64 < 1024; }
+LevelConfig level_small(LevelConfig c);
 
 // One level over nent systems: dStart (device, nent entries) holds each
 // entry's first CTA; `tiles` CTAs in total; smem = max over entries.

@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(kThreads) k_expand_phases_batch(const ExpandJo
     }
 }
 
-// dst(g, r) = sum_k P[r][k] src(g, k): CTA = 8 rows x 32 columns g, its four
+// dst(g, r) = sum_k P[r][k] src(g, k) (+ acc): CTA = 8 rows x 32 columns g, its four
 // warps a quarter of K each (fragments straight from L2, two K values per
 // load), the quarters summed in order.  Latency-bound, so a warp has the
 // loads of kBatch K chunks in flight before their products.  A level of one
@@ -557,11 +557,11 @@ __global__ void __launch_bounds__(kNarrowThreads) k_expand_narrow(const LevelArg
     }
     const LevelArgs& a = args[lo];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
-    const int rt = a.M / 8;
+    const int rt = level_rows(a) / 8;
     const long u = t - start[lo], c0 = (u / rt) * kNarrowCols;
     const int r0 = (int)(u % rt) * 8;
     const int cols = (int)min((long)kNarrowCols, a.ncols - c0), ct = (cols + 7) / 8;
-    const int n8 = a.K / 8, k0 = n8 * warp / 4, k1 = n8 * (warp + 1) / 4;
+    const int n8 = level_k(a) / 8, k0 = n8 * warp / 4, k1 = n8 * (warp + 1) / 4;
     const double* pr = a.P + (long)(r0 + g) * a.ldp + 2 * tq;
     const double* z[4];
 #pragma unroll
@@ -582,6 +582,11 @@ __global__ void __launch_bounds__(kNarrowThreads) k_expand_narrow(const LevelArg
         for (int w = 1; w < 4; ++w) {
             v.x += red[w][warp][lane].x;
             v.y += red[w][warp][lane].y;
+        }
+        if (a.acc) {
+            const double2 o = *reinterpret_cast<const double2*>(a.acc + (c0 + 8 * warp + g) * a.acc_gs + r0 + 2 * tq);
+            v.x += o.x;
+            v.y += o.y;
         }
         *reinterpret_cast<double2*>(a.dst + (c0 + 8 * warp + g) * a.dst_gs + r0 + 2 * tq) = v;
     }
@@ -843,7 +848,7 @@ LevelArgs expand_out_args(const ExpandJob& j, double* Y, long limit)
     return a;
 }
 
-long expand_narrow_tiles(const LevelArgs& a) { return (long)(a.M / 8) * ((a.ncols + kNarrowCols - 1) / kNarrowCols); }
+long expand_narrow_tiles(const LevelArgs& a) { return (long)(level_rows(a) / 8) * ((a.ncols + kNarrowCols - 1) / kNarrowCols); }
 
 void launch_expand_narrow(const LevelArgs* dArgs, const long* dStart, int nent, long tiles, cudaStream_t s)
 {

@@ -28,6 +28,14 @@ __host__ __device__ inline int level_ks(int Np)
     return ks & ~3;
 }
 
+// Row warps of the FR = 1 form (Np <= 64), a power of two.
+__host__ __device__ inline int affine_row_warps(int Np)
+{
+    int w = 1;
+    while (w < Np / 8) w <<= 1;
+    return w;
+}
+
 // One CTA owns NC = 8*FC*CW columns and all Np rows of the result; each warp
 // owns an FR x FC block of 8x8 fragments.  P and the source columns are
 // staged through shared memory in K slices of KS (row pitch KS+4 doubles,
@@ -57,6 +65,7 @@ __global__ void __launch_bounds__(kThreads) k_affine_level_grouped(const LevelAr
         else hi = mid - 1;
     }
     const LevelArgs a = args[lo];
+    if (FR == 1) CW = 8 / affine_row_warps(a.Np);  // entries of all scan dimensions up to 64 share a launch
     affine_level_body<FR, FC>(a, t - start[lo], CW, level_ks(a.Np), smem);
 }
 
@@ -148,11 +157,21 @@ __device__ void affine_level_body(const LevelArgs& a, long tile, int CW, int KS,
 // took 90 us without, 82 with; ABM outputs of K = 608 (5.1 GFLOP) 182 and 172.
 // ---------------------------------------------------------------------------
 
-constexpr int kTM = 64, kTN = 64, kTK = 32, kTStages = 3;
-constexpr int kLdBn = kTN + 4;  // B tile, N-contiguous: [32 k][68]: rows t apart by 4 t mod 16 doubles
-constexpr int kStageA = kTM * kTK;
-constexpr int kStageB = (kTN * kTK > kTK * kLdBn) ? kTN * kTK : kTK * kLdBn;
-constexpr size_t kTiledSmem = (size_t)kTStages * (kStageA + kStageB) * sizeof(double);
+// A launch of few 64 x 64 tiles runs 32 x 32 ones (4 warps of 16 x 16), a
+// quarter of the work per CTA and four times the CTAs (level_few_tiles): the same
+// bits, as every element adds its products in the same order.  Squaring the
+// powers of a batch's systems up to NP = 436: 33 us a step, now 20.
+constexpr int kTK = 32, kTStages = 3;
+template <int T>
+struct Tile {
+    static constexpr int threads = 4 * T;
+    static constexpr int I = T / 16, J = 2;      // 8 x 8 fragments of a warp
+    static constexpr int WN = T / 16;            // warps along N
+    static constexpr int rowstep = threads / 16; // rows per pass of the K-contiguous copies
+    static constexpr int ldn = T + 4;            // B tile, N-contiguous: rows t apart by 4 t mod 16 doubles
+    static constexpr int stageA = T * kTK, stageB = kTK * ldn;
+    static constexpr size_t smem = (size_t)kTStages * (stageA + stageB) * sizeof(double);
+};
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -177,12 +196,14 @@ __device__ __forceinline__ double lds64(unsigned at)
 __device__ __forceinline__ int tile_at(int r, int c) { return r * kTK + ((c ^ ((r & 1) << 2)) << 1); }
 
 // A thread's part of a slice's copies: 16-byte chunk tid & 15 of the A rows
-// (tid >> 4) + 16 q and, K-contiguous, of the same B columns; N-contiguous,
-// columns 2 (tid & 31) of the K rows (tid >> 5) + 8 q.  Set up once per tile.
-template <bool kKC>
+// (tid >> 4) + rowstep q and, K-contiguous, of the same B columns;
+// N-contiguous, a pair of columns of the K rows tid / (T / 2) + 8 q.  Set up
+// once per tile.
+template <bool kKC, int T>
 struct TiledLoad {
+    using C = Tile<T>;
     const double *pa, *pb, *pb2;
-    long lda16, ldb;   // pointer steps per q
+    long ldaq, ldb;    // pointer steps per q
     unsigned sa, sb;   // shared byte offsets of q = 0 in a stage
     unsigned okA, okB; // q's rows / columns inside the matrices
     int K, K1, kc;     // kc: the thread's K index in a slice (A; K-contiguous B)
@@ -197,25 +218,25 @@ struct TiledLoad {
         kc = (tid & 15) * 2;
         okA = okB = 0;
         pa = a.P + (long)(m0 + r) * a.ldp + kc;
-        lda16 = 16 * a.ldp;
+        ldaq = C::rowstep * a.ldp;
         sa = 8 * tile_at(r, tid & 15);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-            if (m0 + r + 16 * q < rows) okA |= 1u << q;
+            if (m0 + r + C::rowstep * q < rows) okA |= 1u << q;
         pb2 = nullptr;
         if (kKC) {
             pb = a.src + (n0 + r) * a.src_gs + kc;
             if (K1 > 0) pb2 = a.src2 + (n0 + r) * a.src2_gs + kc - K1;
-            ldb = 16 * a.src_gs;
+            ldb = C::rowstep * a.src_gs;
             sb = sa;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                if (n0 + r + 16 * q < scols) okB |= 1u << q;
+                if (n0 + r + C::rowstep * q < scols) okB |= 1u << q;
         } else {
-            const int kr = tid >> 5, nc = (tid & 31) * 2;
+            const int kr = tid / (T / 2), nc = tid % (T / 2) * 2;
             pb = a.src + (long)kr * a.src_ks + n0 + nc;
             ldb = 8 * a.src_ks;
-            sb = 8 * (kr * kLdBn + nc);
+            sb = 8 * (kr * C::ldn + nc);
             if (n0 + nc < scols) okB = 15;
         }
     }
@@ -225,19 +246,19 @@ struct TiledLoad {
         const bool kin = k0 + kc < K;
         const double* p = pa + k0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) copy(A + sa + q * 16 * kTK * 8, p + q * lda16, kin && (okA >> q & 1), a.P);
+        for (int q = 0; q < 4; ++q) copy(A + sa + q * C::rowstep * kTK * 8, p + q * ldaq, kin && (okA >> q & 1), a.P);
         if (kKC) {
             const bool two = K1 > 0 && k0 + kc >= K1;
             const double* b = (two ? pb2 : pb) + k0;
-            const long step = two ? 16 * a.src2_gs : ldb;
+            const long step = two ? C::rowstep * a.src2_gs : ldb;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) copy(B + sb + q * 16 * kTK * 8, b + q * step, kin && (okB >> q & 1), a.src);
+            for (int q = 0; q < 4; ++q) copy(B + sb + q * C::rowstep * kTK * 8, b + q * step, kin && (okB >> q & 1), a.src);
         } else {
             const double* b = pb + (long)k0 * a.src_ks;
-            const int kr = threadIdx.x >> 5;
+            const int kr = threadIdx.x / (T / 2);
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                copy(B + sb + q * 8 * kLdBn * 8, b + q * ldb, k0 + kr + 8 * q < K && (okB >> q & 1), a.src);
+                copy(B + sb + q * 8 * C::ldn * 8, b + q * ldb, k0 + kr + 8 * q < K && (okB >> q & 1), a.src);
         }
     }
     // 16 bytes, or zeros (nothing read)
@@ -256,32 +277,34 @@ __device__ __forceinline__ int tri_limit(const LevelArgs& a, int r)
     return min(a.K1, a.tri_base + (min(r, rows - 1) / a.tri_p) * a.tri_step);
 }
 
-template <bool kKC>
+template <bool kKC, int T>
 __device__ void tiled_level_body(const LevelArgs& a, long tile, double* smem)
 {
+    using C = Tile<T>;
+    constexpr int I = C::I, J = C::J, kStageA = C::stageA, kStageB = C::stageB, kRows = T / 2;  // rows per warp
     const int rows = level_rows(a), K = level_k(a);
-    const int mt = (rows + kTM - 1) / kTM;
-    const int m0 = (int)(tile % mt) * kTM;
-    const long n0 = (tile / mt) * kTN;
+    const int mt = (rows + T - 1) / T;
+    const int m0 = (int)(tile % mt) * T;
+    const long n0 = (tile / mt) * T;
     const unsigned sA = (unsigned)__cvta_generic_to_shared(smem), sB = sA + 8 * kTStages * kStageA;
-    const TiledLoad<kKC> fetch(a, m0, n0);
+    const TiledLoad<kKC, T> fetch(a, m0, n0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wm = warp >> 2, wn = warp & 3;
+    const int wm = warp / C::WN, wn = warp % C::WN;
     const int gq = lane >> 2, tq = lane & 3;
     // a tile wholly beyond the source columns only writes acc (or zeros)
     const long scols = a.src_cols > 0 ? a.src_cols : a.ncols;
     const int all = n0 >= scols ? 0 : (K + kTK - 1) / kTK;
     // slices [0, n1) and [s2, all): those between hold only zeros of these rows
-    const int n1 = min(all, (tri_limit(a, m0 + kTM - 1) + kTK - 1) / kTK), s2 = max(n1, min(all, a.K1 / kTK));
+    const int n1 = min(all, (tri_limit(a, m0 + T - 1) + kTK - 1) / kTK), s2 = max(n1, min(all, a.K1 / kTK));
     const int nk = n1 + all - s2;
-    const int wlim = tri_limit(a, m0 + wm * 32 + 31);  // this warp's rows
+    const int wlim = tri_limit(a, m0 + wm * kRows + kRows - 1);  // this warp's rows
     auto slice = [&](int i) { return (i < n1 ? i : s2 + i - n1) * kTK; };
 
-    double acc[4][2][2];
+    double acc[I][J][2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < I; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        for (int j = 0; j < J; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
 #pragma unroll
     for (int s = 0; s < kTStages - 1; ++s) {
@@ -301,31 +324,31 @@ __device__ void tiled_level_body(const LevelArgs& a, long tile, double* smem)
         st = st + 1 == kTStages ? 0 : st + 1;
         const int k0 = slice(kt);
         auto at64 = [&](unsigned base, int r, int k) { return lds64(base + 8 * (tile_at(r, k >> 1) + (k & 1))); };
-        auto load = [&](int c, double2 (&af)[4], double2 (&bf)[2]) {
+        auto load = [&](int c, double2 (&af)[I], double2 (&bf)[J]) {
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
+            for (int j = 0; j < J; ++j) {
                 const int col = wn * 16 + j * 8 + gq;
                 if (kKC) bf[j] = lds128(Bs + 8 * tile_at(col, 4 * c + tq));
-                else bf[j] = make_double2(lds64(Bs + 8 * ((8 * c + tq) * kLdBn + col)), lds64(Bs + 8 * ((8 * c + 4 + tq) * kLdBn + col)));
+                else bf[j] = make_double2(lds64(Bs + 8 * ((8 * c + tq) * C::ldn + col)), lds64(Bs + 8 * ((8 * c + 4 + tq) * C::ldn + col)));
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = wm * 32 + i * 8 + gq;
+            for (int i = 0; i < I; ++i) {
+                const int r = wm * kRows + i * 8 + gq;
                 if (kKC) af[i] = lds128(As + 8 * tile_at(r, 4 * c + tq));
                 else af[i] = make_double2(at64(As, r, 8 * c + tq), at64(As, r, 8 * c + 4 + tq));
             }
         };
-        auto products = [&](const double2 (&af)[4], const double2 (&bf)[2]) {
+        auto products = [&](const double2 (&af)[I], const double2 (&bf)[J]) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < I; ++i)
 #pragma unroll
-                for (int j = 0; j < 2; ++j) dmma_m8n8k4(acc[i][j][0], acc[i][j][1], af[i].x, bf[j].x);
+                for (int j = 0; j < J; ++j) dmma_m8n8k4(acc[i][j][0], acc[i][j][1], af[i].x, bf[j].x);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < I; ++i)
 #pragma unroll
-                for (int j = 0; j < 2; ++j) dmma_m8n8k4(acc[i][j][0], acc[i][j][1], af[i].y, bf[j].y);
+                for (int j = 0; j < J; ++j) dmma_m8n8k4(acc[i][j][0], acc[i][j][1], af[i].y, bf[j].y);
         };
-        double2 a0[4], b0[2], a1[4], b1[2];
+        double2 a0[I], b0[J], a1[I], b1[J];
         if (k0 + kTK <= K && (k0 + kTK <= wlim || k0 >= a.K1)) {
             // fragments one chunk ahead of their products
             load(0, a0, b0);
@@ -353,10 +376,10 @@ __device__ void tiled_level_body(const LevelArgs& a, long tile, double* smem)
     // waiting behind the store before it
     if (a.acc) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const long r = m0 + wm * 32 + i * 8 + gq;
+        for (int i = 0; i < I; ++i) {
+            const long r = m0 + wm * kRows + i * 8 + gq;
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < J; ++j)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const long g = n0 + wn * 16 + j * 8 + 2 * tq + e;
@@ -368,11 +391,11 @@ __device__ void tiled_level_body(const LevelArgs& a, long tile, double* smem)
         }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const long r = m0 + wm * 32 + i * 8 + gq;
+    for (int i = 0; i < I; ++i) {
+        const long r = m0 + wm * kRows + i * 8 + gq;
         if (r >= rows) continue;
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < J; ++j)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const long g = n0 + wn * 16 + j * 8 + 2 * tq + e;
@@ -384,18 +407,18 @@ __device__ void tiled_level_body(const LevelArgs& a, long tile, double* smem)
     }
 }
 
-template <bool kKC>
-__global__ void __launch_bounds__(kThreads, 2) k_level_tiled(LevelArgs a)
+template <bool kKC, int T>
+__global__ void __launch_bounds__(Tile<T>::threads, T == 64 ? 2 : 4) k_level_tiled(LevelArgs a)
 {
-    extern __shared__ double smem[];
-    tiled_level_body<kKC>(a, blockIdx.x, smem);
+    extern __shared__ __align__(16) double smem[];
+    tiled_level_body<kKC, T>(a, blockIdx.x, smem);
 }
 
-template <bool kKC>
-__global__ void __launch_bounds__(kThreads, 2) k_level_tiled_grouped(const LevelArgs* __restrict__ args,
+template <bool kKC, int T>
+__global__ void __launch_bounds__(Tile<T>::threads, T == 64 ? 2 : 4) k_level_tiled_grouped(const LevelArgs* __restrict__ args,
                                                                      const long* __restrict__ start, int nent)
 {
-    extern __shared__ double smem[];
+    extern __shared__ __align__(16) double smem[];
     const long t = blockIdx.x;
     int lo = 0, hi = nent - 1;
     while (lo < hi) {
@@ -404,7 +427,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_level_tiled_grouped(const Level
         else hi = mid - 1;
     }
     const LevelArgs a = args[lo];
-    tiled_level_body<kKC>(a, t - start[lo], smem);
+    tiled_level_body<kKC, T>(a, t - start[lo], smem);
 }
 
 // Down-sweep bookkeeping before a tiled level: cpy(g, i) <-> dst(g, i).
@@ -651,9 +674,34 @@ LevelArgs tiled_args(const LevelArgs& a)
     return b;
 }
 
-long tiled_tiles(const LevelArgs& b)
+long tiled_tiles(const LevelArgs& b, int T)
 {
-    return (long)((level_rows(b) + kTM - 1) / kTM) * ((b.ncols + kTN - 1) / kTN);
+    return (long)((level_rows(b) + T - 1) / T) * ((b.ncols + T - 1) / T);
+}
+
+template <bool kKC, int T>
+void tiled_t(const LevelArgs& a, cudaStream_t s)
+{
+    using C = Tile<T>;
+    PARODE_CUDA(cudaFuncSetAttribute(k_level_tiled<kKC, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
+    k_level_tiled<kKC, T><<<(unsigned)tiled_tiles(a, T), C::threads, C::smem, s>>>(a);
+    PARODE_CUDA(cudaGetLastError());
+}
+
+void launch_tiled(const LevelArgs& a, cudaStream_t s)
+{
+    const bool kc = a.src_ks == 1, small = level_few_tiles(tiled_tiles(a, 64));
+    if (kc) small ? tiled_t<true, 32>(a, s) : tiled_t<true, 64>(a, s);
+    else small ? tiled_t<false, 32>(a, s) : tiled_t<false, 64>(a, s);
+}
+
+template <bool kKC, int T>
+void tiled_grouped_t(const LevelArgs* args, const long* start, int nent, long tiles, cudaStream_t s)
+{
+    using C = Tile<T>;
+    PARODE_CUDA(cudaFuncSetAttribute(k_level_tiled_grouped<kKC, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
+    k_level_tiled_grouped<kKC, T><<<(unsigned)tiles, C::threads, C::smem, s>>>(args, start, nent);
+    PARODE_CUDA(cudaGetLastError());
 }
 
 template <int FR, int FC>
@@ -684,14 +732,7 @@ void launch_affine_level(const LevelArgs& a, cudaStream_t s)
             k_swap<<<(unsigned)std::min<long>(blocks_for(a.ncols * (long)a.Np, 256), 4096), 256, 0, s>>>(a);
             PARODE_CUDA(cudaGetLastError());
         }
-        PARODE_CUDA(cudaFuncSetAttribute(k_level_tiled<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kTiledSmem));
-        PARODE_CUDA(cudaFuncSetAttribute(k_level_tiled<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kTiledSmem));
-        const long tiles = tiled_tiles(b);
-        if (b.src_ks == 1) k_level_tiled<true><<<(unsigned)tiles, kThreads, kTiledSmem, s>>>(b);
-        else k_level_tiled<false><<<(unsigned)tiles, kThreads, kTiledSmem, s>>>(b);
-        PARODE_CUDA(cudaGetLastError());
+        launch_tiled(b, s);
         return;
     }
     const int rf = a.Np / 8;
@@ -804,16 +845,14 @@ LevelConfig level_config(const LevelArgs& a)
     if (Np > 64 || a.M > 0 || a.K > 0) {
         const LevelArgs b = tiled_args(a);
         c.id = b.src_ks == 1 ? 5 : 6;
-        c.NC = kTN;
-        c.smem = kTiledSmem;
+        c.NC = 64;
+        c.smem = Tile<64>::smem;
         return c;
     }
     const int rf = Np / 8;
     if (rf <= 8) {
-        int RW = 1;
-        while (RW < rf) RW <<= 1;
         c.id = 0;
-        c.CW = 8 / RW;
+        c.CW = 8 / affine_row_warps(Np);
     } else if (rf <= 16) {
         c.id = 1;
     } else if (rf <= 32) {
@@ -846,13 +885,12 @@ void launch_affine_level_grouped(const LevelConfig& c, const LevelArgs* dArgs, c
 {
     if (nent <= 0 || tiles <= 0) return;
     if (c.id >= 5) {
-        PARODE_CUDA(cudaFuncSetAttribute(k_level_tiled_grouped<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kTiledSmem));
-        PARODE_CUDA(cudaFuncSetAttribute(k_level_tiled_grouped<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kTiledSmem));
-        if (c.id == 5) k_level_tiled_grouped<true><<<(unsigned)tiles, kThreads, kTiledSmem, s>>>(dArgs, dStart, nent);
-        else k_level_tiled_grouped<false><<<(unsigned)tiles, kThreads, kTiledSmem, s>>>(dArgs, dStart, nent);
-        PARODE_CUDA(cudaGetLastError());
+        switch (c.id) {
+        case 5: tiled_grouped_t<true, 64>(dArgs, dStart, nent, tiles, s); break;
+        case 6: tiled_grouped_t<false, 64>(dArgs, dStart, nent, tiles, s); break;
+        case 7: tiled_grouped_t<true, 32>(dArgs, dStart, nent, tiles, s); break;
+        default: tiled_grouped_t<false, 32>(dArgs, dStart, nent, tiles, s); break;
+        }
         return;
     }
     if (smem > 200 * 1024) throw Error(kInvalidArgument, "grouped level: shared memory above 200 KB");
@@ -876,19 +914,22 @@ void launch_gemm_tiled(const LevelArgs& a, cudaStream_t s)
     if (a.K1 > 0 && ((a.K1 & 1) || a.K1 >= level_k(a) || a.src_ks != 1 || !a.src2 || (a.src2_gs & 1) ||
                      (a.src_gs & 1)))
         throw Error(kInvalidArgument, "tiled GEMM: two-part source needs even K1 < K, K-contiguous, even strides");
-    PARODE_CUDA(cudaFuncSetAttribute(k_level_tiled<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kTiledSmem));
-    PARODE_CUDA(cudaFuncSetAttribute(k_level_tiled<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kTiledSmem));
-    const long tiles = tiled_tiles(a);
-    if (a.src_ks == 1) k_level_tiled<true><<<(unsigned)tiles, kThreads, kTiledSmem, s>>>(a);
-    else k_level_tiled<false><<<(unsigned)tiles, kThreads, kTiledSmem, s>>>(a);
-    PARODE_CUDA(cudaGetLastError());
+    launch_tiled(a, s);
+}
+
+LevelConfig level_small(LevelConfig c)
+{
+    if (c.id == 5 || c.id == 6) {
+        c.id += 2;
+        c.NC = 32;
+        c.smem = Tile<32>::smem;
+    }
+    return c;
 }
 
 long level_tiles(const LevelConfig& c, const LevelArgs& stored)
 {
-    if (c.id >= 5) return tiled_tiles(stored);
+    if (c.id >= 5) return tiled_tiles(stored, c.NC);
     return (stored.ncols + c.NC - 1) / c.NC;
 }
 
