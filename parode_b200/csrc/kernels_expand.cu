@@ -20,8 +20,8 @@
 // the outputs and 2 NP (NP + H) / B for the states, H = 2 m terms, so the
 // blocks can be long (B = 64).  Measured on one B200: RK4 n = 64, m = p = 8,
 // 2^20 steps mixed 0.277 ms (samples 0.034, 3xTF32 windows 0.085, carry 0.105,
-// state part 0.07) -> 0.095 ms; a free response of 24 states, 10^5 steps
-// (FP64) 0.240 ms with the in-block sweeps -> 0.022 ms.
+// state part 0.07) -> 0.086 ms; a free response of 24 states, 10^5 steps
+// (FP64) 0.240 ms with the in-block sweeps -> 0.016 ms.
 //
 // The phases of a block's start are sincos of the argument rounded as the
 // oracle rounds it; within a block they advance exactly (by the tables), so
@@ -34,6 +34,7 @@
 #include "device_common.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 namespace parode {
@@ -347,7 +348,7 @@ struct OutCfg {
 template <int KS>
 __global__ void __launch_bounds__(OutCfg<KS>::threads, 1)
     k_expand_out(const double* __restrict__ W, int M, int Ms, int slices, const double* Z, double* Y,
-                 long gs, long c0, long c1, long limit, int parts, int vec)
+                 long gs, long c0, long c1, long limit, int vec)
 {
     extern __shared__ __align__(16) double Ws[];
     constexpr int Kc = 4 * KS, ld = Kc + ((Kc & 8) ? 0 : 8), CT = OutCfg<KS>::CT, kT = OutCfg<KS>::threads;
@@ -365,12 +366,12 @@ __global__ void __launch_bounds__(OutCfg<KS>::threads, 1)
     grid_dep_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
     const long nt = (c1 - c0 + 8 * CT - 1) / (8 * CT);
-    const long t0 = nt * idx / nidx, t1 = nt * (idx + 1) / nidx;
-    const long tasks = (t1 - t0) * parts;
-    for (long q = warp; q < tasks; q += kT / 32) {
-        const long tile = t0 + q / parts;
-        const int part = (int)(q % parts);
-        const int r0 = RT * part / parts, r1 = RT * (part + 1) / parts;
+    // the slice's row tiles, tile after tile, in equal parts to its CTAs' warps
+    const long total = nt * RT, gw = (long)idx * (kT / 32) + warp, nw = (long)nidx * (kT / 32);
+    long left = total * (gw + 1) / nw - total * gw / nw, tile = total * gw / nw / RT;
+    int r0 = (int)(total * gw / nw - tile * RT);
+    for (int r1; left > 0; left -= r1 - r0, r0 = 0, ++tile) {
+        r1 = (int)min((long)RT, r0 + left);
         const long b0 = c0 + tile * 8 * CT;
         double2 za[CT][KS / 2];
 #pragma unroll
@@ -615,23 +616,33 @@ void out_t(const ExpandTables& t, const double* Z, double* Y, long c0, long c1, 
 {
     using C = OutCfg<KS>;
     const int M = t.sh.rows(), ld = smem_pitch(t.sh.Kc);
-    const int cap = (int)(kSmemMax / (ld * sizeof(double))) & ~7;
-    const int M8 = (M + 7) & ~7;
-    const int slices = (M8 + cap - 1) / cap;
-    const int Ms = ((M8 + slices - 1) / slices + 7) & ~7;
+    const int cap = (int)(kSmemMax / (ld * sizeof(double))) / 8, tiles8 = (M + 7) / 8;  // row tiles: of a slice, of W
+    const long nt = (c1 - c0 + 8 * C::CT - 1) / (8 * C::CT);
+    const int warps = C::threads / 32;
+    // Slices of W: cycles to stage one (a CTA draws about 32 bytes a cycle with
+    // all SMs reading), to fetch a warp's blocks (500 for each tile it starts)
+    // and for its products (three warps share a sub-partition).  A slice
+    // as large as fits staged 147 KB for 98 tiles of a free response of 24
+    // states, 10^5 steps, and dealt out whole tiles: the solve took 20.6 us,
+    // 16.0 in 16 slices; 64 states, 2^20 steps, mixed 116.6, 108.5 in 4 for 3.
+    int slices = (tiles8 + cap - 1) / cap;
+    double best = 1e300;
+    for (int k = slices, end = std::min(tiles8, std::max(slices, std::min(sms, 40))); k <= end; ++k) {
+        const int rt = (tiles8 + k - 1) / k;
+        const double per = std::ceil((double)nt * rt / ((long)std::max(1, sms / k) * warps));
+        const double cost = 2.0 * rt * t.sh.Kc + 500.0 * (per / rt + 1.0) + per * (warps / 4) * 16.0 * C::CT * KS;
+        if (cost < best) best = cost, slices = k;
+    }
+    const int Ms = (tiles8 + slices - 1) / slices * 8;
+    slices = (M + Ms - 1) / Ms;
     const size_t smem = (size_t)Ms * ld * sizeof(double);
     PARODE_CUDA(cudaFuncSetAttribute(k_expand_out<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const long nt = (c1 - c0 + 8 * C::CT - 1) / (8 * C::CT);
-    const long row_tiles = Ms / 8;
-    // CTAs: no more than the SMs, each with at least a warp's row tile per warp
-    const long work = nt * row_tiles * slices;
-    const long ctas = std::max<long>(slices, std::min<long>(sms, work / (C::threads / 32)));
-    const long per_cta = std::max<long>(1, nt * slices / ctas);
-    const int parts = (int)std::max<long>(1, std::min<long>(row_tiles, (96 + per_cta - 1) / per_cta));
+    // CTAs: no more than the SMs, each with at least a row tile per warp
+    const long ctas = std::max<long>(slices, std::min<long>(sms, nt * tiles8 / warps));
     const long gs = M;
     const int vec = ((reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (gs & 1) == 0) ? 1 : 0;
     launch_dependent(k_expand_out<KS>, dim3((unsigned)ctas), dim3(C::threads), smem, s, t.W, M, Ms, slices, Z, Y, gs, c0,
-                     c1, limit, parts, vec);
+                     c1, limit, vec);
 }
 
 template <class F>

@@ -192,3 +192,16 @@ def test_large_plan_runs_doublings(pb, solver, n, m, T, terms):
     ref = oracle.simulate_affine(oracle.System(c.A, c.B, c.C, c.D, c.x0), oracle.Input.sinusoid(s.a, s.f, s.phi),
                                  solver, c.t0, c.t_end, c.h)
     assert oracle.rel_err(y, ref) <= TOL_PHASES
+
+
+@pytest.mark.parametrize("n,p,T", [(24, 24, 64 * 16 * 9 + 1), (3, 1, 4100), (64, 5, 9000), (17, 33, 64 * 16 * 3), (40, 1, 70_000)])
+def test_output_slices(pb, n, p, T):
+    """Outputs in slices of the table by a cost model, row tiles dealt to the
+    warps in parts that start and end inside a tile: many rows and few blocks,
+    one row, ragged ends.  FP64 free response, gate 1e-12 as for the other forms."""
+    c = wl.small(51000 + n + T, 0, n, 1, p, T, h=1e-3)
+    plan = _plan(pb, c, 0, pb.FP64, B=False, D=False)
+    ref = oracle.simulate_affine(oracle.System(c.A, None, c.C, None, c.x0), oracle.Input.zero(), 0, c.t0, c.t_end, c.h)
+    for offset in (0, 1):
+        assert oracle.rel_err(_device_y(plan, offset), ref) <= TOL_FREE, offset
+    plan.close()
