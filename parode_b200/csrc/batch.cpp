@@ -6,12 +6,17 @@
 #include "common.h"
 
 #include <algorithm>
-#include <map>
-#include <mutex>
+#include <atomic>
 #include <chrono>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstring>
+#include <functional>
+#include <map>
+#include <memory>
+#include <mutex>
+#include <system_error>
 #include <thread>
 
 namespace parode {
@@ -36,71 +41,106 @@ struct Layout {
     }
 };
 
-double sinusoid_host(const InputEntry* e, int i, double t)
-{
-    const double two_pi = 6.283185307179586476925286766559;
-    double v = 0.0;
-    for (int k = 0; k < e->K; ++k) {
-        const int q = i * e->K + k;
-        v += e->a[q] * std::sin(two_pi * e->f[q] * t + e->phi[q]);
-    }
-    return v;
-}
-
 // A batch discretises on the host threads when no system takes more than
 // kHostDiscMaxSystem multiply-adds (RK4 n <= 69, ABM n <= 100: about a
 // millisecond on one core) and the batch no more than kHostDiscMaxBatch.
 constexpr double kHostDiscMaxSystem = 1e6;
 constexpr double kHostDiscMaxBatch = 8e6;
 
+// Host threads for the set-up loops, kept for the process (at most one fewer
+// than the cores, and 31): 16 systems formed, solved and dropped took 2.9 ms
+// with threads started and streams created for each batch, 1.7 without.  The
+// caller works too, so a loop ends even when no thread is free (another
+// batch's loop has them).
+class HostThreads {
+public:
+    static HostThreads& get()
+    {
+        static HostThreads* t = new HostThreads();  // never destroyed: its threads may outlive main's statics
+        return *t;
+    }
+    void run(int n, const std::function<void(int)>& f)
+    {
+        auto job = std::make_shared<Job>();
+        job->n = n;
+        job->f = &f;
+        int want = 0;
+        {
+            std::lock_guard<std::mutex> g(mu_);
+            want = std::min(n, (int)std::min(32u, std::max(1u, std::thread::hardware_concurrency()))) - 1;
+            try {
+                while ((int)threads_ < want) {
+                    std::thread([this] { serve(); }).detach();
+                    ++threads_;
+                }
+            } catch (const std::system_error&) {  // no more threads: those there are, and the caller
+            }
+            jobs_.push_back(job);
+        }
+        for (int t = 0; t < want; ++t) cv_.notify_one();
+        work(*job);
+        std::unique_lock<std::mutex> g(mu_);
+        jobs_.erase(std::remove(jobs_.begin(), jobs_.end(), job), jobs_.end());
+        done_.wait(g, [&] { return job->busy == 0; });
+        if (job->error) std::rethrow_exception(job->error);
+    }
+
+private:
+    struct Job {
+        int n = 0;
+        const std::function<void(int)>* f = nullptr;
+        std::atomic<int> next{0};
+        int busy = 0;  // threads inside, under mu_
+        std::exception_ptr error;
+    };
+
+    void work(Job& j)
+    {
+        for (int i; (i = j.next.fetch_add(1)) < j.n;) {
+            try {
+                (*j.f)(i);
+            } catch (...) {
+                std::lock_guard<std::mutex> g(mu_);
+                if (!j.error) j.error = std::current_exception();
+                j.next = j.n;
+            }
+        }
+    }
+    void serve()
+    {
+        std::unique_lock<std::mutex> g(mu_);
+        for (;;) {
+            std::shared_ptr<Job> job;
+            for (auto& j : jobs_)
+                if (j->next < j->n) {
+                    job = j;
+                    break;
+                }
+            if (!job) {
+                cv_.wait(g);
+                continue;
+            }
+            ++job->busy;
+            g.unlock();
+            work(*job);
+            g.lock();
+            if (--job->busy == 0) done_.notify_all();
+        }
+    }
+    std::mutex mu_;
+    std::condition_variable cv_, done_;
+    std::vector<std::shared_ptr<Job>> jobs_;
+    int threads_ = 0;
+};
+
 template <class F>
 void parallel_for(int n, F&& f)
 {
-    if (n <= 1) {  // one item: no thread to start (a server's small batches)
+    if (n <= 1) {  // one item: nothing to share (a server's small batches)
         if (n == 1) f(0);
         return;
     }
-    int nt = (int)std::min<unsigned>(std::max(1u, std::thread::hardware_concurrency()), 32u);
-    nt = std::min(nt, std::max(1, n));
-    std::vector<std::thread> th;
-    std::vector<std::exception_ptr> err(nt);
-    for (int t = 0; t < nt; ++t)
-        th.emplace_back([&, t] {
-            try {
-                for (int i = t; i < n; i += nt) f(i);
-            } catch (...) {
-                err[t] = std::current_exception();
-            }
-        });
-    for (auto& x : th) x.join();
-    for (auto& e : err)
-        if (e) std::rethrow_exception(e);
-}
-
-// The discretisation of one system on the host, as the device kernel writes
-// it (kernels_disc.cu): the compact Phi, Bbar zero-filled to n x W max(m, 1),
-// its transpose when asked, and ||Phi - R||_inf over the stored rows (each
-// row summed in order), every operation in the kernel's order.
-double discretise_host(int solver, int n, int Ns, int W, double h, const SystemDesc& s, double* phi, double* bbar,
-                       double* bbarT)
-{
-    const int mB = s.zeroB ? 0 : s.m, Wm = W * mB;
-    std::fill(bbar, bbar + (size_t)n * W * std::max(mB, 1), 0.0);
-    if (solver == kRK4) discretise_rk4(n, mB, s.A.data(), mB ? s.B.data() : nullptr, h, phi, bbar);
-    else discretise_abm_last(n, mB, s.A.data(), mB ? s.B.data() : nullptr, h, phi, bbar);
-    if (bbarT) {
-        std::fill(bbarT, bbarT + (size_t)std::max(Wm, 1) * n, 0.0);
-        for (int r = 0; r < n; ++r)
-            for (int c = 0; c < Wm; ++c) bbarT[(size_t)c * n + r] = bbar[(size_t)r * Wm + c];
-    }
-    const int d0 = solver == kRK4 ? 0 : 3 * n;
-    double dmax = 0.0;
-    for (int r = 0; r < n; ++r) {
-        double sum = 0.0;
-        for (int c = 0; c < Ns; ++c) sum += std::fabs(phi[(size_t)r * Ns + c] + -(c == d0 + r ? 1.0 : 0.0));
-        dmax = std::max(dmax, sum);
-    }
-    return dmax;
+    HostThreads::get().run(n, f);
 }
 
 }  // namespace
@@ -428,7 +468,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
     // batch of small systems runs it on the host threads, with no device round
     // trip (a server sets batches up while others run); a large one on the
     // device.
-    PARODE_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
+    stream_ = take_stream(device_);
     struct DiscOff {
         size_t A, B, phi, bbar, bbarT, work;
     };
@@ -451,15 +491,15 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
     cudaStream_t dstream = nullptr;
     std::unique_ptr<HostStage> dstage, ddelta;
     struct StreamGuard {
+        int device, priority;
         cudaStream_t* s;
         ~StreamGuard()
         {
-            if (*s) {
-                cudaStreamSynchronize(*s);
-                cudaStreamDestroy(*s);
-            }
+            if (!*s) return;
+            if (cudaStreamSynchronize(*s) == cudaSuccess) give_stream(device, *s, priority);
+            else cudaStreamDestroy(*s);
         }
-    } dguard{&dstream};
+    } dguard{device_, 0, &dstream};
     if (disc_host) {
         Layout D;
         for (int i = 0; i < N; ++i) {
@@ -494,7 +534,8 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         {
             int least = 0, greatest = 0;
             PARODE_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-            PARODE_CUDA(cudaStreamCreateWithPriority(&dstream, cudaStreamNonBlocking, greatest));
+            dguard.priority = greatest;
+            dstream = take_stream(device_, greatest);
         }
         Layout D;
         for (int i = 0; i < N; ++i) {  // staged inputs first
@@ -1542,8 +1583,8 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
     events_.resize(forks_.size() + 1 + two_chains_, nullptr);
     for (auto& e : events_) PARODE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     launch_chains(stream_, {&ls_power_}, [&] {
-        // after the large chain's launches: its kernels run meanwhile (a stream takes about 50 us)
-        for (auto& f : forks_) PARODE_CUDA(cudaStreamCreateWithFlags(&f, cudaStreamNonBlocking));
+        // after the large chain's launches: its kernels run meanwhile (a new stream takes about 50 us)
+        for (auto& f : forks_) f = take_stream(device_);
     });
     if (!ex_.empty()) {
         const int ne = (int)ex_.size();
@@ -1706,8 +1747,9 @@ BatchPlan::~BatchPlan() { release(); }
 void BatchPlan::release()
 {
     cudaSetDevice(device_);
-    if (last_stream_ && last_stream_ != stream_) cudaStreamSynchronize(last_stream_);
-    if (stream_) cudaStreamSynchronize(stream_);
+    bool ok = true;  // idle streams go back to the pool, those of a failed context are destroyed
+    if (last_stream_ && last_stream_ != stream_) ok = cudaStreamSynchronize(last_stream_) == cudaSuccess;
+    if (stream_) ok = cudaStreamSynchronize(stream_) == cudaSuccess && ok;
     last_stream_ = nullptr;
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     graph_exec_ = nullptr;
@@ -1716,8 +1758,8 @@ void BatchPlan::release()
     disc_ = nullptr;
     for (auto& f : forks_)
         if (f) {
-            cudaStreamSynchronize(f);
-            cudaStreamDestroy(f);
+            ok = cudaStreamSynchronize(f) == cudaSuccess && ok;
+            ok ? give_stream(device_, f) : (void)cudaStreamDestroy(f);
             f = nullptr;
         }
     for (auto& e : events_)
@@ -1730,8 +1772,8 @@ void BatchPlan::release()
     if (arena_) cudaFreeAsync(arena_, fs);
     arena_ = nullptr;
     if (stream_) {
-        cudaStreamSynchronize(stream_);
-        cudaStreamDestroy(stream_);
+        ok = cudaStreamSynchronize(stream_) == cudaSuccess && ok;
+        ok ? give_stream(device_, stream_) : (void)cudaStreamDestroy(stream_);
     }
     stream_ = nullptr;
 }

@@ -284,4 +284,26 @@ void abm_startup(const SystemDesc& s, const double* U9, double h, double* X0)
     }
 }
 
+double discretise_host(int solver, int n, int Ns, int W, double h, const SystemDesc& s, double* phi, double* bbar,
+                       double* bbarT)
+{
+    const int mB = s.zeroB ? 0 : s.m, Wm = W * mB;
+    std::fill(bbar, bbar + (size_t)n * W * std::max(mB, 1), 0.0);
+    if (solver == 0) discretise_rk4(n, mB, s.A.data(), mB ? s.B.data() : nullptr, h, phi, bbar);
+    else discretise_abm_last(n, mB, s.A.data(), mB ? s.B.data() : nullptr, h, phi, bbar);
+    if (bbarT) {
+        std::fill(bbarT, bbarT + (size_t)std::max(Wm, 1) * n, 0.0);
+        for (int r = 0; r < n; ++r)
+            for (int c = 0; c < Wm; ++c) bbarT[(size_t)c * n + r] = bbar[(size_t)r * Wm + c];
+    }
+    const int d0 = solver == 0 ? 0 : 3 * n;
+    double dmax = 0.0;
+    for (int r = 0; r < n; ++r) {
+        double sum = 0.0;
+        for (int c = 0; c < Ns; ++c) sum += std::fabs(phi[(size_t)r * Ns + c] + -(c == d0 + r ? 1.0 : 0.0));
+        dmax = std::max(dmax, sum);
+    }
+    return dmax;
+}
+
 }  // namespace parode

@@ -38,6 +38,14 @@ void discretise_abm(int n, int m, const double* A, const double* B, double h, do
 // rows above it are the exact shift (block b reads block b + 1).
 void discretise_abm_last(int n, int m, const double* A, const double* B, double h, double* last, double* Bbar);
 
+// The discretisation of one system, as the device kernels write it
+// (kernels_disc.cu): the compact Phi (RK4: n x n; ABM: its last block row, n x
+// 4n), Bbar zero-filled to n x W max(m, 1), its transpose when asked, and
+// ||Phi - R||_inf over the stored rows (R: the exact 0/1 part; each row summed
+// in order), every operation in the kernels' order.
+double discretise_host(int solver, int n, int Ns, int W, double h, const SystemDesc& s, double* phi, double* bbar,
+                       double* bbarT);
+
 // ABM start-up: X0 = [x0; x1; x2; x3] from three classical RK4 steps with the
 // nine inputs U[j] = u(t0 + j h/2), j = 0..8 (U is 9 x m, row-major)
 // (reference Sources/AdamsMoulton.cpp:29-104).

@@ -7,6 +7,7 @@
 
 #include <nvrtc.h>
 
+#include <cmath>
 #include <cstring>
 
 namespace parode {
@@ -95,6 +96,17 @@ int InputRegistry::add_user(const std::string& source)
     compile(e.get(), 0);
     entries_.push_back(std::move(e));
     return (int)entries_.size() - 1;
+}
+
+double sinusoid_host(const InputEntry* e, int i, double t)
+{
+    const double two_pi = 6.283185307179586476925286766559;
+    double v = 0.0;
+    for (int k = 0; k < e->K; ++k) {
+        const int q = i * e->K + k;
+        v += e->a[q] * std::sin(two_pi * e->f[q] * t + e->phi[q]);
+    }
+    return v;
 }
 
 int InputRegistry::add_sinusoid(int m, int K, const double* a, const double* f, const double* phi)

@@ -28,6 +28,9 @@ struct InputEntry {
     std::vector<double*> dparams;  // per device: a | f | phi, 3*m*K doubles
 };
 
+// u_i(t) of a sinusoid input, on the host.
+double sinusoid_host(const InputEntry* e, int i, double t);
+
 class InputRegistry {
 public:
     ~InputRegistry();

@@ -18,12 +18,17 @@ namespace parode {
 
 namespace {
 
-// Streams and events of finished plans, kept per device for the next plan
+// Streams and events of finished plans and batches, kept per device for the next
 // (creating two streams and five events cost ~0.1 ms of every one-shot
-// SimulateODE call).  Returned idle: the plan synchronises them first.
+// SimulateODE call).  Returned idle: the owner synchronises them first.
+constexpr size_t kMaxIdleStreams = 64;
 struct HandlePool {
     std::mutex mu;
-    std::vector<std::pair<int, cudaStream_t>> streams;
+    struct Stream {
+        int dev, priority;
+        cudaStream_t s;
+    };
+    std::vector<Stream> streams;
     std::vector<std::pair<int, cudaEvent_t>> events;
     std::vector<char*> pinned;
 };
@@ -32,24 +37,6 @@ HandlePool& handles()
 {
     static HandlePool* p = new HandlePool();
     return *p;
-}
-
-cudaStream_t take_stream(int dev)
-{
-    {
-        HandlePool& h = handles();
-        std::lock_guard<std::mutex> g(h.mu);
-        for (size_t k = 0; k < h.streams.size(); ++k)
-            if (h.streams[k].first == dev) {
-                cudaStream_t s = h.streams[k].second;
-                h.streams[k] = h.streams.back();
-                h.streams.pop_back();
-                return s;
-            }
-    }
-    cudaStream_t s = nullptr;
-    PARODE_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    return s;
 }
 
 cudaEvent_t take_event(int dev)
@@ -68,13 +55,6 @@ cudaEvent_t take_event(int dev)
     cudaEvent_t e = nullptr;
     PARODE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     return e;
-}
-
-void give_stream(int dev, cudaStream_t s)
-{
-    HandlePool& h = handles();
-    std::lock_guard<std::mutex> g(h.mu);
-    h.streams.emplace_back(dev, s);
 }
 
 void give_event(int dev, cudaEvent_t e)
@@ -117,6 +97,37 @@ void give_pinned(char* p)
 }
 
 }  // namespace
+
+cudaStream_t take_stream(int dev, int priority)
+{
+    {
+        HandlePool& h = handles();
+        std::lock_guard<std::mutex> g(h.mu);
+        for (size_t k = 0; k < h.streams.size(); ++k)
+            if (h.streams[k].dev == dev && h.streams[k].priority == priority) {
+                cudaStream_t s = h.streams[k].s;
+                h.streams[k] = h.streams.back();
+                h.streams.pop_back();
+                return s;
+            }
+    }
+    cudaStream_t s = nullptr;
+    PARODE_CUDA(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, priority));
+    return s;
+}
+
+void give_stream(int dev, cudaStream_t s, int priority)
+{
+    {
+        HandlePool& h = handles();
+        std::lock_guard<std::mutex> g(h.mu);
+        if (h.streams.size() < kMaxIdleStreams) {
+            h.streams.push_back({dev, priority, s});
+            return;
+        }
+    }
+    cudaStreamDestroy(s);
+}
 
 Plan::Plan(int device, const SystemDesc& sys, InputRegistry* inputs, int uIndex, int solver, double t0,
            double tEnd, double h, const PlanOptions& opt)
@@ -329,31 +340,54 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
     double* st = nullptr;
     double* dPar = nullptr;  // expansion: the input's amplitudes, angular frequencies, phases
     long npow = std::max(levels_, 1);
-    want.emplace_back(&dPow_, npow * (long)Np_ * Np_);
-    want.emplace_back(&dBbar_, (long)n * W * std::max(mB, 1));
+    const bool blocked = !(path_ == kPathLevel || path_ == kPathGeneral);
+    // A small system is discretised on the host (the same operations in the
+    // same order as the device's, so the same bits): up to 20 K multiply-adds,
+    // a few microseconds, against five launches.
+    const bool disc_host = (solver == kRK4 ? 3.0 : 1.0) * n * n * (n + mB) <= 2e4;
+    // ABM start-up inputs of sinusoids on the host, as in a batch (a user
+    // function needs the device, and a wait for it)
+    const bool startup_host = solver == kABM && (mu_ == 0 || (input_->kind == InputEntry::kSinusoid && input_->m >= mu_));
+    double* dra = nullptr;
+    const auto words = [](size_t bytes) { return (long)((bytes + 7) / 8); };
+    // ---- constants, sent in one copy (open_image).  With the host's share above,
+    // a one-shot ABM solve of 4 states and 2000 steps took 188 us, now 103: eleven
+    // copies, five launches and a wait for nine samples less.
+    want.emplace_back(&st, 1);
+    want.emplace_back(&dC_, std::max<long>(1, (long)p_ * n));
+    want.emplace_back(&dD_, std::max<long>(1, (long)p_ * std::max(sys.m, 1)));
+    want.emplace_back(&dX0_, Np_);
+    if (solver == kABM) want.emplace_back(&dYpre_, 3L * p_);
+    if (blocked) want.emplace_back(&dCext_, (long)p_ * Np_);
+    if (br_) want.emplace_back(&dra, words(sizeof(ResponseArgs)));
+    if (ex_) want.emplace_back(&dPar, std::max(1L, 3L * ext_.sh.H / 2));
     // the discretisation's inputs and work (kernels_disc.cu: the host
     // restatement's operation order, so the same bits as host_math.cpp)
     double *dDA = nullptr, *dDB = nullptr, *dPhiC = nullptr, *dDWork = nullptr;
     double *dDJob = nullptr, *dPhiJob = nullptr;
     double* dTiles[3] = {nullptr, nullptr, nullptr};
     long ntiles[3] = {0, 0, 0};
-    {
+    size_t image_end;  // entries of the image; a host-formed Phi is the power table's level 0, right behind them
+    if (disc_host) {
+        want.emplace_back(&dBbar_, (long)n * W * std::max(mB, 1));
+        image_end = want.size();
+    } else {
         const long tn = (n + 31) / 32, tm = mB > 0 ? (mB + 31) / 32 : 0;
         for (int st = 0; st < (solver == kRK4 ? 3 : 1); ++st) ntiles[st] = tn * tn + tn * tm;
-        const auto words = [](size_t bytes) { return (long)((bytes + 7) / 8); };
         want.emplace_back(&dDA, (long)n * n);
         if (mB) want.emplace_back(&dDB, (long)n * mB);
-        want.emplace_back(&dPhiC, (long)n * Ns_);
-        want.emplace_back(&dDWork, discretise_work_doubles(n, mB));
         want.emplace_back(&dDJob, words(sizeof(DiscJob)));
         want.emplace_back(&dPhiJob, words(sizeof(PhiJob)));
         for (int st = 0; st < 3; ++st)
             if (ntiles[st]) want.emplace_back(&dTiles[st], words(sizeof(DiscTile) * (size_t)ntiles[st]));
+        image_end = want.size();
     }
-    want.emplace_back(&dC_, std::max<long>(1, (long)p_ * n));
-    want.emplace_back(&dD_, std::max<long>(1, (long)p_ * std::max(sys.m, 1)));
-    want.emplace_back(&dX0_, Np_);
-    want.emplace_back(&st, 1);
+    want.emplace_back(&dPow_, npow * (long)Np_ * Np_);
+    if (!disc_host) {
+        want.emplace_back(&dBbar_, (long)n * W * std::max(mB, 1));
+        want.emplace_back(&dPhiC, (long)n * Ns_);
+        want.emplace_back(&dDWork, discretise_work_doubles(n, mB));
+    }
     if (path_ == kPathLevel || path_ == kPathGeneral) {
         want.emplace_back(&dV_, (Tp_ + 1) * (long)Np_);  // a leading slot holds the initial state
         if (path_ == kPathGeneral) {
@@ -365,9 +399,7 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         want.emplace_back(&ext_.E, (long)e.pow_levels * e.NP * e.Kc);
         want.emplace_back(&ext_.T, std::max(1L, e.table_rows() * e.Kc));
         want.emplace_back(&ext_.W, (long)e.rows() * e.Kc);
-        want.emplace_back(&dPar, std::max(1L, 3L * e.H / 2));
         want.emplace_back(&dZ_, e.nblocks * e.Kc);
-        want.emplace_back(&dCext_, (long)p_ * Np_);
     } else {
         want.emplace_back(&dG_, nblocks_ * (long)Np_);
         want.emplace_back(&dWork_, std::max(blocked_items_scratch(shape_, nblocks_),
@@ -379,7 +411,7 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
             want.emplace_back(&dTop_, (items + chunk_carry_scratch(items) + 1) * (long)Np_);
         }
         want.emplace_back(&dCP_, (long)shape_.B * p_ * Np_);
-        want.emplace_back(&dCext_, (long)p_ * Np_);
+        if (br_) want.emplace_back(&dW_, (long)(shape_.B * p_ + Np_) * (brKpad_ + Np_));
     }
     want.emplace_back(&dY_, nOut_ * (long)p_);
     if (solver == kRK4) {
@@ -415,9 +447,15 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
     }
     carve(want);
     phase("allocate", false);
+    {
+        char* end = reinterpret_cast<char*>(*want[image_end].first);
+        if (disc_host) end += sizeof(double) * (size_t)Np_ * Np_;
+        open_image(st, (size_t)(end - reinterpret_cast<char*>(st)));
+    }
     dStatus_ = reinterpret_cast<int*>(st);
-    PARODE_CUDA(cudaMemsetAsync(st, 0, sizeof(double), stream_));
-    if (!(path_ == kPathLevel || path_ == kPathGeneral)) {
+    const double zero_word = 0.0;
+    h2d(st, &zero_word, sizeof(double));
+    if (blocked) {
         // output rows of the scan state: C at the state block (the last n of
         // the ABM companion state), or the state itself when C and D are absent
         std::vector<double> Cext((size_t)p_ * Np_, 0.0);
@@ -431,146 +469,68 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
             }
         h2d(dCext_, Cext.data(), sizeof(double) * Cext.size());
     }
-    phase("output rows", false);
-    if (sampled) {
-        // every execute writes all nU x mu samples: only the padding is zeroed
-        if (dU_ && pad) PARODE_CUDA(cudaMemsetAsync(dU_ + nU_ * mu_, 0, sizeof(double) * (size_t)pad, stream_));
-        const size_t used = (size_t)nU_ * mu_;  // rewritten by every execute
-        if (dh) {
-            dUh_ = reinterpret_cast<float*>(dh);
-            PARODE_CUDA(cudaMemsetAsync(dUh_ + used, 0, sizeof(float) * ((size_t)nf - used), stream_));
-        }
-        if (dl) {
-            dUl_ = reinterpret_cast<float*>(dl);
-            PARODE_CUDA(cudaMemsetAsync(dUl_ + used, 0, sizeof(float) * ((size_t)nf - used), stream_));
-        }
-    }
-    phase("padding", true);
-    // ---- discretisation on the device: A and B up, Phi's compact form and
-    // Bbar from the tiled products, Phi expanded into the power table's
-    // level 0 (zero padded; ABM: the shift rows above the last block row)
-    {
-        DiscJob j;
-        j.A = dDA;
-        j.B = mB ? dDB : nullptr;
-        j.phi = dPhiC;
-        j.bbar = dBbar_;
-        j.work = dDWork;
-        j.delta = nullptr;  // the distance to the exact part sizes batch layouts only
-        j.n = n;
-        j.m = mB;
-        j.solver = solver;
-        j.h = h;
-        h2d(dDA, sys.A.data(), sizeof(double) * (size_t)n * n);
-        if (mB) h2d(dDB, sys.B.data(), sizeof(double) * (size_t)n * mB);
-        h2d(dDJob, &j, sizeof j);
-        const DiscTile* dt[3] = {nullptr, nullptr, nullptr};
-        for (int st = 0; st < 3; ++st) {
-            if (!ntiles[st]) continue;
-            std::vector<DiscTile> tl;
-            tl.reserve((size_t)ntiles[st]);
-            discretise_tiles(j, st, tl);
-            if ((long)tl.size() != ntiles[st]) throw Error(kDeviceError, "discretisation tiles: count mismatch");
-            h2d(dTiles[st], tl.data(), sizeof(DiscTile) * tl.size());
-            dt[st] = reinterpret_cast<const DiscTile*>(dTiles[st]);
-        }
-        // no transpose, no distance: the finish's elements spread over CTAs
-        const int parts = std::max(1, std::min(32, (n * n + 255) / 256));
-        launch_discretise_batch(reinterpret_cast<const DiscJob*>(dDJob), 1, dt, ntiles, sms_, stream_, parts);
-        PhiJob pj;
-        pj.dst = dPow_;
-        pj.src = dPhiC;
-        pj.n = n;
-        pj.Np = Np_;
-        pj.solver = solver;
-        h2d(dPhiJob, &pj, sizeof pj);
-        launch_phi_batch(reinterpret_cast<const PhiJob*>(dPhiJob), 1, (long)Np_ * Np_, stream_);
-    }
-    phase("discretise (device)", true);
     if (!sys.zeroC)
         h2d(dC_, sys.C.data(), sizeof(double) * (size_t)p_ * n);
     if (!sys.zeroD)
         h2d(dD_, sys.D.data(), sizeof(double) * (size_t)p_ * sys.m);
-
     // ---- initial scan state -------------------------------------------------
-    if (solver == kRK4) {
-        for (int r = 0; r < n; ++r) X0[r] = sys.x0[r];
-    } else {
-        // start-up inputs u(t0 + j h/2), j = 0..8, evaluated on the device
-        // as the reference does (Sources/AdamsMoulton.cpp:51-88)
-        std::vector<double> U9((size_t)9 * std::max(sys.m, 1), 0.0);
-        if (mu_ > 0) {
-            double* dU9 = nullptr;
-            alloc(&dU9, 9L * mu_);
-            inputs_->fill(input_, device_, dU9, mu_, t0, 0.5 * h, 9, opt_.input_double, stream_);
-            PARODE_CUDA(cudaMemcpyAsync(U9.data(), dU9, sizeof(double) * 9 * mu_, cudaMemcpyDeviceToHost, stream_));
-            PARODE_CUDA(cudaStreamSynchronize(stream_));
-        }
-        SystemDesc s0 = sys;
-        if (s0.zeroB) s0.m = 0;
-        std::vector<double> Xs((size_t)4 * n);
-        abm_startup(s0, U9.data(), h, Xs.data());
-        for (int r = 0; r < 4 * n; ++r) X0[r] = Xs[r];
-        // outputs 0..2 from the start-up states (Sources/GPUFixedStepIterative.cpp:150-172)
-        ypre_.assign((size_t)3 * p_, 0.0);
-        for (int i = 0; i < 3; ++i) {
-            const double* x = &Xs[(size_t)i * n];
-            const double* u = &U9[(size_t)(2 * i) * std::max(sys.m, 1)];
-            for (int o = 0; o < p_; ++o) {
-                double v = 0.0;
-                if (sys.zeroC && sys.zeroD) {
-                    v = x[o];
-                } else {
-                    if (!sys.zeroC)
-                        for (int c = 0; c < n; ++c) v += sys.C[(size_t)o * n + c] * x[c];
-                    if (!sys.zeroD)
-                        for (int c = 0; c < sys.m; ++c) v += sys.D[(size_t)o * sys.m + c] * u[c];
+    auto startup = [&] {
+        if (solver == kRK4) {
+            for (int r = 0; r < n; ++r) X0[r] = sys.x0[r];
+        } else {
+            // start-up inputs u(t0 + j h/2), j = 0..8 (the reference evaluates them on
+            // the device, Sources/AdamsMoulton.cpp:51-88)
+            std::vector<double> U9((size_t)9 * std::max(sys.m, 1), 0.0);
+            if (startup_host) {
+                for (int j = 0; j < 9; ++j)
+                    for (int c = 0; c < mu_; ++c) U9[(size_t)j * mu_ + c] = sinusoid_host(input_, c, t0 + j * 0.5 * h);
+            } else {
+                double* dU9 = nullptr;
+                alloc(&dU9, 9L * mu_);
+                inputs_->fill(input_, device_, dU9, mu_, t0, 0.5 * h, 9, opt_.input_double, stream_);
+                PARODE_CUDA(cudaMemcpyAsync(U9.data(), dU9, sizeof(double) * 9 * mu_, cudaMemcpyDeviceToHost, stream_));
+                PARODE_CUDA(cudaStreamSynchronize(stream_));
+            }
+            SystemDesc s0 = sys;
+            if (s0.zeroB) s0.m = 0;
+            std::vector<double> Xs((size_t)4 * n);
+            abm_startup(s0, U9.data(), h, Xs.data());
+            for (int r = 0; r < 4 * n; ++r) X0[r] = Xs[r];
+            // outputs 0..2 from the start-up states (Sources/GPUFixedStepIterative.cpp:150-172)
+            ypre_.assign((size_t)3 * p_, 0.0);
+            for (int i = 0; i < 3; ++i) {
+                const double* x = &Xs[(size_t)i * n];
+                const double* u = &U9[(size_t)(2 * i) * std::max(sys.m, 1)];
+                for (int o = 0; o < p_; ++o) {
+                    double v = 0.0;
+                    if (sys.zeroC && sys.zeroD) {
+                        v = x[o];
+                    } else {
+                        if (!sys.zeroC)
+                            for (int c = 0; c < n; ++c) v += sys.C[(size_t)o * n + c] * x[c];
+                        if (!sys.zeroD)
+                            for (int c = 0; c < sys.m; ++c) v += sys.D[(size_t)o * sys.m + c] * u[c];
+                    }
+                    ypre_[(size_t)i * p_ + o] = v;
                 }
-                ypre_[(size_t)i * p_ + o] = v;
             }
+            h2d(dYpre_, ypre_.data(), sizeof(double) * ypre_.size());
         }
-        alloc(&dYpre_, 3L * p_);
-        h2d(dYpre_, ypre_.data(), sizeof(double) * ypre_.size());
-    }
-    h2d(dX0_, X0.data(), sizeof(double) * Np_);
-    phase("copies+start-up", true);
-    if (ex_) {
-        ext_.solver = solver;
-        ext_.n = n;
-        ext_.mu = mu_;
-        ext_.terms = mu_ > 0 ? input_->K : 0;
-        ext_.zeroB = sys.zeroB || mu_ == 0;
-        ext_.zeroD = sys.zeroD || mu_ == 0;
-        ext_.dt = u_dt_;
-        ext_.Phi = dPow_;
-        ext_.Bbar = dBbar_;
-        ext_.Cext = dCext_;
-        ext_.D = dD_;
-        ext_.par = dPar;
-        if (mu_ > 0) {
-            // the parameters of the system's channels, the angular frequency rounded as the samplers round it
-            const size_t q = (size_t)mu_ * input_->K;
-            std::vector<double> par(3 * q);
-            for (size_t k = 0; k < q; ++k) {
-                par[k] = input_->a[k];
-                par[q + k] = 6.283185307179586476925286766559 * input_->f[k];
-                par[2 * q + k] = input_->phi[k];
-            }
-            h2d(dPar, par.data(), sizeof(double) * par.size());
+        h2d(dX0_, X0.data(), sizeof(double) * Np_);
+    };
+    if (solver == kRK4 || startup_host) startup();
+    if (ex_ && mu_ > 0) {
+        // the parameters of the system's channels, the angular frequency rounded as the samplers round it
+        const size_t q = (size_t)mu_ * input_->K;
+        std::vector<double> par(3 * q);
+        for (size_t k = 0; k < q; ++k) {
+            par[k] = input_->a[k];
+            par[q + k] = 6.283185307179586476925286766559 * input_->f[k];
+            par[2 * q + k] = input_->phi[k];
         }
-        launch_expand_tables(ext_, stream_);
-        phase("expansion tables", true);
+        h2d(dPar, par.data(), sizeof(double) * par.size());
     }
     if (br_) {
-        // the carry's powers P_1 .. P_levels (Phi^(2^l)) depend on Phi alone:
-        // formed once here, on the side stream beside W (both only read level 0)
-        PARODE_CUDA(cudaEventRecord(fork_[0], stream_));
-        PARODE_CUDA(cudaStreamWaitEvent(side_, fork_[0], 0));
-        launch_blocked_tables(shape_, dPow_, 1, levels_, nullptr, nullptr, p_, side_);
-        PARODE_CUDA(cudaEventRecord(fork_[1], side_));
-        tables_forked = true;
-        // block response matrix from Phi (power-table level 0), Bbar, Cext, D
-        alloc(&dW_, (long)(shape_.B * p_ + Np_) * (brKpad_ + Np_));
         ResponseArgs ra;
         ra.solver = solver;
         ra.n = n;
@@ -588,9 +548,102 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         ra.K = brK_;
         ra.Kpad = brKpad_;
         ra.NPstate = Np_;
-        double* dra = nullptr;
-        alloc(&dra, (long)((sizeof(ResponseArgs) + 7) / 8));
         h2d(dra, &ra, sizeof(ra));
+    }
+    // ---- discretisation: Phi's compact form and Bbar, Phi expanded into the
+    // power table's level 0 (zero padded; ABM: the shift rows above the last
+    // block row); on the device from the tiled products
+    const DiscTile* dt[3] = {nullptr, nullptr, nullptr};
+    if (disc_host) {
+        std::vector<double> phi((size_t)n * Ns_), bbar((size_t)n * W * std::max(mB, 1)), p0((size_t)Np_ * Np_, 0.0);
+        discretise_host(solver, n, Ns_, W, h, sys, phi.data(), bbar.data(), nullptr);
+        const int top = solver == kRK4 ? 0 : 3 * n;
+        for (int r = 0; r < top; ++r) p0[(size_t)r * Np_ + r + n] = 1.0;
+        for (int r = 0; r < n; ++r)
+            std::copy(&phi[(size_t)r * Ns_], &phi[(size_t)(r + 1) * Ns_], &p0[(size_t)(top + r) * Np_]);
+        h2d(dBbar_, bbar.data(), sizeof(double) * bbar.size());
+        h2d(dPow_, p0.data(), sizeof(double) * p0.size());
+    } else {
+        DiscJob j;
+        j.A = dDA;
+        j.B = mB ? dDB : nullptr;
+        j.phi = dPhiC;
+        j.bbar = dBbar_;
+        j.work = dDWork;
+        j.delta = nullptr;  // the distance to the exact part sizes batch layouts only
+        j.n = n;
+        j.m = mB;
+        j.solver = solver;
+        j.h = h;
+        h2d(dDA, sys.A.data(), sizeof(double) * (size_t)n * n);
+        if (mB) h2d(dDB, sys.B.data(), sizeof(double) * (size_t)n * mB);
+        h2d(dDJob, &j, sizeof j);
+        for (int st = 0; st < 3; ++st) {
+            if (!ntiles[st]) continue;
+            std::vector<DiscTile> tl;
+            tl.reserve((size_t)ntiles[st]);
+            discretise_tiles(j, st, tl);
+            if ((long)tl.size() != ntiles[st]) throw Error(kDeviceError, "discretisation tiles: count mismatch");
+            h2d(dTiles[st], tl.data(), sizeof(DiscTile) * tl.size());
+            dt[st] = reinterpret_cast<const DiscTile*>(dTiles[st]);
+        }
+        PhiJob pj;
+        pj.dst = dPow_;
+        pj.src = dPhiC;
+        pj.n = n;
+        pj.Np = Np_;
+        pj.solver = solver;
+        h2d(dPhiJob, &pj, sizeof pj);
+    }
+    flush_image();
+    phase("constants", true);
+    if (sampled) {
+        // every execute writes all nU x mu samples: only the padding is zeroed
+        if (dU_ && pad) PARODE_CUDA(cudaMemsetAsync(dU_ + nU_ * mu_, 0, sizeof(double) * (size_t)pad, stream_));
+        const size_t used = (size_t)nU_ * mu_;  // rewritten by every execute
+        if (dh) {
+            dUh_ = reinterpret_cast<float*>(dh);
+            PARODE_CUDA(cudaMemsetAsync(dUh_ + used, 0, sizeof(float) * ((size_t)nf - used), stream_));
+        }
+        if (dl) {
+            dUl_ = reinterpret_cast<float*>(dl);
+            PARODE_CUDA(cudaMemsetAsync(dUl_ + used, 0, sizeof(float) * ((size_t)nf - used), stream_));
+        }
+    }
+    if (!disc_host) {
+        // no transpose, no distance: the finish's elements spread over CTAs
+        const int parts = std::max(1, std::min(32, (n * n + 255) / 256));
+        launch_discretise_batch(reinterpret_cast<const DiscJob*>(dDJob), 1, dt, ntiles, sms_, stream_, parts);
+        launch_phi_batch(reinterpret_cast<const PhiJob*>(dPhiJob), 1, (long)Np_ * Np_, stream_);
+    }
+    phase("discretise", true);
+    if (solver == kABM && !startup_host) startup();
+    phase("copies+start-up", true);
+    if (ex_) {
+        ext_.solver = solver;
+        ext_.n = n;
+        ext_.mu = mu_;
+        ext_.terms = mu_ > 0 ? input_->K : 0;
+        ext_.zeroB = sys.zeroB || mu_ == 0;
+        ext_.zeroD = sys.zeroD || mu_ == 0;
+        ext_.dt = u_dt_;
+        ext_.Phi = dPow_;
+        ext_.Bbar = dBbar_;
+        ext_.Cext = dCext_;
+        ext_.D = dD_;
+        ext_.par = dPar;
+        launch_expand_tables(ext_, stream_);
+        phase("expansion tables", true);
+    }
+    if (br_) {
+        // the carry's powers P_1 .. P_levels (Phi^(2^l)) depend on Phi alone:
+        // formed once here, on the side stream beside W (both only read level 0)
+        PARODE_CUDA(cudaEventRecord(fork_[0], stream_));
+        PARODE_CUDA(cudaStreamWaitEvent(side_, fork_[0], 0));
+        launch_blocked_tables(shape_, dPow_, 1, levels_, nullptr, nullptr, p_, side_);
+        PARODE_CUDA(cudaEventRecord(fork_[1], side_));
+        tables_forked = true;
+        // block response matrix from Phi (power-table level 0), Bbar, Cext, D
         launch_block_response(reinterpret_cast<const ResponseArgs*>(dra), 1, Np_, p_, brKpad_, stream_);
         phase("W", true);
         if (br_tc_) {
@@ -747,6 +800,11 @@ void Plan::h2d(void* dst, const void* src, size_t bytes)
         pin_ = take_pinned();
         pin_tried_ = true;
     }
+    char* to = static_cast<char*>(dst);
+    if (image_ && to >= image_ && to + bytes <= image_ + image_bytes_) {
+        std::memcpy(pin_ + (to - image_), src, bytes);
+        return;
+    }
     const size_t at = (pin_used_ + 15) & ~(size_t)15;
     if (pin_ && at + bytes <= kPinBlock) {
         std::memcpy(pin_ + at, src, bytes);
@@ -755,6 +813,26 @@ void Plan::h2d(void* dst, const void* src, size_t bytes)
         return;
     }
     PARODE_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream_));
+}
+
+void Plan::open_image(double* first, size_t bytes)
+{
+    if (!pin_ && !pin_tried_) {
+        pin_ = take_pinned();
+        pin_tried_ = true;
+    }
+    if (!pin_ || pin_used_ > 0 || bytes > kPinBlock / 2) return;  // the copies then go one by one
+    image_ = reinterpret_cast<char*>(first);
+    image_bytes_ = bytes;
+    pin_used_ = bytes;
+}
+
+void Plan::flush_image()
+{
+    if (!image_) return;
+    char* dst = image_;
+    image_ = nullptr;
+    PARODE_CUDA(cudaMemcpyAsync(dst, pin_, image_bytes_, cudaMemcpyHostToDevice, stream_));
 }
 
 void Plan::alloc(double** p, long n)

@@ -66,6 +66,12 @@ struct PlanOptions {
 // large ones on the device), or forced to one side.  Both give the same bits.
 enum DiscretiseAt { kDiscAuto = 0, kDiscHost = 1, kDiscDevice = 2 };
 
+// Idle non-blocking streams of finished plans and batches, kept per device and
+// priority (at most kMaxIdleStreams; the rest are destroyed).  A stream is given
+// back synchronised.
+cudaStream_t take_stream(int device, int priority = 0);
+void give_stream(int device, cudaStream_t s, int priority = 0);
+
 class Plan {
 public:
     Plan(int device, const SystemDesc& sys, InputRegistry* inputs, int uIndex, int solver, double t0, double tEnd,
@@ -212,6 +218,12 @@ private:
     char* pin_ = nullptr;  // pinned staging of the set-up copies (h2d)
     size_t pin_used_ = 0;
     bool pin_tried_ = false;
+    // set-up constants gathered in the pinned block and sent in one copy
+    // (flush_image): device bytes [image_, image_ + image_bytes_)
+    char* image_ = nullptr;
+    size_t image_bytes_ = 0;
+    void open_image(double* first, size_t bytes);
+    void flush_image();
     // the launch list as a CUDA graph (execute): 0 none, 1 executed once into
     // graph_y_, 2 graph ready for graph_y_, -1 capture failed
     int graph_state_ = 0;
