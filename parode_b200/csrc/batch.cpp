@@ -490,6 +490,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
     // guard waits for the stream before they go, also when a step fails)
     cudaStream_t dstream = nullptr;
     std::unique_ptr<HostStage> dstage, ddelta;
+    bool distances = false;
     struct StreamGuard {
         int device, priority;
         cudaStream_t* s;
@@ -536,6 +537,13 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             PARODE_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
             dguard.priority = greatest;
             dstream = take_stream(device_, greatest);
+        }
+        // the distances size the mixed form's tensor-core levels only: without
+        // them the host does not wait for the device
+        bool rows = false;
+        for (const Sys& q : sys_) {
+            distances = distances || (q.precision == kMixed && !q.blocked && !q.ex);
+            rows = rows || q.level_sync();
         }
         Layout D;
         for (int i = 0; i < N; ++i) {  // staged inputs first
@@ -590,7 +598,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             j.bbar = reinterpret_cast<double*>(db + doff[i].bbar);
             j.bbarT = doff[i].bbarT ? reinterpret_cast<double*>(db + doff[i].bbarT) : nullptr;
             j.work = reinterpret_cast<double*>(db + doff[i].work);
-            j.delta = reinterpret_cast<double*>(db + delta_at) + i;
+            j.delta = distances ? reinterpret_cast<double*>(db + delta_at) + i : nullptr;
             j.n = q.n;
             j.m = mB;
             j.solver = q.solver;
@@ -607,10 +615,16 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             dtiles[st] = reinterpret_cast<const DiscTile*>(db + tiles_at[st]);
         }
         PARODE_CUDA(cudaMemcpyAsync(db, hs_data, staged, cudaMemcpyHostToDevice, dstream));
-        launch_discretise_batch(reinterpret_cast<const DiscJob*>(db + jobs_at), N, dtiles, ntiles, sms_, dstream);
-        ddelta = std::make_unique<HostStage>(sizeof(double) * (size_t)N);
-        PARODE_CUDA(cudaMemcpyAsync(ddelta->data(), db + delta_at, sizeof(double) * (size_t)N, cudaMemcpyDeviceToHost,
-                                    dstream));
+        launch_discretise_batch(reinterpret_cast<const DiscJob*>(db + jobs_at), N, dtiles, ntiles, sms_, dstream, rows || distances);
+        if (distances) {
+            ddelta = std::make_unique<HostStage>(sizeof(double) * (size_t)N);
+            PARODE_CUDA(cudaMemcpyAsync(ddelta->data(), db + delta_at, sizeof(double) * (size_t)N, cudaMemcpyDeviceToHost,
+                                        dstream));
+        } else {
+            PARODE_CUDA(cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming));
+            PARODE_CUDA(cudaEventRecord(ready_, dstream));
+            PARODE_CUDA(cudaStreamWaitEvent(stream_, ready_, 0));
+        }
         }
     phase(disc_host ? "discretise (host)" : "discretise (device)", false);
     // ---- constant region: layout first, then the host set-up (threads over
@@ -742,7 +756,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         }
     });
     phase("abm-start-up", false);
-    if (dstream) {
+    if (ddelta) {
         PARODE_CUDA(cudaStreamSynchronize(dstream));
         const double* dl = reinterpret_cast<const double*>(ddelta->data());
         for (int i = 0; i < N; ++i) sys_[i].delta = dl[i];
@@ -1602,7 +1616,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
         launch_level_split(dSplit_ + k, std::min(65535, nSplit_ - k), maxSplitElems_, stream_);
     // no wait for the device here: executes are ordered after the set-up by
     // ready_, and the host images stay alive with the plan
-    PARODE_CUDA(cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming));
+    if (!ready_) PARODE_CUDA(cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming));
     PARODE_CUDA(cudaEventRecord(ready_, stream_));
     host_stage_ = std::move(stage);
     host_jobs_ = std::move(jstage);

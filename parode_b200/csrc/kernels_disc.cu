@@ -6,8 +6,9 @@
 //
 // The matrix products (A^2, A^3, A^4 and A B, A^2 B, A^3 B; ABM needs A^2 and
 // A B) run as grouped GEMMs over 32 x 32 output tiles of every system, one
-// launch per dependency stage, so a large system spreads over many SMs; one
-// CTA per system then forms Phi, Bbar, the transpose and the distance.  Every
+// launch per dependency stage, so a large system spreads over many SMs; a few
+// CTAs per system then form Phi and Bbar, and a second launch, where asked for,
+// the transpose and the distance.  Every
 // product and sum is taken in the order of the host restatement (host_math.cpp:
 // discretise_rk4, discretise_abm_last; its GEMM accumulates each element over
 // the inner index in order, built without FMA contraction): explicit
@@ -78,9 +79,9 @@ __global__ void __launch_bounds__(kThreads) k_disc_gemm(const DiscTile* __restri
     }
 }
 
-// Per system: Phi, Bbar (and its transpose) from the products, then the
-// distance to R.  gridDim.y CTAs share a system's elementwise part (only for
-// jobs without a transpose or a distance, which read all of it).
+// Per system: Phi and Bbar from the products, element by element, gridDim.y CTAs
+// a system (16 systems up to n = 436: 80 us with one CTA a system and the
+// distance in it, 5 in 32 each).
 __global__ void __launch_bounds__(kThreads) k_discretise_finish(const DiscJob* __restrict__ jobs)
 {
     const DiscJob jb = jobs[blockIdx.x];
@@ -147,35 +148,34 @@ __global__ void __launch_bounds__(kThreads) k_discretise_finish(const DiscJob* _
             }
         }
     }
-    __syncthreads();
-    // Bbar transposed (level-synchronous systems' coalesced forcing kernel)
-    if (jb.bbarT) {
-        const int Wm = W * m;
-        for (int e = threadIdx.x; e < max(Wm, 1) * n; e += kThreads) jb.bbarT[e] = 0.0;
-        __syncthreads();
-        for (int e = threadIdx.x; e < n * Wm; e += kThreads) {
-            const int r = e / Wm, c = e - r * Wm;
-            jb.bbarT[(long)c * n + r] = jb.bbar[e];
+    if (tid == 0 && jb.delta) *jb.delta = 0.0;
+}
+
+// The readers of whole rows: Bbar transposed (level-synchronous systems'
+// coalesced forcing kernel) and ||Phi - R||_inf over the stored rows, a thread a
+// row, summed in order (a batch sizes the mixed form's layout with it).
+__global__ void __launch_bounds__(kThreads) k_discretise_rows(const DiscJob* __restrict__ jobs)
+{
+    const DiscJob jb = jobs[blockIdx.x];
+    const int n = jb.n, N = jb.solver == 0 ? n : 4 * n, Wm = (jb.solver == 0 ? 3 : 5) * jb.m;
+    const int tid = blockIdx.y * kThreads + threadIdx.x, nthr = gridDim.y * kThreads;
+    if (jb.bbarT)
+        for (int e = tid; e < n * max(Wm, 1); e += nthr) {
+            const int c = e / n, r = e - c * n;
+            jb.bbarT[e] = Wm > 0 ? jb.bbar[(long)r * Wm + c] : 0.0;
         }
-    }
-    // ||Phi - R||_inf over the stored rows (each row summed in order), when
-    // asked for (a batch sizes its layout with it; a single plan does not)
     if (!jb.delta) return;
-    __shared__ double rowmax[kThreads];
     const int d0 = jb.solver == 0 ? 0 : 3 * n;
     double dmax = 0.0;
-    for (int r = threadIdx.x; r < n; r += kThreads) {
+    for (int r = tid; r < n; r += nthr) {
         double sum = 0.0;
+#pragma unroll 8
         for (int c = 0; c < N; ++c) sum = add(sum, fabs(add(jb.phi[(long)r * N + c], -(c == d0 + r ? 1.0 : 0.0))));
         dmax = fmax(dmax, sum);
     }
-    rowmax[threadIdx.x] = dmax;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double v = 0.0;
-        for (int t = 0; t < kThreads; ++t) v = fmax(v, rowmax[t]);
-        *jb.delta = v;
-    }
+    // non-negative doubles order as their bits
+    if (dmax > 0.0)
+        atomicMax(reinterpret_cast<unsigned long long*>(jb.delta), (unsigned long long)__double_as_longlong(dmax));
 }
 
 void push_tiles(const double* X, const double* Y, double* Z, int r, int k, int c, std::vector<DiscTile>& out)
@@ -221,7 +221,7 @@ void discretise_tiles(const DiscJob& j, int stage, std::vector<DiscTile>& out)
 }
 
 void launch_discretise_batch(const DiscJob* jobs, int njobs, const DiscTile* const tiles[3], const long ntiles[3],
-                             int sms, cudaStream_t s, int parts)
+                             int sms, cudaStream_t s, bool rows)
 {
     for (int st = 0; st < 3; ++st) {
         if (ntiles[st] <= 0) continue;
@@ -229,9 +229,13 @@ void launch_discretise_batch(const DiscJob* jobs, int njobs, const DiscTile* con
         k_disc_gemm<<<(unsigned)grid, kThreads, 0, s>>>(tiles[st], ntiles[st]);
         PARODE_CUDA(cudaGetLastError());
     }
+    const unsigned parts = (unsigned)std::max(1, std::min(32, 4 * std::max(sms, 1) / std::max(njobs, 1)));
     for (int k = 0; k < njobs; k += 65535) {
-        const int cnt = std::min(65535, njobs - k);
-        k_discretise_finish<<<dim3((unsigned)cnt, (unsigned)std::max(parts, 1)), kThreads, 0, s>>>(jobs + k);
+        const dim3 grid((unsigned)std::min(65535, njobs - k), parts);
+        k_discretise_finish<<<grid, kThreads, 0, s>>>(jobs + k);
+        PARODE_CUDA(cudaGetLastError());
+        if (!rows) continue;
+        k_discretise_rows<<<grid, kThreads, 0, s>>>(jobs + k);
         PARODE_CUDA(cudaGetLastError());
     }
 }

@@ -611,9 +611,7 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         }
     }
     if (!disc_host) {
-        // no transpose, no distance: the finish's elements spread over CTAs
-        const int parts = std::max(1, std::min(32, (n * n + 255) / 256));
-        launch_discretise_batch(reinterpret_cast<const DiscJob*>(dDJob), 1, dt, ntiles, sms_, stream_, parts);
+        launch_discretise_batch(reinterpret_cast<const DiscJob*>(dDJob), 1, dt, ntiles, sms_, stream_, false);
         launch_phi_batch(reinterpret_cast<const PhiJob*>(dPhiJob), 1, (long)Np_ * Np_, stream_);
     }
     phase("discretise", true);
