@@ -1152,7 +1152,9 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             // up to 32 columns, a narrow CTA's own width, go to the narrow
             // kernel; up to 512 when the level's tiles would leave SMs idle (one
             // large system, NP = 512, 64 columns: 8 tiles of 64 x 64, 19 us,
-            // against 128 narrow CTAs)
+            // against 128 narrow CTAs); up to 16 when they are many and the
+            // columns' rereads by every row tile count (a thousand systems: 52
+            // against 55 us at 16 columns, 75 against 55 at 32)
             auto may_narrow = [&](const LevelArgs& a) {
                 return (narrow == Narrow::kAll || (narrow == Narrow::kTiled && a.Np > 64)) && a.ncols > 0 &&
                        a.src_ks == 1 && a.dst_is == 1 && !a.cpy && a.K1 == 0 && a.dst_limit < 0 && a.src_cols == 0;
@@ -1160,7 +1162,7 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             long ntiles = 0;
             for (const auto& e : ents)
                 if (may_narrow(e.second)) ntiles += level_tiles(level_config(e.second), e.second);
-            const long cap = ntiles < sms_ ? 512 : 32;
+            const long cap = ntiles < sms_ ? 512 : ntiles < 4 * sms_ ? 32 : 16;
             // mixed form: levels below the top four of a system run on the
             // tensor cores (3xTF32); the top four, where high powers of Phi
             // amplify rounding, stay FP64
@@ -1197,9 +1199,17 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             }
             for (PreparedGroup& G : P.groups) {
                 if (G.cfg.id == 5 || G.cfg.id == 6) {
+                    const LevelConfig small = level_small(G.cfg);
                     long tiles = 0;
-                    for (const LevelArgs& a : G.stored) tiles += level_tiles(G.cfg, a);
-                    if (level_few_tiles(tiles)) G.cfg = level_small(G.cfg);
+                    double work = 0.0, work32 = 0.0;  // products with the tiles' padding
+                    for (const LevelArgs& a : G.stored) {
+                        const long t64 = level_tiles(G.cfg, a), t32 = level_tiles(small, a);
+                        tiles += t64;
+                        work += 4.0 * (double)t64 * (a.K > 0 ? a.K : a.Np);
+                        work32 += (double)t32 * (a.K > 0 ? a.K : a.Np);
+                    }
+                    // small tiles cost up to 3 % more per product in long launches
+                    if (level_few_tiles(tiles) || 1.03 * work32 < work) G.cfg = small;
                 }
                 for (const LevelArgs& a : G.stored) {
                     const LevelConfig c = G.cfg.id >= 5 ? G.cfg : level_config(a);
@@ -1245,10 +1255,13 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
                 GroupedLaunch gl;
                 gl.cfg.id = kNarrowConfig;
                 gl.nent = (int)P.narrow.size();
+                long split = 0;
+                for (const LevelArgs& a : P.narrow) split += expand_narrow_tiles(a, true);
+                gl.split = split <= 8L * sms_;  // two waves at four CTAs an SM
                 std::vector<long> start;
                 for (const LevelArgs& a : P.narrow) {
                     start.push_back(gl.tiles);
-                    gl.tiles += expand_narrow_tiles(a);
+                    gl.tiles += expand_narrow_tiles(a, gl.split);
                 }
                 gl.args = reinterpret_cast<LevelArgs*>(base + jput(P.narrow.data(), sizeof(LevelArgs) * P.narrow.size()));
                 gl.start = reinterpret_cast<long*>(base + jput(start.data(), sizeof(long) * start.size()));
@@ -1962,7 +1975,7 @@ int BatchPlan::launch_chains(cudaStream_t s, std::initializer_list<const std::ve
 
 void BatchPlan::launch_grouped(const GroupedLaunch& g, cudaStream_t s)
 {
-    if (g.cfg.id == kNarrowConfig) launch_expand_narrow(g.args, g.start, g.nent, g.tiles, s);
+    if (g.cfg.id == kNarrowConfig) launch_expand_narrow(g.args, g.start, g.nent, g.tiles, g.split, s);
     else if (g.cfg.id == kTcConfig) launch_level_tc(g.args, g.start, g.nent, g.cta, g.ctas, dStatus_, s);
     else launch_affine_level_grouped(g.cfg, g.args, g.start, g.nent, g.tiles, g.smem, s);
 }

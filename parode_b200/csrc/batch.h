@@ -153,6 +153,7 @@ private:
         int nent = 0;
         long tiles = 0;
         size_t smem = 0;
+        bool split = false;         // narrow launch: K split over a CTA's warps
         LevelArgs* swaps = nullptr;  // device: down-sweep entries of the tiled form, swapped first
         int nswap = 0;
         long swap_elems = 0;

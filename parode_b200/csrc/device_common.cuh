@@ -36,6 +36,24 @@ void launch_dependent(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, 
     PARODE_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
 }
 
+// The entry of a grouped launch that tile t belongs to: the last e with start[e]
+// <= t, start ascending from 0.  A warp looks at 32 entries a round: two trips to
+// L2 for a thousand entries where a bisection makes ten (about 1.5 us of a CTA's
+// life).  All lanes call it and get the same answer.
+__device__ __forceinline__ int find_entry(const long* __restrict__ start, int nent, long t)
+{
+    const int lane = threadIdx.x & 31;
+    int lo = 0;
+    for (int n = nent; n > 1;) {
+        const int step = (n + 31) / 32, at = lane * step;
+        const unsigned le = __ballot_sync(0xffffffffu, at < n && (at == 0 || start[lo + at] <= t));
+        const int k = (31 - __clz(le)) * step;
+        lo += k;
+        n = min(step, n - k);
+    }
+    return lo;
+}
+
 // D(8x8) += A(8x4, row) * B(4x8, col), FP64 tensor-core MMA.
 // Fragments (PTX ISA, mma.m8n8k4 .f64): lane = 4*g + t with g = lane>>2,
 // t = lane&3; A holds A[g][t], B holds B[t][g], D holds D[g][2t], D[g][2t+1].

@@ -103,9 +103,10 @@ LevelArgs expand_level_args(const ExpandJob& j, int l);
 LevelArgs expand_out_args(const ExpandJob& j, double* Y, long limit);
 
 // dst = P src (+ acc, which may be dst) for a few columns (K-contiguous, rows
-// and K multiples of 8): 8 rows x 32 columns per CTA with K split over its warps, where the
-// 64 x 64 tiles would mostly multiply padding.
-long expand_narrow_tiles(const LevelArgs& a);
-void launch_expand_narrow(const LevelArgs* dArgs, const long* dStart, int nent, long tiles, cudaStream_t s);
+// and K multiples of 8), where the square tiles would mostly multiply padding.
+// A tile is 32 columns and 8 rows, K split over the CTA's warps (split), or 32
+// rows, a warp each 8 (launches of many tiles).
+long expand_narrow_tiles(const LevelArgs& a, bool split);
+void launch_expand_narrow(const LevelArgs* dArgs, const long* dStart, int nent, long tiles, bool split, cudaStream_t s);
 
 }  // namespace parode

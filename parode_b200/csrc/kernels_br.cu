@@ -228,17 +228,6 @@ __host__ __device__ inline int resp_wm2(const ResponseArgs& a) { return ((a.solv
 constexpr int kPerThread = 4;
 constexpr int kPerCta = kThreads * kPerThread;
 
-__device__ __forceinline__ int find_entry(const long* __restrict__ start, int nent, long t)
-{
-    int lo = 0, hi = nent - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (start[mid] <= t) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
 // CP_0 = Cext, Q_0 = the identity's forcing columns (n2 = n rounded up to
 // even columns, the last one zero when n is odd), and BbarE = Bbar in the
 // forcing rows of an NP x WM2 zero matrix (WM2 = W m rounded up to even).

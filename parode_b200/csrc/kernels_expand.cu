@@ -545,24 +545,25 @@ __device__ __forceinline__ void narrow_mma(const double* pr, const double* const
     }
 }
 
+// kSplit: CTA = 8 rows, a quarter of K a warp; else a row tile a warp, its whole
+// K.  The first level of a thousand systems (133 MB of powers, 20 us): 79 us in
+// 9.7 K split CTAs that each bisected the entries, 60 with find_entry, 46 a row
+// tile a warp; later levels of as many bytes 75, 39.
+template <bool kSplit>
 __global__ void __launch_bounds__(kNarrowThreads) k_expand_narrow(const LevelArgs* __restrict__ args,
                                                                   const long* __restrict__ start, int nent)
 {
-    __shared__ double2 red[4][4][32];
+    __shared__ double2 red[kSplit ? 4 : 1][4][32];
     const long t = blockIdx.x;
-    int lo = 0, hi = nent - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (start[mid] <= t) lo = mid;
-        else hi = mid - 1;
-    }
+    const int lo = find_entry(start, nent, t);
     const LevelArgs& a = args[lo];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
-    const int rt = level_rows(a) / 8;
+    const int rows = level_rows(a), rt = kSplit ? rows / 8 : (rows + 31) / 32;
     const long u = t - start[lo], c0 = (u / rt) * kNarrowCols;
-    const int r0 = (int)(u % rt) * 8;
+    const int r0 = kSplit ? (int)(u % rt) * 8 : (int)(u % rt) * 32 + 8 * warp;
+    if (!kSplit && r0 >= rows) return;
     const int cols = (int)min((long)kNarrowCols, a.ncols - c0), ct = (cols + 7) / 8;
-    const int n8 = level_k(a) / 8, k0 = n8 * warp / 4, k1 = n8 * (warp + 1) / 4;
+    const int n8 = level_k(a) / 8, k0 = kSplit ? n8 * warp / 4 : 0, k1 = kSplit ? n8 * (warp + 1) / 4 : n8;
     const double* pr = a.P + (long)(r0 + g) * a.ldp + 2 * tq;
     const double* z[4];
 #pragma unroll
@@ -574,22 +575,31 @@ __global__ void __launch_bounds__(kNarrowThreads) k_expand_narrow(const LevelArg
     case 3: narrow_mma<3>(pr, z, k0, k1, acc); break;
     default: narrow_mma<4>(pr, z, k0, k1, acc); break;
     }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) red[warp][c][lane] = make_double2(acc[c][0], acc[c][1]);
-    __syncthreads();
-    if (8 * warp + g < cols) {  // this warp stores column tile `warp`
-        double2 v = red[0][warp][lane];
-#pragma unroll
-        for (int w = 1; w < 4; ++w) {
-            v.x += red[w][warp][lane].x;
-            v.y += red[w][warp][lane].y;
-        }
+    auto store = [&](int c, double2 v) {  // column tile c
         if (a.acc) {
-            const double2 o = *reinterpret_cast<const double2*>(a.acc + (c0 + 8 * warp + g) * a.acc_gs + r0 + 2 * tq);
+            const double2 o = *reinterpret_cast<const double2*>(a.acc + (c0 + 8 * c + g) * a.acc_gs + r0 + 2 * tq);
             v.x += o.x;
             v.y += o.y;
         }
-        *reinterpret_cast<double2*>(a.dst + (c0 + 8 * warp + g) * a.dst_gs + r0 + 2 * tq) = v;
+        *reinterpret_cast<double2*>(a.dst + (c0 + 8 * c + g) * a.dst_gs + r0 + 2 * tq) = v;
+    };
+    if constexpr (kSplit) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) red[warp][c][lane] = make_double2(acc[c][0], acc[c][1]);
+        __syncthreads();
+        if (8 * warp + g < cols) {  // this warp stores column tile `warp`
+            double2 v = red[0][warp][lane];
+#pragma unroll
+            for (int w = 1; w < 4; ++w) {
+                v.x += red[w][warp][lane].x;
+                v.y += red[w][warp][lane].y;
+            }
+            store(warp, v);
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (8 * c + g < cols) store(c, make_double2(acc[c][0], acc[c][1]));
     }
 }
 
@@ -859,12 +869,16 @@ LevelArgs expand_out_args(const ExpandJob& j, double* Y, long limit)
     return a;
 }
 
-long expand_narrow_tiles(const LevelArgs& a) { return (long)(level_rows(a) / 8) * ((a.ncols + kNarrowCols - 1) / kNarrowCols); }
+long expand_narrow_tiles(const LevelArgs& a, bool split)
+{
+    return (long)(split ? level_rows(a) / 8 : (level_rows(a) + 31) / 32) * ((a.ncols + kNarrowCols - 1) / kNarrowCols);
+}
 
-void launch_expand_narrow(const LevelArgs* dArgs, const long* dStart, int nent, long tiles, cudaStream_t s)
+void launch_expand_narrow(const LevelArgs* dArgs, const long* dStart, int nent, long tiles, bool split, cudaStream_t s)
 {
     if (tiles <= 0) return;
-    k_expand_narrow<<<(unsigned)tiles, kNarrowThreads, 0, s>>>(dArgs, dStart, nent);
+    if (split) k_expand_narrow<true><<<(unsigned)tiles, kNarrowThreads, 0, s>>>(dArgs, dStart, nent);
+    else k_expand_narrow<false><<<(unsigned)tiles, kNarrowThreads, 0, s>>>(dArgs, dStart, nent);
     PARODE_CUDA(cudaGetLastError());
 }
 

@@ -58,12 +58,7 @@ __global__ void __launch_bounds__(kThreads) k_affine_level_grouped(const LevelAr
 {
     extern __shared__ double smem[];
     const long t = blockIdx.x;
-    int lo = 0, hi = nent - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (start[mid] <= t) lo = mid;
-        else hi = mid - 1;
-    }
+    const int lo = find_entry(start, nent, t);
     const LevelArgs a = args[lo];
     if (FR == 1) CW = 8 / affine_row_warps(a.Np);  // entries of all scan dimensions up to 64 share a launch
     affine_level_body<FR, FC>(a, t - start[lo], CW, level_ks(a.Np), smem);
@@ -420,12 +415,7 @@ __global__ void __launch_bounds__(Tile<T>::threads, T == 64 ? 2 : 4) k_level_til
 {
     extern __shared__ __align__(16) double smem[];
     const long t = blockIdx.x;
-    int lo = 0, hi = nent - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (start[mid] <= t) lo = mid;
-        else hi = mid - 1;
-    }
+    const int lo = find_entry(start, nent, t);
     const LevelArgs a = args[lo];
     tiled_level_body<kKC, T>(a, t - start[lo], smem);
 }

@@ -43,3 +43,23 @@ def test_levels_match_oracle(pb, k, path):
             assert y.shape == ref.shape
             assert oracle.rel_err(y, ref) <= 1e-11, (i, rep)
     batch.close()
+
+
+def test_many_systems_in_one_launch(pb):
+    """A batch whose levels are launches of thousands of tiles: entries found
+    among several hundred, a row tile per warp in the narrow kernel, 32-row
+    tiles where 64 would be padding.  Mixed form (the expansion, FP64 phases):
+    gate 1e-10, as for its single plans."""
+    cases = [wl.small(33000 + i, i % 2, 3 + (7 * i) % 60, 1 + i % 3, 2, 1500 + 37 * (i % 41), h=1e-3) for i in range(400)]
+    specs = [dict(A=c.A, B=c.B, C=c.C, D=c.D, x0=c.x0, u=pb.register_sinusoid(c.u.a, c.u.f, c.u.phi), solver=c.solver,
+                  t0=c.t0, t_end=c.t_end, h=c.h) for c in cases]
+    batch = pb.Batch(specs, precision=pb.MIXED)
+    batch.execute()
+    for i in list(range(0, 400, 23)) + [1, 398, 399]:
+        c = cases[i]
+        _, y = batch.output(i)
+        ref = oracle.simulate_affine(oracle.System(c.A, c.B, c.C, c.D, c.x0), oracle.Input.sinusoid(c.u.a, c.u.f, c.u.phi),
+                                     c.solver, c.t0, c.t_end, c.h)
+        assert y.shape == ref.shape
+        assert oracle.rel_err(y, ref) <= 1e-10, i
+    batch.close()
