@@ -69,9 +69,12 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // a level took 8 us at NP = 64, Kc = 112, 0.16 ms for 20 levels.
 constexpr int kSqCtas = 8;
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_barrier()
 {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 
 __device__ __forceinline__ void store_remote(double* local, unsigned rank, double v0, double v1)
@@ -85,6 +88,7 @@ __device__ __forceinline__ void store_remote(double* local, unsigned rank, doubl
 __global__ void __cluster_dims__(kSqCtas, 1, 1) __launch_bounds__(kThreads, 1) k_expand_squarings(const ExpandTables t)
 {
     extern __shared__ __align__(16) double sm[];
+    cluster_arrive();  // waited for before the first store into a peer's shared memory
     const int NP = t.sh.NP, Kc = t.sh.Kc, ld = NP + 4;  // 4 mod 8 doubles: conflict-free fragments
     const int rank = blockIdx.x;
     const int HQ = t.sh.H / 2, n = t.n, m = t.mu, K = t.terms;
@@ -119,6 +123,10 @@ __global__ void __cluster_dims__(kSqCtas, 1, 1) __launch_bounds__(kThreads, 1) k
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
     const int MT = NP / 8;
     int cur = 0;
+    // every CTA of the cluster runs: its shared memory may be written (the
+    // ranks' S_1 take different times, none at all without inputs)
+    __syncwarp();
+    cluster_wait();
     for (int l = 0;; ++l) {
         for (int u = threadIdx.x; u < 4 * own; u += kThreads) {
             const int q = ((u / 4) * kSqCtas + rank) * 4 + u % 4;
