@@ -693,14 +693,16 @@ __device__ void tables_body(double* P, int l0, int l1, double* CP, const double*
     }
 }
 
-template <class K>
-void set_smem(K kernel, size_t bytes)
-{
-    PARODE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-}
-
 constexpr size_t kSmemCap = 220 * 1024;
 constexpr size_t kSmemOptInMax = 232448 - 1024;  // 227 KB per CTA on sm_100, less a little headroom
+
+// The limit is the function's, for all host threads: always the same one,
+// whatever the launch needs.
+template <class K>
+void set_smem(K kernel)
+{
+    PARODE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemOptInMax));
+}
 
 }  // namespace
 
@@ -744,7 +746,7 @@ static void leaf_t(const BlockedShape& sh, const LeafArgs& a, int grid, cudaStre
 {
     size_t smem = a.stage ? blocked_leaf_stage_bytes(sh, a.n, a.m, a.p, a.solver) : sh.leaf_smem;
     if (smem == 0) throw Error(kInvalidArgument, "leaf staging does not fit");
-    set_smem(k_leaf<NP>, smem);
+    set_smem(k_leaf<NP>);
     unsigned g = (unsigned)std::max<long>(1, std::min<long>(a.ntiles, grid));
     k_leaf<NP><<<g, kThreads, smem, s>>>(a, sh.R, sh.S);
     PARODE_CUDA(cudaGetLastError());
@@ -781,8 +783,8 @@ static int carry_t(const BlockedShape& sh, double* items, long count, int base_l
     std::vector<long> cnt{count};
     std::vector<int> lev{base_level};
     int launches = 0;
-    set_smem(k_items_up<NP>, sh.items_smem);
-    set_smem(k_items_down<NP>, sh.items_smem);
+    set_smem(k_items_up<NP>);
+    set_smem(k_items_down<NP>);
     double* w = work;
     while (cnt.back() > sh.S_items) {
         long c = cnt.back();
@@ -802,7 +804,7 @@ static int carry_t(const BlockedShape& sh, double* items, long count, int base_l
         int L = 1;
         while (L < c) L <<= 1;
         size_t smem = (mat + (size_t)L * NP) * sizeof(double);
-        set_smem(k_items_top<NP>, smem);
+        set_smem(k_items_top<NP>);
         k_items_top<NP><<<1, kThreads, smem, s>>>(arr.back(), c, P + lev.back() * mat, L, X0);
         PARODE_CUDA(cudaGetLastError());
         ++launches;
@@ -859,7 +861,7 @@ static void tables_t(const BlockedShape& sh, double* P, int l0, int l1, double* 
                      cudaStream_t s)
 {
     size_t smem = 2 * (size_t)NP * NP * sizeof(double);
-    set_smem(k_tables<NP>, smem);
+    set_smem(k_tables<NP>);
     k_tables<NP><<<1, kThreads, smem, s>>>(P, l0, l1, CP, Cext, p, sh.R);
     PARODE_CUDA(cudaGetLastError());
 }
@@ -911,12 +913,12 @@ static void batch_t(int what, const BlockedShape& sh, const BatchLaunch& b, cuda
     switch (what) {
     case 0: {
         size_t smem = 2 * (size_t)NP * NP * sizeof(double);
-        set_smem(k_tables_batch<NP>, smem);
+        set_smem(k_tables_batch<NP>);
         k_tables_batch<NP><<<b.nsys, kThreads, smem, s>>>(b.sys, b.CPs, b.Cexts, sh.R + 1, sh.R);
         break;
     }
     case 1: {
-        set_smem(k_leaf_batch<NP>, b.leaf_smem);
+        set_smem(k_leaf_batch<NP>);
         k_leaf_batch<NP><<<b.grid, kThreads, b.leaf_smem, s>>>(b.sys, b.items, b.nitems, sh.R, sh.S, b.ms);
         break;
     }

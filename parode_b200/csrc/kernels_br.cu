@@ -31,6 +31,7 @@ namespace {
 
 constexpr int kCols = 8;        // window columns per CTA (a cfg2 W: 41 CTAs)
 constexpr int kThreads = 256;
+constexpr size_t kSmemMax = 220 * 1024;
 
 // z (NP x kCols, row-major in shared memory): z <- Phi z + S_j, and the
 // output rows of step j, for the CTA's columns [c0, c0 + kCols).
@@ -200,8 +201,8 @@ template <int NP>
 void block_response_mma_t(const ResponseArgs* dArgs, int max_p, int max_kpad, cudaStream_t s)
 {
     const size_t smem = (2 * (size_t)NP * (kCols + 4) + (size_t)max_p * NP) * sizeof(double);
-    if (smem > 220 * 1024) throw Error(kInvalidArgument, "block response: shared memory");
-    PARODE_CUDA(cudaFuncSetAttribute(k_block_response_mma<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kSmemMax) throw Error(kInvalidArgument, "block response: shared memory");
+    PARODE_CUDA(cudaFuncSetAttribute(k_block_response_mma<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     dim3 grid((unsigned)((max_kpad + NP + kCols - 1) / kCols), 1);
     k_block_response_mma<NP><<<grid, kThreads, smem, s>>>(dArgs);
     PARODE_CUDA(cudaGetLastError());
@@ -486,8 +487,8 @@ void launch_block_response(const ResponseArgs* dArgs, int nsys, int max_np, int 
         }
     }
     const size_t smem = ((size_t)max_np * max_np + 2 * (size_t)max_np * kCols + (size_t)max_p * max_np) * sizeof(double);
-    if (smem > 220 * 1024) throw Error(kInvalidArgument, "block response: shared memory");
-    PARODE_CUDA(cudaFuncSetAttribute(k_block_response, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kSmemMax) throw Error(kInvalidArgument, "block response: shared memory");
+    PARODE_CUDA(cudaFuncSetAttribute(k_block_response, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     dim3 grid((unsigned)((max_kpad + max_np + kCols - 1) / kCols), (unsigned)nsys);
     k_block_response<<<grid, kThreads, smem, s>>>(dArgs);
     PARODE_CUDA(cudaGetLastError());

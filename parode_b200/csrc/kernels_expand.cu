@@ -654,7 +654,7 @@ void out_t(const ExpandTables& t, const double* Z, double* Y, long c0, long c1, 
     const int Ms = (tiles8 + slices - 1) / slices * 8;
     slices = (M + Ms - 1) / Ms;
     const size_t smem = (size_t)Ms * ld * sizeof(double);
-    PARODE_CUDA(cudaFuncSetAttribute(k_expand_out<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PARODE_CUDA(cudaFuncSetAttribute(k_expand_out<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     // CTAs: no more than the SMs, each with at least a row tile per warp
     const long ctas = std::max<long>(slices, std::min<long>(sms, nt * tiles8 / warps));
     const long gs = M;
@@ -731,7 +731,7 @@ void launch_expand_tables(const ExpandTables& t, cudaStream_t s)
 {
     const int maxown = ((t.sh.Kc - t.sh.NP) / 8 + kSqCtas - 1) / kSqCtas;
     size_t smem = (2 * (size_t)t.sh.NP * (t.sh.NP + 4 + 8 * maxown + 4) + 8 * maxown) * sizeof(double);
-    PARODE_CUDA(cudaFuncSetAttribute(k_expand_squarings, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PARODE_CUDA(cudaFuncSetAttribute(k_expand_squarings, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     k_expand_squarings<<<kSqCtas, kThreads, smem, s>>>(t);
     PARODE_CUDA(cudaGetLastError());
     const int out_tiles = (t.sh.rows() + 7) / 8;
@@ -784,8 +784,9 @@ int expand_log2_block(int NP, int Kc, int p, long nScan, double executions)
 
 void launch_expand_init(const ExpandJob* dJobs, int njobs, int max_hq, long max_elems, cudaStream_t s)
 {
+    // within the 48 KB that need no limit of the function's own
+    static_assert(sizeof(double) * 2 * 5 * kExpandMaxPairs <= 48 * 1024, "trig table");
     const size_t smem = sizeof(double) * 2 * 5 * (size_t)std::max(max_hq, 1);
-    PARODE_CUDA(cudaFuncSetAttribute(k_expand_init_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_expand_init_batch<<<dim3(batch_x(max_elems, njobs), (unsigned)njobs), kThreads, smem, s>>>(dJobs);
     PARODE_CUDA(cudaGetLastError());
 }

@@ -33,6 +33,7 @@ namespace {
 using namespace tc05;
 
 constexpr int kTcThreads = 256;
+constexpr size_t kSmemMax = 232448 - 1024;  // 227 KB per CTA on sm_100, less a little headroom
 constexpr long long kWaitLimit = 1LL << 31;  // SM cycles (about a second) before a wait gives up
 
 struct TcLayout {
@@ -414,7 +415,7 @@ void leaf_tc_t(const BlockedShape& sh, const LeafArgs& a, int grid, cudaStream_t
     int tcols = 32;
     while (tcols < slices * NP) tcols <<= 1;
     if (tcols > 512) throw Error(kInvalidArgument, "mixed leaf: TMEM columns exceed 512");
-    PARODE_CUDA(cudaFuncSetAttribute(k_leaf_tc<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+    PARODE_CUDA(cudaFuncSetAttribute(k_leaf_tc<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     unsigned g = (unsigned)std::max<long>(1, std::min<long>(a.ntiles, grid));
     k_leaf_tc<NP><<<g, kTcThreads, L.total, s>>>(a, sh.R, sh.S, tcols);
     PARODE_CUDA(cudaGetLastError());
@@ -428,7 +429,7 @@ size_t blocked_leaf_tc_bytes(const BlockedShape& sh, int n, int m, int p, int so
     if (sh.S < 128 || sh.S < 4 * sh.B || sh.S % sh.B != 0) return 0;
     if (((sh.S + 127) >> 7) * sh.NP > 512) return 0;
     TcLayout L = tc_layout(sh.NP, sh.R, sh.S, n, m, p, solver);
-    return L.total <= 232448 - 1024 ? L.total : 0;
+    return L.total <= kSmemMax ? L.total : 0;
 }
 
 void launch_blocked_leaf_tc(const BlockedShape& sh, const LeafArgs& a, int grid, cudaStream_t s)

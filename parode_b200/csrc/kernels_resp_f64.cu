@@ -261,7 +261,7 @@ bool launch_resp_f64(const LevelArgs& l, int sms, cudaStream_t s)
         used += (int)n;
     }
     a.cta0[a.slices] = (short)used;
-    PARODE_CUDA(cudaFuncSetAttribute(k_resp_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PARODE_CUDA(cudaFuncSetAttribute(k_resp_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     launch_dependent(k_resp_f64, dim3((unsigned)used), dim3(kThreads), smem, s, a);
     return true;
 }

@@ -27,6 +27,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
+constexpr size_t kSmemMax = 200 * 1024;
 
 template <int NP>
 constexpr int kpitch()
@@ -104,8 +105,8 @@ bool state_t(const double* W, long ld, int M, const double* X, const double* acc
 {
     const int Mp = (M + 7) & ~7;
     const size_t smem = state_smem<NP>(Mp);
-    if (smem > 200 * 1024) return false;
-    PARODE_CUDA(cudaFuncSetAttribute(k_state_out<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kSmemMax) return false;
+    PARODE_CUDA(cudaFuncSetAttribute(k_state_out<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     int per_sm = 0;
     PARODE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_state_out<NP>, kThreads, smem));
     const long tiles = (nblocks + 15) / 16;

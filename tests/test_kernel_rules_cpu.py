@@ -54,3 +54,16 @@ def test_peer_shared_memory_is_written_between_cluster_barriers():
         assert waits and waits[0] < stores[0], f"{name}: a remote store before the cluster's first barrier"
         assert waits[-1] > stores[-1], f"{name}: no barrier after the last remote store"
     assert seen >= 2
+
+
+def test_shared_memory_limits_are_constants():
+    """The dynamic shared memory limit belongs to the function on the device, not
+    to the launch: a host thread that sets the size of its own launch lowers
+    the limit under another thread's.  Every limit is a constant."""
+    constant = re.compile(r"^(?:\(int\))?\s*(?:k[A-Z]\w*|C::smem|\d+(?: \* \d+)*)$")
+    seen = 0
+    for name, text in _sources():
+        for m in re.finditer(r"cudaFuncAttributeMaxDynamicSharedMemorySize,\s*([^;]*?)\)\);", text):
+            seen += 1
+            assert constant.match(m.group(1).strip()), f"{name}: limit {m.group(1).strip()} of one launch"
+    assert seen >= 10
