@@ -94,19 +94,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_resp_f64(const __grid_constant_
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
-    // The carry's last kernel, the one before this, lets it start after waiting
-    // for its own predecessor, so the samples are complete already: only the
-    // carried states (and y) wait for it.  The first tile's window products then
-    // run beside the carry where an SM is free (a solve of 8 states and 4096 steps:
-    // 17.8 -> 16.4 us).
-    bool waited = false;
-    auto states_ready = [&] {
-        if (!waited) {
-            grid_dep_wait();
-            grid_dep_trigger();
-            waited = true;
-        }
-    };
+    grid_dep_wait();  // the samples, the carried states
+    grid_dep_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     __shared__ int lim[kRT];  // window columns of each row tile
     if (threadIdx.x < kRT) lim[threadIdx.x] = (int)threadIdx.x < nrt ? window_limit(a, m0 + threadIdx.x * 8 + 7) : 0;
@@ -121,7 +110,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_resp_f64(const __grid_constant_
         if (tile + CT > end) return;
         auto load = [&](long at, int s, double2 (&z)[CT][kSeg / 8]) {
             const bool win = s < segs_w;
-            if (!win) states_ready();
             const int k0 = (win ? s : s - segs_w) * kSeg + 2 * t, left = (win ? a.K1 : a.K2) - k0;
             const double* base = (win ? a.U : a.X) + k0;
             const long stride = win ? a.ugs : a.xgs;
@@ -185,7 +173,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_resp_f64(const __grid_constant_
             else if (tile + 2 * CT <= end) load(tile + CT, 0, z0);
             if (s + 1 < segs) products(s + 1, z1);
         }
-        states_ready();
 #pragma unroll
         for (int rt = 0; rt < kRT; ++rt) {
             if (rt >= nrt) break;

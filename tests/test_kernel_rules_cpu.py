@@ -67,3 +67,30 @@ def test_shared_memory_limits_are_constants():
             seen += 1
             assert constant.match(m.group(1).strip()), f"{name}: limit {m.group(1).strip()} of one launch"
     assert seen >= 10
+
+
+def test_dependent_kernels_wait_before_they_read():
+    """A kernel launched as a dependent sees the results of the grids before it
+    after griddepcontrol.wait only.  Every thread waits once, at the top level
+    of the kernel or at the start of its warp's role, not in a helper called
+    where the reads happen to be."""
+    seen = 0
+    for name, body in _kernels():
+        waits = [m.start() for m in re.finditer(r"grid_dep_wait\(\)", body)]
+        if not waits:
+            continue
+        seen += 1
+        for at in waits:
+            # the enclosing blocks: none may be a lambda's
+            starts, depth = [], 0
+            for k in range(at - 1, -1, -1):
+                if body[k] == "}":
+                    depth += 1
+                elif body[k] == "{":
+                    if depth == 0:
+                        starts.append(k)
+                    else:
+                        depth -= 1
+            for k in starts[:-1]:
+                assert not re.search(r"\[[&=]?\]\s*(?:\([^()]*\)\s*)?$", body[:k]), f"{name}: waits inside a lambda"
+    assert seen >= 10
