@@ -116,14 +116,19 @@ __device__ __forceinline__ double sample_time(double base, double dt, long j)
     return __dadd_rn(base, __dmul_rn(dt, (double)j));
 }
 
-// A run of samples by Reinsch's recurrence, for nominal steps |dl| <= 1 and
-// arguments below 1e7 (else false, nothing written): S_j = amp sin(a0 + j dl)
+// A run of samples by Reinsch's recurrence, for nominal steps |dl| <= 1,
+// arguments below 1e7 and amplitudes well inside the range of floats (else
+// false, nothing written): S_j = amp sin(a0 + j dl)
 // advances as D <- D - 4 sin^2(dl / 2) S, S <- S + D, two FP64 operations a
 // term; the argument is formed rounded, as sinusoid_value rounds it, and its
-// difference e from a0 + j dl (the roundings of t_j and of the argument, below
-// 1e-8) enters to first order as amp cos(a0 + j dl) e, whose cosine comes from
-// a rotation in FP32 (its relative error of 1e-5 is 1e-13 of e's bound; the
-// neglected e^2 / 2 is below 1e-16).  7 FP64 operations a term instead of
+// difference e from a0 + j dl (the roundings of t_j and of the argument, a few
+// 1e-9 at the largest arguments) enters to first order as amp cos(a0 + j dl) e.
+// That term alone is formed in FP32, from a cosine rotated there: off by 1e-5
+// of itself at the most, 1e-13 of the amplitude at arguments of 1e7 and 1e-15
+// at 1e5; the neglected e^2 / 2 is below 1e-16.  Errors against the sine of the
+// rounded argument, runs of 64, arguments up to 2e6, of the amplitude: 1.1e-15
+// at the most for dl <= 0.1, 8e-15 for dl <= 1, where the rotation in FP64
+// below has 6.7e-15 and 8e-15.  7 FP64 operations a term instead of
 // sinusoid_run_terms' 14: the sampler is bound by the FP64 pipe.
 template <int KT, class Out>
 __device__ __forceinline__ bool sinusoid_run_reinsch(const double* a, const double* f, const double* phi, int i,
@@ -139,7 +144,9 @@ __device__ __forceinline__ bool sinusoid_run_reinsch(const double* a, const doub
         ph[q] = phi[i * KT + q];
         a0[q] = __dadd_rn(__dmul_rn(w[q], sample_time(base, dt, joff + j0)), ph[q]);
         dl[q] = __dmul_rn(w[q], dt);
-        fit = fit && fabs(dl[q]) <= 1.0 && fabs(a0[q]) < 1e7 && fabs(w[q] * tl) < 1e7;
+        const double amp = fabs(a[i * KT + q]);
+        fit = fit && fabs(dl[q]) <= 1.0 && fabs(a0[q]) < 1e7 && fabs(w[q] * tl) < 1e7 &&
+              (amp == 0.0 || (amp >= 1e-20 && amp <= 1e20));
     }
     if (!fit) return false;
     double S[KT], D[KT], kap[KT];
