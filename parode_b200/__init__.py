@@ -330,9 +330,9 @@ def affine_scan_general(M_ptr: int, V_ptr: int, x0_ptr: int, ns: int, count: int
 
 
 def tune_response_block(solver: int, n: int, m: int, p: int, T: int, precision: int = FP64):
-    """ParODE_TuneResponseBlock: times the response leaf's block lengths for
-    this class of systems on the current device and records the fastest.
-    Returns (log2 of the block length, its median ms, the untuned choice's ms)."""
+    """ParODE_TuneResponseBlock: times the block lengths of the plans that this
+    class of systems gets on the current device and records the fastest.
+    Returns (log2 of the block length, its median ms, the untuned plan's ms)."""
     r = C.c_int(0)
     best, model = C.c_float(0), C.c_float(0)
     e = C.c_int(0)

@@ -1048,27 +1048,25 @@ void ParODE_TuneResponseBlock(int solver, int nStates, int nInputs, int nOutputs
         const double h = 1e-3, tEnd = ((double)nSteps - 0.5) * h;
         long nScan = 0;
         num_outputs(solver, 0.0, tEnd, h, &nScan);
-        // the untuned choice: the blocked shape's block for scan dimensions up
-        // to 64 (single solves), else the cost model's
         const int np = (int)round_up(Ns, 8);
-        int Rdefault = 0;
-        BlockedShape sh;
-        if (Ns <= 64 && blocked_shape(Ns, nInputs, solver, &sh)) {
-            Rdefault = sh.R;
-        } else {
-            double cost = 0.0;
-            Rdefault = response_log2_block(solver, np, nStates, nInputs, nOutputs, nScan,
-                                           precision != PARODE_PRECISION_FP64 ? 0.25 : 1.0, (double)L.executions,
-                                           &cost);
-        }
-        while (Rdefault > 2 && (1L << Rdefault) / 2 >= nScan) --Rdefault;
-        auto time_R = [&](int R) -> float {
+        struct Timed {
+            float ms = 0.f;
+            int log2B = 0, leaf = -1;
+        };
+        // a plan of the class with block length 2^R (-1: the one that an untuned plan takes), timed
+        auto timed = [&](int path, int R) -> Timed {
             PlanOptions opt;
             opt.precision = precision;
-            opt.path = kPathBlockedResponse;
+            opt.path = path;
             opt.input_double = true;
             opt.force_log2_block = R;
             Plan plan(dev, s, &L.inputs, uIndex, solver, 0.0, tEnd, h, opt);
+            Timed r;
+            r.leaf = plan.tune_leaf();
+            if (r.leaf < 0) return r;
+            long long shape[4];
+            plan.response_shape(shape);
+            r.log2B = ilog2((long)shape[0]);
             cudaStream_t st = plan.stream();
             cudaEvent_t e0 = nullptr, e1 = nullptr;
             PARODE_CUDA(cudaEventCreate(&e0));
@@ -1094,36 +1092,55 @@ void ParODE_TuneResponseBlock(int solver, int nStates, int nInputs, int nOutputs
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
             std::sort(ts.begin(), ts.end());
-            return ts[ts.size() / 2];
+            r.ms = ts[ts.size() / 2];
+            return r;
         };
-        int best = -1;
-        float best_ms = 0.f, model_ms = 0.f;
-        for (int R = 2; R <= 7; ++R) {
-            const long B = 1L << R;
-            if (R > 2 && B / 2 >= nScan) break;
-            const long K = response_window(solver, (int)B, nInputs);
-            if (8.0 * ((double)B * nOutputs + np) * ((double)K + np) > 256e6) break;
-            float ms = 0.f;
-            try {
-                ms = time_R(R);
-            } catch (const Error& e) {
-                // a block length the engine cannot build for this class (a
-                // resource limit) is not a candidate; anything else is an error
-                if (e.code != kNotEnoughResources && e.code != kInvalidArgument) throw;
-                continue;
+        // The fastest block length of the plans that `path` makes, stored under
+        // their leaf: the untuned plan's own, timed before and after the others,
+        // unless another is faster by more than such times differ (2 %).
+        auto tune = [&](int path, Timed* best, Timed* untuned) {
+            *untuned = timed(path, -1);
+            if (untuned->leaf < 0) return false;
+            std::vector<Timed> others;
+            for (int R = 2; R <= 7; ++R) {
+                const long B = 1L << R;
+                if (R > 2 && B / 2 >= nScan) break;
+                const double cols = untuned->leaf == kTuneWindows ? response_window(solver, (int)B, nInputs) + np : np + 6.0 * nInputs;
+                if (8.0 * ((double)B * nOutputs + np) * cols > 256e6) break;
+                if (R == untuned->log2B) continue;
+                try {
+                    const Timed t = timed(path, R);
+                    if (t.leaf == untuned->leaf) others.push_back(t);
+                } catch (const Error& e) {
+                    // a block length the engine cannot build for this class (a
+                    // resource limit) is not a candidate; anything else is an error
+                    if (e.code != kNotEnoughResources && e.code != kInvalidArgument) throw;
+                }
             }
-            if (R == Rdefault) model_ms = ms;
-            if (best < 0 || ms < best_ms) {
-                best = R;
-                best_ms = ms;
+            untuned->ms = std::min(untuned->ms, timed(path, -1).ms);
+            *best = *untuned;
+            for (const Timed& t : others)
+                if (t.ms < 0.98f * untuned->ms && t.ms < best->ms) *best = t;
+            tune_store(tune_class(solver, Ns, nInputs, nOutputs, nScan, precision, best->leaf), best->log2B, best->ms);
+            return true;
+        };
+        // the plan that a sinusoid input of the class takes; where that has no
+        // block length to tune, the response leaf that the caller may force
+        Timed best, untuned, windows, u;
+        if (!tune(kPathAuto, &best, &untuned) && !tune(kPathBlockedResponse, &best, &untuned))
+            throw Error(kInvalidSystem, "no block length fits the class");
+        // user functions of the class are sampled even where sinusoids enter as
+        // phases: their leaf too, where it fits
+        if (best.leaf != kTuneWindows) {
+            try {
+                tune(kPathBlockedResponse, &windows, &u);
+            } catch (const Error& e) {
+                if (e.code != kNotEnoughResources && e.code != kInvalidArgument) throw;
             }
         }
-        if (best < 0) throw Error(kInvalidSystem, "no block length fits the class");
-        if (model_ms == 0.f) model_ms = time_R(Rdefault);
-        tune_store(tune_class(solver, Ns, nInputs, nOutputs, nScan, precision), best, best_ms);
-        if (log2B) log2B[0] = best;
-        if (msBest) msBest[0] = best_ms;
-        if (msModel) msModel[0] = model_ms;
+        if (log2B) log2B[0] = best.log2B;
+        if (msBest) msBest[0] = best.ms;
+        if (msModel) msModel[0] = untuned.ms;
     });
     if (nErr) nErr[0] = rc;
 }

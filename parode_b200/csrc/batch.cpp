@@ -266,9 +266,8 @@ bool BatchPlan::choose_expand(Sys& q, const PlanOptions& opt)
     const int kc = (int)round_up(np + 2 * hq, 8);
     int R = expand_log2_block(np, kc, q.p, q.nScan, opt.executions);
     if (phases) {
-        int Rt = opt.force_log2_block;
-        if (Rt < 2) Rt = tuned_log2_block(tune_class(q.solver, q.Ns, q.mu, q.p, q.nScan, opt.precision));
-        if (Rt >= 2 && Rt <= 7) {
+        int Rt = asked_log2_block(opt, q.solver, q.Ns, q.mu, q.p, q.nScan, kTuneDoublings);
+        if (Rt >= 0) {
             while (Rt > 2 && (1L << Rt) / 2 >= q.nScan) --Rt;
             R = Rt;
         }
@@ -385,9 +384,8 @@ void BatchPlan::build(std::vector<BatchSpec> specs, InputRegistry* inputs, const
             int R = response_log2_block(q.solver, np, q.n, q.mu, q.p, q.nScan, wweight, opt.executions, &cost);
             // a block length forced by the caller or measured for this class of
             // systems (tuner.h) replaces the cost model's
-            int Rt = opt.force_log2_block;
-            if (Rt < 2) Rt = tuned_log2_block(tune_class(q.solver, q.Ns, q.mu, q.p, q.nScan, opt.precision));
-            if (Rt >= 2 && Rt <= 7) {
+            int Rt = asked_log2_block(opt, q.solver, q.Ns, q.mu, q.p, q.nScan, kTuneWindows);
+            if (Rt >= 0) {
                 while (Rt > 2 && (1L << Rt) / 2 >= q.nScan) --Rt;
                 R = Rt;
             }

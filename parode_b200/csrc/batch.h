@@ -26,6 +26,7 @@
 #include "inputs.h"
 #include "kernels.h"
 #include "solver.h"
+#include "tuner.h"
 
 #include <cuda_runtime.h>
 
@@ -87,6 +88,11 @@ public:
         const Sys& q = sys_[i];
         if (q.ex) return q.mu > 0 ? kPathBlockedResponse : q.Ns <= 64 ? kPathBlocked : kPathLevel;
         return q.resp ? kPathBlockedResponse : q.blocked ? kPathBlocked : kPathLevel;
+    }
+    int tune_leaf(int i) const
+    {
+        const Sys& q = sys_[i];
+        return q.resp ? (int)kTuneWindows : q.ex && q.mu > 0 ? (int)kTuneDoublings : -1;
     }
     // Response leaf geometry of system i: block length, window columns,
     // padded scan dimension, blocks (zeros on other paths).

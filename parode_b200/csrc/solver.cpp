@@ -259,9 +259,8 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
             if (br_tc_) precision_used_ = one_pass_ ? kTF32 : kMixed;
             // a block length forced by the caller or measured for this class of
             // systems (tuner.h) replaces the default
-            int Rt = opt.force_log2_block;
-            if (Rt < 2) Rt = tuned_log2_block(tune_class(solver, Ns_, mu_, p_, nScan_, opt.precision));
-            if (Rt < 2 || Rt > 7) Rt = solver == kRK4 && shape_.NP == 64 && nScan_ < 32768 ? 3 : 4;
+            int Rt = asked_log2_block(opt, solver, Ns_, mu_, p_, nScan_, kTuneWindows);
+            if (Rt < 0) Rt = solver == kRK4 && shape_.NP == 64 && nScan_ < 32768 ? 3 : 4;
             while (Rt > 2 && (1L << Rt) / 2 >= nScan_) --Rt;
             shape_.R = Rt;
             shape_.B = 1 << Rt;
@@ -982,6 +981,19 @@ void Plan::response_shape(long long info[4]) const
     info[3] = (nScan_ + shape_.B - 1) / shape_.B;
 }
 
+int Plan::tune_leaf() const
+{
+    if (batch_) return batch_->tune_leaf(0);
+    return br_ ? (int)kTuneWindows : ex_ && mu_ > 0 ? (int)kTunePhases : -1;
+}
+
+int asked_log2_block(const PlanOptions& opt, int solver, int Ns, int mu, int p, long nScan, int leaf)
+{
+    int R = opt.force_log2_block;
+    if (R >= 0 && R < 2) R = tuned_log2_block(tune_class(solver, Ns, mu, p, nScan, opt.precision, leaf));
+    return R < 2 || R > 7 ? -1 : R;
+}
+
 bool Plan::choose_expand(const PlanOptions& opt)
 {
     // A solve without inputs in any form; with sinusoid inputs in the mixed
@@ -1001,9 +1013,8 @@ bool Plan::choose_expand(const PlanOptions& opt)
     if (!free_response && !phases) return false;
     // Long blocks cost only table rows; 64 steps leave enough blocks to fill
     // the chip from 4096 steps on.  A forced or measured length wins.
-    int R = phases ? opt.force_log2_block : 0;
-    if (R < 2 && phases) R = tuned_log2_block(tune_class(solver_, Ns_, mu_, p_, nScan_, opt.precision));
-    if (R < 2 || R > 7) R = nScan_ >= 4096 ? 6 : 4;
+    int R = phases ? asked_log2_block(opt, solver_, Ns_, mu_, p_, nScan_, kTunePhases) : -1;
+    if (R < 0) R = nScan_ >= 4096 ? 6 : 4;
     while (R > 2 && (1L << R) / 2 >= nScan_) --R;
     if (!expand_shape(Ns_, mu_, mu_ > 0 ? input_->K : 0, p_, nScan_, R, &ext_.sh)) return false;
     ex_ = true;

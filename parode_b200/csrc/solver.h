@@ -48,8 +48,8 @@ struct PlanOptions {
     // test hook (PARODE_OPT_FAULT_WITHHOLD): the mixed response kernel's
     // first CTA withholds one pipeline arrive, so its bounded waits give up
     bool fault_withhold = false;
-    // block-response leaf: log2 of the block length (0: the tuned value of
-    // the system's class, else the cost model's / the shape's default)
+    // log2 of the leaf's block length (0: the tuned value of the system's
+    // class, else the engine's own choice; -1: the engine's own choice)
     int force_log2_block = 0;
     // time partition of the solve across devices (setup_shard): this plan is
     // shard `shard` of `shards` (shards > 1)
@@ -61,6 +61,10 @@ struct PlanOptions {
     // device work, which the solve queues behind and whose synchronise ends both
     bool one_shot = false;
 };
+
+// The block length (log2) asked for by the options or measured for a system's
+// class and leaf (TuneLeaf), in [2, 7]; -1: the engine's own choice.
+int asked_log2_block(const PlanOptions& opt, int solver, int Ns, int mu, int p, long nScan, int leaf);
 
 // Batch discretisation: by its cost (small batches on the host threads,
 // large ones on the device), or forced to one side.  Both give the same bits.
@@ -112,6 +116,7 @@ public:
     // dimension, blocks (zeros when not that path)
     void response_shape(long long info[4]) const;
     int precision_used() const { return precision_used_; }
+    int tune_leaf() const;  // the leaf whose block length a tuned class sets (TuneLeaf), or -1
 
     // Time shard (PlanOptions::shards > 1; block-response path only).  The
     // plan covers the scan steps [info[0], info[0] + info[1]) of the horizon;

@@ -13,7 +13,7 @@ namespace parode {
 
 namespace {
 
-using Key = std::tuple<int, int, int, int, int, int>;
+using Key = std::tuple<int, int, int, int, int, int, int>;
 
 struct Entry {
     int log2B = -1;
@@ -27,7 +27,7 @@ std::map<Key, Entry>& table()
     return *t;
 }
 
-Key key_of(const TuneClass& c) { return Key(c.solver, c.np, c.m, c.p, c.tclass, c.precision); }
+Key key_of(const TuneClass& c) { return Key(c.solver, c.np, c.m, c.p, c.tclass, c.precision, c.leaf); }
 
 int pow2_at_least(long v)
 {
@@ -38,7 +38,7 @@ int pow2_at_least(long v)
 
 }  // namespace
 
-TuneClass tune_class(int solver, int Ns, int m, int p, long nScan, int precision)
+TuneClass tune_class(int solver, int Ns, int m, int p, long nScan, int precision, int leaf)
 {
     TuneClass c;
     c.solver = solver;
@@ -47,6 +47,7 @@ TuneClass tune_class(int solver, int Ns, int m, int p, long nScan, int precision
     c.p = pow2_at_least(std::max(1, p));
     c.tclass = ilog2(std::max(1L, nScan));
     c.precision = precision;
+    c.leaf = leaf;
     return c;
 }
 
@@ -76,7 +77,8 @@ std::string tune_dump(const std::string& gpu)
     for (const auto& kv : table()) {
         const Key& k = kv.first;
         os << gpu << ' ' << std::get<0>(k) << ' ' << std::get<1>(k) << ' ' << std::get<2>(k) << ' ' << std::get<3>(k)
-           << ' ' << std::get<4>(k) << ' ' << std::get<5>(k) << ' ' << kv.second.log2B << ' ' << kv.second.ms << '\n';
+           << ' ' << std::get<4>(k) << ' ' << std::get<5>(k) << ' ' << kv.second.log2B << ' ' << kv.second.ms << ' '
+           << std::get<6>(k) << '\n';
     }
     return os.str();
 }
@@ -94,7 +96,8 @@ int tune_load_text(const std::string& text, const std::string& gpu)
         int log2B = -1;
         float ms = 0.f;
         if (!(ls >> name >> c.solver >> c.np >> c.m >> c.p >> c.tclass >> c.precision >> log2B >> ms)) continue;
-        if (name != gpu || log2B < 2 || log2B > 7) continue;
+        if (!(ls >> c.leaf)) c.leaf = kTuneWindows;  // a file written when that was the only leaf
+        if (name != gpu || log2B < 2 || log2B > 7 || c.leaf < kTuneWindows || c.leaf > kTuneDoublings) continue;
         table()[key_of(c)] = Entry{log2B, ms};
         ++n;
     }
