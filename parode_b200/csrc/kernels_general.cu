@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(DownCfg<NP>::threads) k_scan_down(const double
 #pragma unroll
     for (int a = 0; a < kAhead; ++a) load(a, k0 + a);
     for (int e = ct; e < R::NI * 16; e += 32 * C::warps) {
-        xs[ch][0][e] = e < ns && starts ? starts[c * ss + e] : 0.0;
+        xs[ch][0][e] = e < min(ns, ss) && starts ? starts[c * ss + e] : 0.0;  // ss < ns: the caller's x0 at a padded level
         xs[ch][1][e] = 0.0;
     }
     sync();
