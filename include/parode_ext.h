@@ -270,10 +270,11 @@ void ParODE_AffineScanDevice(const double* dPhi, const double* dGamma, const dou
  * (Kernels/MMKernelScanUpsweep.cl:13-56, Kernels/MVVKernelScanUpsweep.cl:14-50,
  * MVVKernelScanDownsweep.cl:14-50), chunk by chunk.  precision:
  * PARODE_PRECISION_FP64 or PARODE_PRECISION_MIXED; the arithmetic is FP64
- * (FP64 tensor cores) in both.  dX may be dV.  Enqueued on `stream` (NULL: the
- * legacy default stream); returns once the scan is done.  Scratch (about
- * count / 15 times ns^2 + 2 ns doubles with ns rounded up to 8) comes from the
- * device's stream-ordered pool. */
+ * (FP64 tensor cores) in both.  dX may be dV or lie over any part of the inputs.
+ * Enqueued on `stream` (NULL: the legacy default stream); returns once the scan
+ * is done.  Scratch (about count / 15 times ns^2 + 2 ns doubles with ns rounded
+ * up to 8, and count ns more where dX lies over dM, or over dV at another
+ * offset) comes from the device's stream-ordered pool. */
 void ParODE_AffineScanGeneral(const double* dM, const double* dV, const double* dX0, int ns, long long count,
                               int precision, double* dX, void* stream, int nErr[]);
 

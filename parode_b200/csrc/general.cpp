@@ -9,6 +9,7 @@
 #include "kernels.h"
 
 #include <algorithm>
+#include <functional>
 #include <vector>
 
 namespace parode {
@@ -55,6 +56,13 @@ void general_scan(const double* M, const double* V, const double* x0, int ns, lo
     if (count < 1) throw Error(kInvalidArgument, "general scan: count must be >= 1");
     if (precision != kFP64 && precision != kMixed) throw Error(kInvalidArgument, "unknown precision");
     const int NP = (int)round_up(ns, 8);
+    // A chunk writes its states while others still read their maps: X over V
+    // itself is safe (a step's v is loaded before its state is stored, and by
+    // its own chunk only), X over any other part of the inputs goes by way of
+    // the scratch.  x0 is read before the first state is written.
+    const size_t states = (size_t)count * ns;
+    const auto over = [&](const double* p, size_t n) { return p && std::less<>()(p, X + states) && std::less<>()(X, p + n); };
+    const bool by_scratch = over(M, states * ns) || (X != V && over(V, states));
     // level 0: the caller's maps; level l + 1: the compositions of level l's
     // chunks (all but the last, whose composition no state needs)
     std::vector<ScanLevel> lev(1);
@@ -71,6 +79,8 @@ void general_scan(const double* M, const double* V, const double* x0, int ns, lo
         doubles += (size_t)u.count * NP * (NP + 2);
         lev.push_back(u);
     }
+    const size_t x_at = doubles;
+    if (by_scratch) doubles += states;
     double* buf = nullptr;
     if (fault_alloc_now()) throw Error(kNotEnoughResources, "general scan: device allocation failed (injected)");
     if (doubles) {
@@ -81,6 +91,7 @@ void general_scan(const double* M, const double* V, const double* x0, int ns, lo
             throw Error(kNotEnoughResources, "general scan: device allocation failed");
         }
     }
+    if (by_scratch) lev[0].X = buf + x_at;
     try {
         for (size_t l = 1; l < lev.size(); ++l) {
             ScanLevel& u = lev[l];
@@ -94,6 +105,7 @@ void general_scan(const double* M, const double* V, const double* x0, int ns, lo
             const bool top = l + 1 == lev.size();
             launch_scan_down(lev[l], NP, top ? x0 : lev[l + 1].X, top ? ns : NP, s);
         }
+        if (by_scratch) PARODE_CUDA(cudaMemcpyAsync(X, lev[0].X, sizeof(double) * states, cudaMemcpyDeviceToDevice, s));
     } catch (...) {
         if (buf) cudaFreeAsync(buf, s);
         throw;
