@@ -148,6 +148,10 @@ struct ResponseArgs {
 // Window length (columns of W) for B steps: RK4 (2B + 1) m, ABM (B + 4) m.
 int response_window(int solver, int B, int m);
 void launch_block_response(const ResponseArgs* dArgs, int nsys, int max_np, int max_p, int max_kpad, cudaStream_t s);
+// Whether a single system's W can be formed: its output rows in shared memory
+// (p NP doubles: p up to 436 at NP = 64, 3,500 at 8) and, with blocks of 16
+// steps, at most 4 GB.
+bool block_response_fits(int NP, int solver, int m, int p);
 // The same W for any NP, over many systems.  dStart[e] is entry e's first CTA
 // (response_init_ctas / response_fill_ctas CTAs each, `ctas` in total).
 // Order: init (CP_0, Q_0, BbarE); for l = 0 .. log2(B) - 1 the tiled GEMMs of

@@ -33,6 +33,9 @@ constexpr int kCols = 8;        // window columns per CTA (a cfg2 W: 41 CTAs)
 constexpr int kThreads = 256;
 constexpr size_t kSmemMax = 220 * 1024;
 
+// Shared memory of k_block_response_mma: two steps of z and the output rows.
+size_t block_response_smem(int NP, int p) { return (2 * (size_t)NP * (kCols + 4) + (size_t)p * NP) * sizeof(double); }
+
 // z (NP x kCols, row-major in shared memory): z <- Phi z + S_j, and the
 // output rows of step j, for the CTA's columns [c0, c0 + kCols).
 __global__ void __launch_bounds__(kThreads) k_block_response(const ResponseArgs* __restrict__ args)
@@ -200,7 +203,7 @@ __global__ void __launch_bounds__(kThreads) k_block_response_mma(const ResponseA
 template <int NP>
 void block_response_mma_t(const ResponseArgs* dArgs, int max_p, int max_kpad, cudaStream_t s)
 {
-    const size_t smem = (2 * (size_t)NP * (kCols + 4) + (size_t)max_p * NP) * sizeof(double);
+    const size_t smem = block_response_smem(NP, max_p);
     if (smem > kSmemMax) throw Error(kInvalidArgument, "block response: shared memory");
     PARODE_CUDA(cudaFuncSetAttribute(k_block_response_mma<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     dim3 grid((unsigned)((max_kpad + NP + kCols - 1) / kCols), 1);
@@ -468,6 +471,12 @@ int response_log2_block(int solver, int NP, int n, int m, int p, long nScan, dou
     }
     if (flops_per_step) *flops_per_step = best_cost;
     return best;
+}
+
+bool block_response_fits(int NP, int solver, int m, int p)
+{
+    const double K = response_window(solver, 16, m);
+    return block_response_smem(NP, p) <= kSmemMax && 8.0 * (16.0 * p + NP) * (K + 1.0 + NP) <= 4e9;
 }
 
 void launch_block_response(const ResponseArgs* dArgs, int nsys, int max_np, int max_p, int max_kpad, cudaStream_t s)

@@ -220,7 +220,16 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
             throw Error(kInvalidArgument, "the blocked path supports scan dimensions up to 64");
         if (opt.path != kPathLevel && can_block) path_ = kPathBlocked;
     }
-    if (path_ == kPathBlocked && choose_expand(opt)) {
+    if (path_ == kPathBlocked && !choose_expand(opt)) {
+        // sampled inputs: the response leaf where its tables fit, else the sweeps or the levels
+        br_ = mu_ > 0 && opt.path != kPathBlockedSweep &&
+              (opt.path == kPathBlockedResponse || block_response_fits(shape_.NP, solver, mu_, p_));
+        if (!br_ && !blocked_shape(Ns_, mu_, solver, &shape_)) {
+            if (opt.path != kPathAuto) throw Error(kInvalidArgument, "the blocked path: too many inputs for its tiles");
+            path_ = kPathLevel;
+        }
+    }
+    if (ex_) {
         Np_ = ext_.sh.NP;
         shape_.R = ext_.sh.R;
         shape_.B = ext_.sh.B;
@@ -252,8 +261,7 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         // The mixed form runs the aggregate and output-window products on the
         // tensor cores (3xTF32) and keeps the initial-state part of the outputs
         // in FP64; at scan dimensions up to 8 it stays in FP64, as ever.
-        if (mu_ > 0 && opt.path != kPathBlockedSweep) {
-            br_ = true;
+        if (br_) {
             br_tc_ = opt.precision != kFP64 && (shape_.NP > 8 || opt.path == kPathBlockedResponse);
             one_pass_ = br_tc_ && opt.precision == kTF32;
             if (br_tc_) precision_used_ = one_pass_ ? kTF32 : kMixed;
