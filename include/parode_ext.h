@@ -24,9 +24,10 @@ extern "C" {
 #define PARODE_PRECISION_FP64   0  /* plain: every sweep, the carry and the outputs in FP64  */
 #define PARODE_PRECISION_MIXED  1  /* leaf sweeps in 3xTF32 on tcgen05 with FP32 accumulation;
                                       Phi, the power table, the upper levels and the carry in FP64.
-                                      A plan's sinusoid inputs enter as phases advanced by the nominal
-                                      step instead of samples at the rounded times; that form's
-                                      arithmetic is FP64 throughout */
+                                      Sinusoid inputs enter as phases advanced by the nominal step
+                                      instead of samples at the rounded times, with FP64 arithmetic
+                                      throughout, as long as the two differ by less than about 1e-8
+                                      (2^-52 times 2 pi f t + phi) */
 #define PARODE_PRECISION_TF32   2  /* single pass: the block-response GEMMs in one TF32 product
                                       (operands rounded to TF32, about 2^-11 relative), the carry and
                                       the initial-state part in FP64; sinusoid inputs as under the mixed

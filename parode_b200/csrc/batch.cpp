@@ -260,16 +260,7 @@ bool BatchPlan::choose_expand(Sys& q, const PlanOptions& opt)
     if (opt.path != kPathAuto && opt.path != kPathBlocked) return false;
     const bool phases = q.mu > 0 && opt.precision == kMixed && q.input->kind == InputEntry::kSinusoid;
     if (q.mu > 0 && !phases) return false;
-    // Within a block the phases advance by the nominal step: against samples at
-    // the rounded times they are off by the roundings of t and of w t + phi, about
-    // 2^-52 of that.
-    // Late or fast enough for that to show beside the form's 1e-7 (RK4 n = 24 at
-    // t = 1e9: 3e-6 against 1.5e-7 with samples) the inputs are sampled.
-    if (phases) {
-        const double t = std::max(std::fabs(q.t0), std::fabs(q.tEnd));
-        for (long k = 0; k < (long)q.mu * q.input->K; ++k)
-            if (!(6.3 * std::fabs(q.input->f[k]) * t + std::fabs(q.input->phi[k]) < 1e-8 * 4503599627370496.0)) return false;
-    }
+    if (phases && sinusoid_late(q.input, q.mu, q.t0, q.tEnd)) return false;
     const int np = (int)round_up(q.Ns, 8);
     const long hq = phases ? (long)q.mu * q.input->K : 0;
     if (np > 1024 || hq > kExpandMaxPairs) return false;

@@ -7,6 +7,7 @@
 
 #include <nvrtc.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -98,6 +99,14 @@ int InputRegistry::add_user(const std::string& source)
     return (int)entries_.size() - 1;
 }
 
+bool sinusoid_late(const InputEntry* e, int m, double t0, double tEnd)
+{
+    const double t = std::max(std::fabs(t0), std::fabs(tEnd));
+    for (long q = 0; q < (long)m * e->K; ++q)
+        if (!(6.3 * std::fabs(e->f[q]) * t + std::fabs(e->phi[q]) < 1e-8 * 4503599627370496.0)) return true;
+    return false;
+}
+
 double sinusoid_host(const InputEntry* e, int i, double t)
 {
     const double two_pi = 6.283185307179586476925286766559;
@@ -172,7 +181,7 @@ void InputRegistry::fill_planes(InputEntry* e, int device, float* hi, float* lo,
                                 double dt, long count, bool double_type, cudaStream_t s, long joff)
 {
     if (m <= 0 || count <= 0) return;
-    if (e->kind == InputEntry::kSinusoid) {
+    if (e->kind == InputEntry::kSinusoid && !scratch) {
         if (e->m < m) throw Error(kInvalidInput, "sinusoid input has fewer channels than the system");
         const long q = (long)e->m * e->K;
         const double* d = sinusoid_device(e, device);

@@ -28,6 +28,13 @@ struct InputEntry {
     std::vector<double*> dparams;  // per device: a | f | phi, 3*m*K doubles
 };
 
+// Whether a sinusoid input's samples at the rounded times differ from phases
+// advanced by the nominal step by more than 1e-8: the roundings of t and of
+// w t + phi, about 2^-52 of that.  The mixed forms then sample in FP64 at the
+// rounded times (RK4 n = 24 at t = 1e9: 3e-6 off by nominal steps, 1.5e-7 of
+// the form's own with samples).
+bool sinusoid_late(const InputEntry* e, int m, double t0, double tEnd);
+
 // u_i(t) of a sinusoid input, on the host.
 double sinusoid_host(const InputEntry* e, int i, double t);
 
@@ -49,8 +56,9 @@ public:
     void fill(InputEntry* e, int device, double* U, int m, double base, double dt, long count, bool double_type,
               cudaStream_t s, long joff = 0);
     // The same samples as TF32 hi / lo planes (hi[j*m + i], lo[j*m + i]; lo
-    // may be null): the sinusoid input writes them directly; a user function
-    // fills `scratch` (count*m doubles) first.
+    // may be null): a sinusoid input without `scratch` writes them directly; a
+    // user function, or a sinusoid with it, fills `scratch` (count*m doubles)
+    // first.
     void fill_planes(InputEntry* e, int device, float* hi, float* lo, double* scratch, int m, double base,
                      double dt, long count, bool double_type, cudaStream_t s, long joff = 0);
     // Device copy of a sinusoid input's parameters: a | f | phi, m*K each.

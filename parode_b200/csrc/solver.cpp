@@ -164,6 +164,8 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
     if (mu_ > 0) {
         input_ = inputs ? inputs->get(uIndex) : nullptr;
         if (!input_) throw Error(kInvalidInput, "uIndex does not name a registered input");
+        late_ = opt.precision != kFP64 && input_->kind == InputEntry::kSinusoid && input_->m >= mu_ &&
+                sinusoid_late(input_, mu_, t0, tEnd);
     }
     Ns_ = solver == kRK4 ? sys.n : 4 * sys.n;
     Np_ = (int)round_up(Ns_, 8);
@@ -440,13 +442,13 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
     const long pad = (sampled && br_) ? (2L * shape_.B + 8) * mu_ + 2 : 0;
     // the mixed response GEMMs read the samples as TF32 planes (their TMA
     // boxes run up to 15 samples past a window); FP64 samples are then only
-    // the scratch a user input function fills before the split
+    // the scratch a user input function, or a late sinusoid, fills before the split
     const bool planes = sampled && br_tc_;
     const long nf = nU_ * (long)mu_ + pad + 16;
     double* dh = nullptr;
     double* dl = nullptr;
     if (sampled) {
-        if (!planes || input_->kind != InputEntry::kSinusoid) want.emplace_back(&dU_, nU_ * (long)mu_ + pad);
+        if (!planes || input_->kind != InputEntry::kSinusoid || late_) want.emplace_back(&dU_, nU_ * (long)mu_ + pad);
         if (planes) {
             want.emplace_back(&dh, (nf + 1) / 2);
             if (!one_pass_) want.emplace_back(&dl, (nf + 1) / 2);  // the single-pass form reads no lo plane
@@ -1006,8 +1008,8 @@ bool Plan::choose_expand(const PlanOptions& opt)
 {
     // A solve without inputs in any form; with sinusoid inputs in the mixed
     // and TF32 forms at the scan dimensions those forms cover (their sample
-    // planes took the nominal phase steps that the expansion takes; the FP64
-    // form samples at the rounded times and keeps its samples).  User input
+    // planes take nominal phase steps too; the FP64 form samples at the rounded
+    // times and keeps its samples, as late sinusoids do).  User input
     // functions, time shards and the fault hook of the tensor-core kernel
     // take the sample windows.  An input with too few channels is refused
     // where the samples are filled, as before.
@@ -1017,7 +1019,7 @@ bool Plan::choose_expand(const PlanOptions& opt)
         return false;
     const bool free_response = mu_ == 0;
     const bool phases = mu_ > 0 && opt.precision != kFP64 && Ns_ > 8 && input_->kind == InputEntry::kSinusoid &&
-                        input_->m >= mu_;
+                        input_->m >= mu_ && !late_;
     if (!free_response && !phases) return false;
     // Long blocks cost only table rows; 64 steps leave enough blocks to fill
     // the chip from 4096 steps on.  A forced or measured length wins.

@@ -188,6 +188,7 @@ private:
     // block states by radix expansion (kernels_expand.cu): no inputs, or
     // sinusoid inputs in the mixed and TF32 forms
     bool ex_ = false;
+    bool late_ = false;  // sinusoids that the mixed forms sample in FP64 (sinusoid_late)
     ExpandTables ext_;
     double* dZ_ = nullptr;      // augmented block states, nblocks x Kc
     double* dMs_ = nullptr;     // general path: T copies of Phi (Ns x Ns each)
