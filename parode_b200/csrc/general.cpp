@@ -48,7 +48,7 @@ size_t general_scan_bytes(int ns, long count)
     return sizeof(double) * (size_t)(Tp * NP * NP + (Tp + 1) * NP);
 }
 
-void general_scan(const double* M, const double* V, const double* x0, int ns, long count, int precision,
+int general_scan(const double* M, const double* V, const double* x0, int ns, long count, int precision,
                   double* X, cudaStream_t s)
 {
     if (!M || !X) throw Error(kInvalidArgument, "general scan: M and X must be device pointers");
@@ -56,6 +56,7 @@ void general_scan(const double* M, const double* V, const double* x0, int ns, lo
     if (count < 1) throw Error(kInvalidArgument, "general scan: count must be >= 1");
     if (precision != kFP64 && precision != kMixed) throw Error(kInvalidArgument, "unknown precision");
     const int NP = (int)round_up(ns, 8);
+    int launches = 0;
     // A chunk writes its states while others still read their maps: X over V
     // itself is safe (a step's v is loaded before its state is stored, and by
     // its own chunk only), X over any other part of the inputs goes by way of
@@ -100,10 +101,12 @@ void general_scan(const double* M, const double* V, const double* x0, int ns, lo
             u.V = m + (size_t)u.count * NP * NP;
             u.X = m + (size_t)u.count * NP * (NP + 1);
             launch_scan_up(lev[l - 1], NP, u.count - 1, m, m + (size_t)u.count * NP * NP, s);
+            ++launches;  // a level above another has at least two maps
         }
         for (size_t l = lev.size(); l-- > 0;) {
             const bool top = l + 1 == lev.size();
             launch_scan_down(lev[l], NP, top ? x0 : lev[l + 1].X, top ? ns : NP, s);
+            ++launches;
         }
         if (by_scratch) PARODE_CUDA(cudaMemcpyAsync(X, lev[0].X, sizeof(double) * states, cudaMemcpyDeviceToDevice, s));
     } catch (...) {
@@ -111,6 +114,7 @@ void general_scan(const double* M, const double* V, const double* x0, int ns, lo
         throw;
     }
     if (buf) PARODE_CUDA(cudaFreeAsync(buf, s));
+    return launches;
 }
 
 }  // namespace parode

@@ -34,8 +34,9 @@ void launch_scan_down(const ScanLevel& l, int NP, const double* starts, int ss, 
 // The whole scan on device data: x_0 = x0 (nullptr: 0), x_{k+1} = M_k x_k +
 // V_k (V nullptr: 0), X[k] = x_k for k < count; M count x ns x ns, V and X
 // count x ns (X over any part of the inputs), row-major FP64.  FP64 in either precision form.
-// Scratch from the stream-ordered pool; returns after enqueueing.
-void general_scan(const double* M, const double* V, const double* x0, int ns, long count, int precision,
+// Scratch from the stream-ordered pool; returns after enqueueing, with the
+// number of kernels launched.
+int general_scan(const double* M, const double* V, const double* x0, int ns, long count, int precision,
                   double* X, cudaStream_t s);
 
 }  // namespace parode

@@ -901,12 +901,15 @@ std::vector<std::pair<std::string, float>> Plan::stage_times()
     return out;
 }
 
-void Plan::fill_inputs(cudaStream_t s)
+int Plan::fill_inputs(cudaStream_t s)
 {
-    if (mu_ <= 0) return;
-    if (dUh_)
+    if (mu_ <= 0) return 0;
+    if (dUh_) {
         inputs_->fill_planes(input_, device_, dUh_, dUl_, dU_, mu_, u_base_, u_dt_, nU_, opt_.input_double, s, u_joff_);
-    else inputs_->fill(input_, device_, dU_, mu_, u_base_, u_dt_, nU_, opt_.input_double, s, u_joff_);
+        return dU_ ? 2 : 1;  // FP64 samples are split into the planes by a second kernel
+    }
+    inputs_->fill(input_, device_, dU_, mu_, u_base_, u_dt_, nU_, opt_.input_double, s, u_joff_);
+    return 1;
 }
 
 void Plan::execute(double* y, cudaStream_t s)
@@ -1058,8 +1061,7 @@ void Plan::execute_body(double* y, cudaStream_t s)
     marks_.clear();
     mark("start", s);
 
-    fill_inputs(s);
-    launches += mu_ > 0 ? 1 : 0;
+    launches += fill_inputs(s);
     mark("inputs", s);
     // V slots: dV_ = slot -1 (the initial state), V1 = slots 0 .. Tp-1
     double* V1 = dV_ + Np;
@@ -1154,16 +1156,14 @@ void Plan::execute_general(double* Y, cudaStream_t s)
     int launches = 0;
     marks_.clear();
     mark("start", s);
-    fill_inputs(s);
-    launches += mu_ > 0 ? 1 : 0;
+    launches += fill_inputs(s);
     mark("inputs", s);
     double* V1 = dV_ + Np_;
     launch_forcing(V1, Np_, sys_.n, sys_.zeroB ? 0 : sys_.m, solver_, dBbar_, dU_, nScan_, Tp_, s);
     launch_distribute(dMs_, dPow_, Np_, nScan_, sms_, s);
     launches += 2;
     mark("maps", s);
-    general_scan(dMs_, V1, dX0_, Np_, nScan_, precision_used_, dXs_, s);
-    launches += 2 * ilog2(Tp_) + 2;
+    launches += general_scan(dMs_, V1, dX0_, Np_, nScan_, precision_used_, dXs_, s);
     mark("scan", s);
     if (solver_ == kRK4) {
         launch_output(Y, dXs_, Np_, 0, sys_.n, mu_, p_, dC_, dD_, sys_.zeroC, sys_.zeroD, dU_, 2, 0, nScan_, 0, s);
@@ -1271,8 +1271,7 @@ int Plan::response_head(cudaStream_t s)
         mark("states", s);
         return launches;
     }
-    fill_inputs(s);
-    ++launches;
+    launches += fill_inputs(s);
     mark("inputs", s);
     if (br_tc_) {
         // mixed: aggregates and output windows on the tensor cores
@@ -1511,8 +1510,7 @@ void Plan::execute_blocked(double* Y, cudaStream_t s)
     PARODE_CUDA(cudaEventRecord(fork_[0], s));
     PARODE_CUDA(cudaStreamWaitEvent(side_, fork_[0], 0));
     if (mu_ > 0 && !gen_) {
-        fill_inputs(side_);
-        ++launches;
+        launches += fill_inputs(side_);
     }
     PARODE_CUDA(cudaEventRecord(fork_[1], side_));
     launch_blocked_tables(shape_, dPow_, 1, shape_.R, dCP_, dCext_, p_, s);

@@ -155,7 +155,7 @@ private:
     void state_part(double* Y, long c0, long c1, cudaStream_t s);
     void check_status();  // after a synchronise: throws when a device-side wait gave up
     void setup_shard(const PlanOptions& opt);
-    void fill_inputs(cudaStream_t s);
+    int fill_inputs(cudaStream_t s);  // returns the launches
 
     int device_ = 0;
     cudaStream_t stream_ = nullptr;
