@@ -79,13 +79,18 @@ __device__ __forceinline__ double sinusoid_value(const double* a, const double* 
     return v;
 }
 
-// Where a sampler puts sample j of its run: FP64 at out[j * stride], or
+// Where a sampler puts sample j of its run: FP64 at out[(j - skip) * stride], or
 // split into two TF32 planes (hi = TF32(x), lo = TF32(x - hi) with
-// x = float(v), both rounded to nearest) for the tensor-core GEMMs.
+// x = float(v), both rounded to nearest) for the tensor-core GEMMs.  The
+// first `skip` samples of a run lie before the buffer.
 struct SampleOut64 {
     double* out;
     long stride;
-    __device__ __forceinline__ void operator()(long j, double v) const { out[j * stride] = v; }
+    int skip = 0;
+    __device__ __forceinline__ void operator()(long j, double v) const
+    {
+        if (j >= skip) out[(j - skip) * stride] = v;
+    }
 };
 
 // x rounded to TF32 (10 mantissa bits), to nearest with ties away from zero:
@@ -101,10 +106,13 @@ struct SampleOutSplit {
     float* hi;
     float* lo;
     long stride;
+    int skip = 0;
     __device__ __forceinline__ void operator()(long j, double v) const
     {
         const float x = (float)v;
         const float h = tf32_rna(x);
+        if (j < skip) return;
+        j -= skip;
         hi[j * stride] = h;
         if (lo) lo[j * stride] = tf32_rna(x - h);  // no lo plane in the single-pass form
     }

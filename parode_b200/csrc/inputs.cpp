@@ -156,7 +156,7 @@ InputEntry* InputRegistry::get(int idx)
 }
 
 void InputRegistry::fill(InputEntry* e, int device, double* U, int m, double base, double dt, long count,
-                         bool double_type, cudaStream_t s, long joff)
+                         bool double_type, cudaStream_t s, long joff, long horizon)
 {
     if (m <= 0 || count <= 0) return;
     if (e->kind == InputEntry::kSinusoid) {
@@ -165,7 +165,7 @@ void InputRegistry::fill(InputEntry* e, int device, double* U, int m, double bas
         const double* d = sinusoid_device(e, device);
         // the kernel indexes parameters as i*K + k for i < m, so a sinusoid
         // input wider than the system is read from its first m channels
-        launch_sinusoid_samples(U, m, e->K, d, d + q, d + 2 * q, base, dt, count, s, joff);
+        launch_sinusoid_samples(U, m, e->K, d, d + q, d + 2 * q, base, dt, count, s, joff, horizon);
         return;
     }
     int v = double_type ? 1 : 0;
@@ -178,18 +178,18 @@ void InputRegistry::fill(InputEntry* e, int device, double* U, int m, double bas
 }
 
 void InputRegistry::fill_planes(InputEntry* e, int device, float* hi, float* lo, double* scratch, int m, double base,
-                                double dt, long count, bool double_type, cudaStream_t s, long joff)
+                                double dt, long count, bool double_type, cudaStream_t s, long joff, long horizon)
 {
     if (m <= 0 || count <= 0) return;
     if (e->kind == InputEntry::kSinusoid && !scratch) {
         if (e->m < m) throw Error(kInvalidInput, "sinusoid input has fewer channels than the system");
         const long q = (long)e->m * e->K;
         const double* d = sinusoid_device(e, device);
-        launch_sinusoid_planes(hi, lo, m, e->K, d, d + q, d + 2 * q, base, dt, count, s, joff);
+        launch_sinusoid_planes(hi, lo, m, e->K, d, d + q, d + 2 * q, base, dt, count, s, joff, horizon);
         return;
     }
     if (!scratch) throw Error(kInvalidArgument, "a user input function needs FP64 scratch for its samples");
-    fill(e, device, scratch, m, base, dt, count, double_type, s, joff);
+    fill(e, device, scratch, m, base, dt, count, double_type, s, joff, horizon);
     launch_split_planes(scratch, hi, lo, count * m, s);
 }
 

@@ -213,14 +213,16 @@ inline long sweep_columns(long nScan, long Tp, long d)
     return used < all ? used : all;
 }
 
-// U[j*m + i] = sum_k a sin(2 pi f t_j + phi), t_j = base + dt*j, j < count.
+// U[j*m + i] = sum_k a sin(2 pi f t_{joff + j} + phi), t_j = base + dt*j, j < count;
+// horizon: samples of the whole horizon where the buffer is a part of it (a
+// time shard takes the whole solve's run length).
 void launch_sinusoid_samples(double* U, int m, int K, const double* a, const double* f, const double* phi,
-                             double base, double dt, long count, cudaStream_t s, long joff = 0);
+                             double base, double dt, long count, cudaStream_t s, long joff = 0, long horizon = 0);
 
 // The same samples written as TF32 hi / lo planes (hi = TF32(x),
 // lo = TF32(x - hi), x = float(u)), the tensor-core GEMMs' operand form.
 void launch_sinusoid_planes(float* hi, float* lo, int m, int K, const double* a, const double* f, const double* phi,
-                            double base, double dt, long count, cudaStream_t s, long joff = 0);
+                            double base, double dt, long count, cudaStream_t s, long joff = 0, long horizon = 0);
 // FP64 samples into those planes (n values).  lo may be null in both (hi only).
 void launch_split_planes(const double* U, float* hi, float* lo, long n, cudaStream_t s);
 // dst[i] = (float)src[i], i < n

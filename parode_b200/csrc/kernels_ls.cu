@@ -444,18 +444,36 @@ __global__ void k_swap_grouped(const LevelArgs* __restrict__ args)
     swap_body(a);
 }
 
+// Run r of a buffer of `count` samples whose first has index joff on the whole
+// horizon.  Runs start at multiples of their length on the horizon, so a time
+// shard's samples are those of the whole solve bit for bit; its first run may
+// start before its buffer.
+struct SampleRun {
+    long j0;   // first sample, relative to the buffer
+    int skip;  // of the run's first samples that lie before the buffer
+    int n;     // samples, 0 past the last run
+};
+__host__ __device__ inline long sample_runs(long count, long joff, int run) { return (joff % run + count + run - 1) / run; }
+__device__ __forceinline__ SampleRun sample_run_of(long r, long count, long joff, int run)
+{
+    SampleRun s;
+    s.j0 = r * run - joff % run;
+    s.skip = s.j0 < 0 ? (int)-s.j0 : 0;
+    s.n = (int)max(0L, min((long)run, count - s.j0));
+    return s;
+}
+
 // One thread per (run of `run` samples, channel); channels fastest.
 template <int KMAX>
 __global__ void k_sinusoid_samples(double* U, int m, int K, const double* a, const double* f, const double* phi,
                                    double base, double dt, long count, long joff, int run)
 {
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long runs = (count + run - 1) / run;
-    if (e >= runs * m) return;
-    const long r = e / m;
-    const int i = (int)(e - r * m);
-    const long j0 = r * run;
-    sinusoid_run<KMAX>(a, f, phi, K, i, base, dt, j0, (int)min((long)run, count - j0), SampleOut64{U + j0 * m + i, m}, joff);
+    const SampleRun s = sample_run_of(e / m, count, joff, run);
+    if (s.n <= 0) return;
+    const int i = (int)(e % m);
+    const long at = (s.j0 + s.skip) * m + i;  // of the run's first sample in the buffer
+    sinusoid_run<KMAX>(a, f, phi, K, i, base, dt, s.j0, s.n, SampleOut64{U + at, m, s.skip}, joff);
 }
 
 // The same samples as TF32 hi / lo planes (the tensor-core GEMMs' operands),
@@ -466,13 +484,11 @@ __global__ void k_sinusoid_planes(float* hi, float* lo, int m, int K, const doub
 {
     grid_dep_trigger();  // the response GEMMs may set up meanwhile (they wait for these samples)
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long runs = (count + run - 1) / run;
-    if (e >= runs * m) return;
-    const long r = e / m;
-    const int i = (int)(e - r * m);
-    const long j0 = r * run;
-    sinusoid_rot<KMAX>(a, f, phi, K, i, base, dt, j0, (int)min((long)run, count - j0),
-                                   SampleOutSplit{hi + j0 * m + i, lo ? lo + j0 * m + i : nullptr, m}, joff);
+    const SampleRun s = sample_run_of(e / m, count, joff, run);
+    if (s.n <= 0) return;
+    const int i = (int)(e % m);
+    const long at = (s.j0 + s.skip) * m + i;  // of the run's first sample in the buffer
+    sinusoid_rot<KMAX>(a, f, phi, K, i, base, dt, s.j0, s.n, SampleOutSplit{hi + at, lo ? lo + at : nullptr, m, s.skip}, joff);
 }
 
 // FP64 samples (any input function) into TF32 hi / lo planes.
@@ -742,11 +758,11 @@ void launch_affine_level(const LevelArgs& a, cudaStream_t s)
 }
 
 void launch_sinusoid_samples(double* U, int m, int K, const double* a, const double* f, const double* phi,
-                             double base, double dt, long count, cudaStream_t s, long joff)
+                             double base, double dt, long count, cudaStream_t s, long joff, long horizon)
 {
     if (count <= 0 || m <= 0) return;
-    const int run = sample_run(count * m);
-    const long total = (count + run - 1) / run * m;
+    const int run = sample_run(std::max(count, horizon) * m);
+    const long total = sample_runs(count, joff, run) * m;
     const unsigned g = (unsigned)blocks_for(total, 256);
     switch (sample_kmax(K)) {
     case 1: k_sinusoid_samples<1><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff, run); break;
@@ -758,11 +774,11 @@ void launch_sinusoid_samples(double* U, int m, int K, const double* a, const dou
 }
 
 void launch_sinusoid_planes(float* hi, float* lo, int m, int K, const double* a, const double* f, const double* phi,
-                            double base, double dt, long count, cudaStream_t s, long joff)
+                            double base, double dt, long count, cudaStream_t s, long joff, long horizon)
 {
     if (count <= 0 || m <= 0) return;
-    const int run = sample_run(count * m);
-    const long total = (count + run - 1) / run * m;
+    const int run = sample_run(std::max(count, horizon) * m);
+    const long total = sample_runs(count, joff, run) * m;
     const unsigned g = (unsigned)blocks_for(total, 256);
     switch (sample_kmax(K)) {
     case 1: k_sinusoid_planes<1><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff, run); break;

@@ -904,11 +904,12 @@ std::vector<std::pair<std::string, float>> Plan::stage_times()
 int Plan::fill_inputs(cudaStream_t s)
 {
     if (mu_ <= 0) return 0;
+    const long horizon = shards_ > 1 ? (solver_ == kRK4 ? 2 * nScanGlobal_ + 1 : nScanGlobal_ + 4) : nU_;
     if (dUh_) {
-        inputs_->fill_planes(input_, device_, dUh_, dUl_, dU_, mu_, u_base_, u_dt_, nU_, opt_.input_double, s, u_joff_);
+        inputs_->fill_planes(input_, device_, dUh_, dUl_, dU_, mu_, u_base_, u_dt_, nU_, opt_.input_double, s, u_joff_, horizon);
         return dU_ ? 2 : 1;  // FP64 samples are split into the planes by a second kernel
     }
-    inputs_->fill(input_, device_, dU_, mu_, u_base_, u_dt_, nU_, opt_.input_double, s, u_joff_);
+    inputs_->fill(input_, device_, dU_, mu_, u_base_, u_dt_, nU_, opt_.input_double, s, u_joff_, horizon);
     return 1;
 }
 
