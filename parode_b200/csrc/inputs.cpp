@@ -20,14 +20,16 @@ namespace {
 // formed in FP64 before the conversion to fType.
 const char* kUKernelTail = R"(
 extern "C" __global__ void parode_u_samples(double* U, int m, double base, double dt, long long count,
-                                            long long joff)
+                                            long long joff, long long* bad)
 {
     long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= count * (long long)m) return;
     long long j = e / m;
     int i = (int)(e - j * m);
     double t = __dadd_rn(base, __dmul_rn(dt, (double)(joff + j)));
-    U[e] = (double)UFunc((fType)t, i);
+    double v = (double)UFunc((fType)t, i);
+    U[e] = v;
+    if (bad && !(v - v == 0.0)) atomicMin(bad, j);
 }
 )";
 
@@ -156,7 +158,7 @@ InputEntry* InputRegistry::get(int idx)
 }
 
 void InputRegistry::fill(InputEntry* e, int device, double* U, int m, double base, double dt, long count,
-                         bool double_type, cudaStream_t s, long joff, long horizon)
+                         bool double_type, cudaStream_t s, long joff, long horizon, long long* bad)
 {
     if (m <= 0 || count <= 0) return;
     if (e->kind == InputEntry::kSinusoid) {
@@ -171,14 +173,15 @@ void InputRegistry::fill(InputEntry* e, int device, double* U, int m, double bas
     int v = double_type ? 1 : 0;
     if (!e->kern[v]) compile(e, v);
     long long cnt = count, off = joff;
-    void* args[] = {&U, &m, &base, &dt, &cnt, &off};
+    void* args[] = {&U, &m, &base, &dt, &cnt, &off, &bad};
     long total = count * m;
     unsigned grid = (unsigned)((total + 255) / 256);
     PARODE_CUDA(cudaLaunchKernel((const void*)e->kern[v], dim3(grid), dim3(256), args, 0, s));
 }
 
 void InputRegistry::fill_planes(InputEntry* e, int device, float* hi, float* lo, double* scratch, int m, double base,
-                                double dt, long count, bool double_type, cudaStream_t s, long joff, long horizon)
+                                double dt, long count, bool double_type, cudaStream_t s, long joff, long horizon,
+                                long long* bad)
 {
     if (m <= 0 || count <= 0) return;
     if (e->kind == InputEntry::kSinusoid && !scratch) {
@@ -189,7 +192,7 @@ void InputRegistry::fill_planes(InputEntry* e, int device, float* hi, float* lo,
         return;
     }
     if (!scratch) throw Error(kInvalidArgument, "a user input function needs FP64 scratch for its samples");
-    fill(e, device, scratch, m, base, dt, count, double_type, s, joff, horizon);
+    fill(e, device, scratch, m, base, dt, count, double_type, s, joff, horizon, bad);
     launch_split_planes(scratch, hi, lo, count * m, s);
 }
 

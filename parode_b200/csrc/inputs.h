@@ -52,15 +52,17 @@ public:
     // U[j*m + i] = u_i(base + dt*(joff + j)) for j < count, i < m, enqueued
     // on `s` (joff, horizon: the first sample's index on the whole horizon and its
     // samples, for a time shard).  `double_type` selects the fType = double variant of a user
-    // function.
+    // function.  bad (may be null): lowered to the first sample of a user
+    // function that is not finite.
     void fill(InputEntry* e, int device, double* U, int m, double base, double dt, long count, bool double_type,
-              cudaStream_t s, long joff = 0, long horizon = 0);
+              cudaStream_t s, long joff = 0, long horizon = 0, long long* bad = nullptr);
     // The same samples as TF32 hi / lo planes (hi[j*m + i], lo[j*m + i]; lo
     // may be null): a sinusoid input without `scratch` writes them directly; a
     // user function, or a sinusoid with it, fills `scratch` (count*m doubles)
     // first.
     void fill_planes(InputEntry* e, int device, float* hi, float* lo, double* scratch, int m, double base,
-                     double dt, long count, bool double_type, cudaStream_t s, long joff = 0, long horizon = 0);
+                     double dt, long count, bool double_type, cudaStream_t s, long joff = 0, long horizon = 0,
+                     long long* bad = nullptr);
     // Device copy of a sinusoid input's parameters: a | f | phi, m*K each.
     const double* sinusoid_device(InputEntry* e, int device);
 

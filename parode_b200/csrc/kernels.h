@@ -148,6 +148,17 @@ struct ResponseArgs {
 // Window length (columns of W) for B steps: RK4 (2B + 1) m, ABM (B + 4) m.
 int response_window(int solver, int B, int m);
 void launch_block_response(const ResponseArgs* dArgs, int nsys, int max_np, int max_p, int max_kpad, cudaStream_t s);
+// Outputs that the leaf's products spoil where a user function's sample is not
+// finite (kernels_br.cu, k_before_bad_sample).
+struct BadSampleArgs {
+    const long long* bad = nullptr;  // first such sample
+    long samples = 0, steps = 0;     // samples in U; scan steps
+    int solver = 0, NP = 0, n = 0, m = 0, p = 0, B = 0, cols = 0, zeroB = 0, zeroD = 0;  // cols: a window's
+    const double *U = nullptr, *X = nullptr, *Phi = nullptr, *Bbar = nullptr, *Cext = nullptr, *D = nullptr;
+    double* Y = nullptr;             // output 0 of the scan
+    long c0 = 0, c1 = 0;             // blocks whose outputs are written
+};
+void launch_before_bad_sample(const BadSampleArgs& a, cudaStream_t s);
 // Whether a single system's W can be formed: its output rows in shared memory
 // (p NP doubles: p up to 436 at NP = 64, 3,500 at 8) and, with blocks of 16
 // steps, at most 4 GB.

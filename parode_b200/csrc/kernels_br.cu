@@ -263,6 +263,52 @@ __global__ void __launch_bounds__(kThreads) k_response_init(const ResponseArgs* 
     }
 }
 
+// The outputs before the first sample that is not finite (*bad; none: past the
+// last), one CTA, FP64.  A block's products read its whole window, and some
+// samples past it against zeros of W, so a NaN or an infinity among them spoils
+// outputs and states of earlier steps, which no recurrence would.  The steps
+// from the last block whose entering state is formed without that sample to
+// the first that reads it are taken one by one.  Nothing to do as a rule: the
+// launch then costs what an empty one does.
+__global__ void __launch_bounds__(kThreads) k_before_bad_sample(const BadSampleArgs a)
+{
+    __shared__ double xs[2][64];
+    grid_dep_wait();
+    const long long bad = *a.bad;
+    if (bad >= a.samples) return;
+    const bool rk4 = a.solver == 0;
+    const int NP = a.NP, n = a.n, m = a.m, W = rk4 ? 3 : 5, coff = rk4 ? 0 : 3 * n;
+    // output k reads samples up to 2 k (RK4), k + 3 (ABM), and so does its state
+    const long first = min(a.steps, rk4 ? (long)(bad + 1) / 2 : max(0L, (long)bad - 3));
+    const long per = (rk4 ? 2L : 1L) * a.B;  // samples per block
+    long b = first / a.B;
+    while (b > 0 && ((b - 1) * per) * m + a.cols + 64 > bad * m) --b;
+    for (int r = threadIdx.x; r < NP; r += kThreads) xs[0][r] = a.X[b * NP + r];
+    __syncthreads();
+    int cur = 0;
+    for (long k = b * a.B; k < first; ++k, cur ^= 1) {
+        const double* x = xs[cur];
+        const double* u = a.U + (rk4 ? 2 * k : k) * m;  // the step's window
+        if (k >= a.c0 * a.B && k < a.c1 * a.B)
+            for (int o = threadIdx.x; o < a.p; o += kThreads) {
+                double v = 0.0;
+                for (int c = 0; c < NP; ++c) v = fma(a.Cext[(long)o * NP + c], x[c], v);
+                if (!a.zeroD)
+                    for (int c = 0; c < m; ++c) v = fma(a.D[(long)o * m + c], u[(rk4 ? 0 : 3L * m) + c], v);
+                a.Y[k * a.p + o] = v;
+            }
+        if (k + 1 < first)
+            for (int r = threadIdx.x; r < NP; r += kThreads) {
+                double v = 0.0;
+                for (int c = 0; c < NP; ++c) v = fma(a.Phi[(long)r * NP + c], x[c], v);
+                if (!a.zeroB && r >= coff && r < coff + n)
+                    for (int c = 0; c < W * m; ++c) v = fma(a.Bbar[(long)(r - coff) * W * m + c], u[c], v);
+                xs[cur ^ 1][r] = v;
+            }
+        __syncthreads();
+    }
+}
+
 // Every element of W from the tables: sums over the steps i whose forcing
 // reads the element's sample (slot w = s - 2i for RK4, s - i for ABM).
 __global__ void __launch_bounds__(kThreads) k_response_fill(const ResponseArgs* __restrict__ args,
@@ -471,6 +517,11 @@ int response_log2_block(int solver, int NP, int n, int m, int p, long nScan, dou
     }
     if (flops_per_step) *flops_per_step = best_cost;
     return best;
+}
+
+void launch_before_bad_sample(const BadSampleArgs& a, cudaStream_t s)
+{
+    launch_dependent(k_before_bad_sample, dim3(1), dim3(kThreads), 0, s, a);
 }
 
 bool block_response_fits(int NP, int solver, int m, int p)

@@ -11,6 +11,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <mutex>
 #include <string>
 
@@ -369,6 +370,11 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
     if (solver == kABM) want.emplace_back(&dYpre_, 3L * p_);
     if (blocked) want.emplace_back(&dCext_, (long)p_ * Np_);
     if (br_) want.emplace_back(&dra, words(sizeof(ResponseArgs)));
+    // the first sample of a user function that is not finite (the function's
+    // values, and so this, are the same in every execute)
+    const bool watch = br_ && input_->kind != InputEntry::kSinusoid;
+    double* bad = nullptr;
+    if (watch) want.emplace_back(&bad, 1);
     if (ex_) want.emplace_back(&dPar, std::max(1L, 3L * ext_.sh.H / 2));
     // the discretisation's inputs and work (kernels_disc.cu: the host
     // restatement's operation order, so the same bits as host_math.cpp)
@@ -462,6 +468,11 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         open_image(st, (size_t)(end - reinterpret_cast<char*>(st)));
     }
     dStatus_ = reinterpret_cast<int*>(st);
+    if (watch) {
+        dBad_ = reinterpret_cast<long long*>(bad);
+        const long long none = std::numeric_limits<long long>::max();
+        h2d(dBad_, &none, sizeof none);
+    }
     const double zero_word = 0.0;
     h2d(st, &zero_word, sizeof(double));
     if (blocked) {
@@ -906,10 +917,11 @@ int Plan::fill_inputs(cudaStream_t s)
     if (mu_ <= 0) return 0;
     const long horizon = shards_ > 1 ? (solver_ == kRK4 ? 2 * nScanGlobal_ + 1 : nScanGlobal_ + 4) : nU_;
     if (dUh_) {
-        inputs_->fill_planes(input_, device_, dUh_, dUl_, dU_, mu_, u_base_, u_dt_, nU_, opt_.input_double, s, u_joff_, horizon);
+        inputs_->fill_planes(input_, device_, dUh_, dUl_, dU_, mu_, u_base_, u_dt_, nU_, opt_.input_double, s, u_joff_, horizon,
+                             dBad_);
         return dU_ ? 2 : 1;  // FP64 samples are split into the planes by a second kernel
     }
-    inputs_->fill(input_, device_, dU_, mu_, u_base_, u_dt_, nU_, opt_.input_double, s, u_joff_, horizon);
+    inputs_->fill(input_, device_, dU_, mu_, u_base_, u_dt_, nU_, opt_.input_double, s, u_joff_, horizon, dBad_);
     return 1;
 }
 
@@ -1293,32 +1305,57 @@ int Plan::response_head(cudaStream_t s)
     return launches;
 }
 
-void Plan::response_outputs(double* Y, long c0, long c1, cudaStream_t s)
+int Plan::response_outputs(double* Y, long c0, long c1, cudaStream_t s)
 {
     // the outputs of blocks [c0, c1) with their carried states, written
     // straight into y (rows (j, o) of block b are contiguous there)
     if (ex_) {
         launch_expand_out(ext_, dZ_, Y + (solver_ == kRK4 ? 0L : 3L * p_), c0, c1, nScan_ * (long)p_, sms_, s);
-        return;
-    }
-    if (br_tc_) {
-        state_part(Y, c0, c1, s);  // y = windows + C Phi^j X_b (FP64)
-        return;
+        return 1;
     }
     LevelArgs h = response_out_args(Y);
-    h.src += c0 * h.src_gs;
-    h.src2 += c0 * h.src2_gs;
-    h.dst += c0 * h.dst_gs;
-    h.dst_limit -= c0 * h.dst_gs;
-    h.ncols = c1 - c0;
-    if (!launch_resp_f64(h, sms_, s)) launch_gemm_tiled(h, s);
+    double* y0 = h.dst;
+    if (br_tc_) {
+        state_part(Y, c0, c1, s);  // y = windows + C Phi^j X_b (FP64)
+    } else {
+        h.src += c0 * h.src_gs;
+        h.src2 += c0 * h.src2_gs;
+        h.dst += c0 * h.dst_gs;
+        h.dst_limit -= c0 * h.dst_gs;
+        h.ncols = c1 - c0;
+        if (!launch_resp_f64(h, sms_, s)) launch_gemm_tiled(h, s);
+    }
+    if (!dBad_) return 1;
+    BadSampleArgs b;
+    b.bad = dBad_;
+    b.samples = nU_;
+    b.steps = nScan_;
+    b.solver = solver_;
+    b.NP = Np_;
+    b.n = sys_.n;
+    b.m = mu_;
+    b.p = p_;
+    b.B = shape_.B;
+    b.cols = brKpad_;
+    b.zeroB = sys_.zeroB;
+    b.zeroD = sys_.zeroD;
+    b.U = dU_;
+    b.X = dG_;
+    b.Phi = dPow_;
+    b.Bbar = dBbar_;
+    b.Cext = dCext_;
+    b.D = dD_;
+    b.Y = y0;
+    b.c0 = c0;
+    b.c1 = c1;
+    launch_before_bad_sample(b, s);
+    return 2;
 }
 
 void Plan::execute_response(double* Y, cudaStream_t s)
 {
     int launches = response_head(s);
-    response_outputs(Y, 0, nblocks_, s);
-    ++launches;
+    launches += response_outputs(Y, 0, nblocks_, s);
     if (solver_ == kABM)
         PARODE_CUDA(cudaMemcpyAsync(Y, dYpre_, sizeof(double) * 3 * p_, cudaMemcpyDeviceToDevice, s));
     mark("outputs", s);
@@ -1361,8 +1398,7 @@ void Plan::solve_to_host(double* yd, float* yf)
     long r[5] = {0, 0, 0, 0, total};
     for (int k = 1; k < 4; ++k) r[k] = std::min(total, base + cut[k] * gs);
     for (int k = 0; k < 4; ++k) {
-        response_outputs(dY_, cut[k], cut[k + 1], s);
-        ++launches;
+        launches += response_outputs(dY_, cut[k], cut[k + 1], s);
         if (k == 0 && solver_ == kABM)
             PARODE_CUDA(cudaMemcpyAsync(dY_, dYpre_, sizeof(double) * 3 * p_, cudaMemcpyDeviceToDevice, s));
         if (dF) {

@@ -151,7 +151,7 @@ private:
     LevelArgs response_agg_args() const;
     LevelArgs response_out_args(double* Y) const;
     int response_head(cudaStream_t s);  // inputs, aggregates, carry; returns the launches
-    void response_outputs(double* Y, long c0, long c1, cudaStream_t s);  // blocks [c0, c1)
+    int response_outputs(double* Y, long c0, long c1, cudaStream_t s);  // blocks [c0, c1); returns the launches
     void state_part(double* Y, long c0, long c1, cudaStream_t s);
     void check_status();  // after a synchronise: throws when a device-side wait gave up
     void setup_shard(const PlanOptions& opt);
@@ -184,6 +184,7 @@ private:
     int precision_used_ = 0;
     bool br_ = false;           // leaf = block response GEMM (kernels_br.cu)
     int brK_ = 0, brKpad_ = 0;  // window columns (padded to even)
+    long long* dBad_ = nullptr;  // user functions: the first sample that is not finite
     double* dW_ = nullptr;      // response matrix, (B p + NP) x (brKpad_ + NP)
     // block states by radix expansion (kernels_expand.cu): no inputs, or
     // sinusoid inputs in the mixed and TF32 forms
