@@ -79,18 +79,13 @@ __device__ __forceinline__ double sinusoid_value(const double* a, const double* 
     return v;
 }
 
-// Where a sampler puts sample j of its run: FP64 at out[(j - skip) * stride], or
+// Where a sampler puts sample j of its run: FP64 at out[j * stride], or
 // split into two TF32 planes (hi = TF32(x), lo = TF32(x - hi) with
-// x = float(v), both rounded to nearest) for the tensor-core GEMMs.  The
-// first `skip` samples of a run lie before the buffer.
+// x = float(v), both rounded to nearest) for the tensor-core GEMMs.
 struct SampleOut64 {
     double* out;
     long stride;
-    int skip = 0;
-    __device__ __forceinline__ void operator()(long j, double v) const
-    {
-        if (j >= skip) out[(j - skip) * stride] = v;
-    }
+    __device__ __forceinline__ void operator()(long j, double v) const { out[j * stride] = v; }
 };
 
 // x rounded to TF32 (10 mantissa bits), to nearest with ties away from zero:
@@ -106,15 +101,23 @@ struct SampleOutSplit {
     float* hi;
     float* lo;
     long stride;
-    int skip = 0;
     __device__ __forceinline__ void operator()(long j, double v) const
     {
         const float x = (float)v;
         const float h = tf32_rna(x);
-        if (j < skip) return;
-        j -= skip;
         hi[j * stride] = h;
         if (lo) lo[j * stride] = tf32_rna(x - h);  // no lo plane in the single-pass form
+    }
+};
+
+// The same for a run whose first `skip` samples lie before the buffer.
+template <class Out>
+struct SampleOutFrom {
+    Out out;
+    int skip;
+    __device__ __forceinline__ void operator()(long j, double v) const
+    {
+        if (j >= skip) out(j - skip, v);
     }
 };
 

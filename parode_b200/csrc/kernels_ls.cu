@@ -13,6 +13,7 @@
 #include "common.h"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace parode {
 
@@ -444,51 +445,58 @@ __global__ void k_swap_grouped(const LevelArgs* __restrict__ args)
     swap_body(a);
 }
 
-// Run r of a buffer of `count` samples whose first has index joff on the whole
-// horizon.  Runs start at multiples of their length on the horizon, so a time
-// shard's samples are those of the whole solve bit for bit; its first run may
-// start before its buffer.
+// Run r of a buffer of `count` samples.  Runs start at multiples of their length
+// on the horizon, so a time shard's samples are those of the whole solve bit
+// for bit; its first run may start `off` samples before its buffer (kPart; a
+// whole solve's writes then need no test: 0.6 us of 18 for 4096 steps of 8 states).
 struct SampleRun {
     long j0;   // first sample, relative to the buffer
     int skip;  // of the run's first samples that lie before the buffer
-    int n;     // samples, 0 past the last run
+    int n;     // samples
 };
-__host__ __device__ inline long sample_runs(long count, long joff, int run) { return (joff % run + count + run - 1) / run; }
-__device__ __forceinline__ SampleRun sample_run_of(long r, long count, long joff, int run)
+template <bool kPart>
+__device__ __forceinline__ SampleRun sample_run_of(long r, long count, int off, int run)
 {
     SampleRun s;
-    s.j0 = r * run - joff % run;
-    s.skip = s.j0 < 0 ? (int)-s.j0 : 0;
-    s.n = (int)max(0L, min((long)run, count - s.j0));
+    s.j0 = r * run - (kPart ? off : 0);
+    s.skip = kPart && s.j0 < 0 ? (int)-s.j0 : 0;
+    s.n = (int)min((long)run, count - s.j0);
     return s;
 }
 
 // One thread per (run of `run` samples, channel); channels fastest.
-template <int KMAX>
+template <int KMAX, bool kPart>
 __global__ void k_sinusoid_samples(double* U, int m, int K, const double* a, const double* f, const double* phi,
-                                   double base, double dt, long count, long joff, int run)
+                                   double base, double dt, long count, long joff, int off, int run)
 {
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const SampleRun s = sample_run_of(e / m, count, joff, run);
-    if (s.n <= 0) return;
-    const int i = (int)(e % m);
-    const long at = (s.j0 + s.skip) * m + i;  // of the run's first sample in the buffer
-    sinusoid_run<KMAX>(a, f, phi, K, i, base, dt, s.j0, s.n, SampleOut64{U + at, m, s.skip}, joff);
+    const long runs = ((kPart ? off : 0) + count + run - 1) / run;
+    if (e >= runs * m) return;
+    const long r = e / m;
+    const int i = (int)(e - r * m);
+    const SampleRun s = sample_run_of<kPart>(r, count, off, run);
+    const SampleOut64 out{U + (s.j0 + s.skip) * m + i, m};
+    if constexpr (kPart) sinusoid_run<KMAX>(a, f, phi, K, i, base, dt, s.j0, s.n, SampleOutFrom<SampleOut64>{out, s.skip}, joff);
+    else sinusoid_run<KMAX>(a, f, phi, K, i, base, dt, s.j0, s.n, out, joff);
 }
 
 // The same samples as TF32 hi / lo planes (the tensor-core GEMMs' operands),
 // by the plain rotation (sinusoid_rot: the planes' own rounding is 2^-22).
-template <int KMAX>
+template <int KMAX, bool kPart>
 __global__ void k_sinusoid_planes(float* hi, float* lo, int m, int K, const double* a, const double* f,
-                                  const double* phi, double base, double dt, long count, long joff, int run)
+                                  const double* phi, double base, double dt, long count, long joff, int off, int run)
 {
     grid_dep_trigger();  // the response GEMMs may set up meanwhile (they wait for these samples)
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const SampleRun s = sample_run_of(e / m, count, joff, run);
-    if (s.n <= 0) return;
-    const int i = (int)(e % m);
-    const long at = (s.j0 + s.skip) * m + i;  // of the run's first sample in the buffer
-    sinusoid_rot<KMAX>(a, f, phi, K, i, base, dt, s.j0, s.n, SampleOutSplit{hi + at, lo ? lo + at : nullptr, m, s.skip}, joff);
+    const long runs = ((kPart ? off : 0) + count + run - 1) / run;
+    if (e >= runs * m) return;
+    const long r = e / m;
+    const int i = (int)(e - r * m);
+    const SampleRun s = sample_run_of<kPart>(r, count, off, run);
+    const long at = (s.j0 + s.skip) * m + i;
+    const SampleOutSplit out{hi + at, lo ? lo + at : nullptr, m};
+    if constexpr (kPart) sinusoid_rot<KMAX>(a, f, phi, K, i, base, dt, s.j0, s.n, SampleOutFrom<SampleOutSplit>{out, s.skip}, joff);
+    else sinusoid_rot<KMAX>(a, f, phi, K, i, base, dt, s.j0, s.n, out, joff);
 }
 
 // FP64 samples (any input function) into TF32 hi / lo planes.
@@ -757,19 +765,33 @@ void launch_affine_level(const LevelArgs& a, cudaStream_t s)
     }
 }
 
+namespace {
+
+// The instance for K terms a channel and a whole or partial horizon.
+template <class F>
+void by_terms(int K, bool part, F&& f)
+{
+    auto go = [&](auto kmax) { part ? f(kmax, std::true_type()) : f(kmax, std::false_type()); };
+    switch (sample_kmax(K)) {
+    case 1: return go(std::integral_constant<int, 1>());
+    case 2: return go(std::integral_constant<int, 2>());
+    case 3: return go(std::integral_constant<int, 3>());
+    default: return go(std::integral_constant<int, 4>());
+    }
+}
+
+}  // namespace
+
 void launch_sinusoid_samples(double* U, int m, int K, const double* a, const double* f, const double* phi,
                              double base, double dt, long count, cudaStream_t s, long joff, long horizon)
 {
     if (count <= 0 || m <= 0) return;
-    const int run = sample_run(std::max(count, horizon) * m);
-    const long total = sample_runs(count, joff, run) * m;
-    const unsigned g = (unsigned)blocks_for(total, 256);
-    switch (sample_kmax(K)) {
-    case 1: k_sinusoid_samples<1><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff, run); break;
-    case 2: k_sinusoid_samples<2><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff, run); break;
-    case 3: k_sinusoid_samples<3><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff, run); break;
-    default: k_sinusoid_samples<4><<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff, run); break;
-    }
+    const int run = sample_run(std::max(count, horizon) * m), off = (int)(joff % run);
+    const unsigned g = (unsigned)blocks_for((off + count + run - 1) / run * m, 256);
+    by_terms(K, off > 0, [&](auto kmax, auto part) {
+        k_sinusoid_samples<decltype(kmax)::value, decltype(part)::value>
+            <<<g, 256, 0, s>>>(U, m, K, a, f, phi, base, dt, count, joff, off, run);
+    });
     PARODE_CUDA(cudaGetLastError());
 }
 
@@ -777,15 +799,12 @@ void launch_sinusoid_planes(float* hi, float* lo, int m, int K, const double* a,
                             double base, double dt, long count, cudaStream_t s, long joff, long horizon)
 {
     if (count <= 0 || m <= 0) return;
-    const int run = sample_run(std::max(count, horizon) * m);
-    const long total = sample_runs(count, joff, run) * m;
-    const unsigned g = (unsigned)blocks_for(total, 256);
-    switch (sample_kmax(K)) {
-    case 1: k_sinusoid_planes<1><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff, run); break;
-    case 2: k_sinusoid_planes<2><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff, run); break;
-    case 3: k_sinusoid_planes<3><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff, run); break;
-    default: k_sinusoid_planes<4><<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff, run); break;
-    }
+    const int run = sample_run(std::max(count, horizon) * m), off = (int)(joff % run);
+    const unsigned g = (unsigned)blocks_for((off + count + run - 1) / run * m, 256);
+    by_terms(K, off > 0, [&](auto kmax, auto part) {
+        k_sinusoid_planes<decltype(kmax)::value, decltype(part)::value>
+            <<<g, 256, 0, s>>>(hi, lo, m, K, a, f, phi, base, dt, count, joff, off, run);
+    });
     PARODE_CUDA(cudaGetLastError());
 }
 
