@@ -175,7 +175,7 @@ private:
     void build_responses();
 
     int device_ = 0;
-    int sms_ = 148;
+    int sms_ = (int)kSmCount;
     int* dStatus_ = nullptr;  // set by a device wait that gave up
     cudaStream_t last_stream_ = nullptr;
     // the launch list as a CUDA graph (execute): 0 no execute yet, 1 one eager

@@ -10,6 +10,10 @@
 
 namespace parode {
 
+// SMs of the B200 that the rules of size are set for (plans ask the device
+// where a launch's own grid depends on it).
+constexpr long kSmCount = 148;
+
 // Error codes: ParODEEnums.h (-1..-7) and parode_ext.h (-8..-10).
 enum Err : int {
     kOK = 0,

@@ -16,13 +16,13 @@ namespace parode {
 
 namespace {
 
-// Maps per chunk: 16, up to 64 at the lowest level while that still leaves a
-// chunk for each of 16 warps per SM (a chunk's maps are composed one after
-// another, so short chunks cost upper-level work and long ones parallelism).
+// Maps per chunk of a level: 16, up to 64 while that still leaves 24 chunks per
+// SM (a chunk's maps are composed one after another, so short chunks cost
+// upper-level work and long ones parallelism).
 int chunk_length(long count)
 {
     int L = 16;
-    while (L < 64 && count / (2 * L) >= 148L * 24) L *= 2;
+    while (L < 64 && count / (2 * L) >= kSmCount * 24) L *= 2;
     return L;
 }
 

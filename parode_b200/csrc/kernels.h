@@ -5,17 +5,21 @@
 
 #include <vector>
 
+#include "common.h"
+
 namespace parode {
 
 // Samples per thread of the input-sampling kernels (one thread advances one
 // channel over a run of consecutive samples), for `total` samples in all
 // channels: 64, which spreads the two sincos that start each term of a run
 // over many rotations, down to 8 where longer runs would leave the chip to a
-// few serial chains (16,386 samples: 16 us by runs of 64).
+// few serial chains (16,386 samples: 16 us by runs of 64).  A time shard counts
+// the whole horizon's samples; a batch counts its systems' together, so one
+// system's samples agree to rounding, not bit for bit, between batches.
 inline int sample_run(long total)
 {
     int run = 64;
-    while (run > 8 && total / run < 148L * 1024) run /= 2;
+    while (run > 8 && total / run < kSmCount * 1024) run /= 2;
     return run;
 }
 

@@ -839,7 +839,7 @@ static void fixup_t(const BlockedShape& sh, double* Y, long ybase, long nScan, i
     const long rgs = ((sh.B * p + 7) / 8 + 7) / 8;
     const long nblocks = (nScan + sh.B - 1) / sh.B;
     const long items = rgs * ((nblocks + 7) / 8);
-    const unsigned grid = (unsigned)std::max<long>(1, std::min<long>((items + 7) / 8, 148L * 8));
+    const unsigned grid = (unsigned)std::max<long>(1, std::min<long>((items + 7) / 8, kSmCount * 8));
     k_fixup<NP><<<grid, kThreads, 0, s>>>(Y, ybase, nScan, p, CP, X, sh.B);
     PARODE_CUDA(cudaGetLastError());
 }

@@ -23,7 +23,8 @@
 // (k_chunk_mid), and level 0 at NP > 32, whose tiles do fill it, takes the form
 // with the fewest products (k_chain_up, k_chain_down).  The form depends on the
 // level's global index only (k_chunk_mid takes the steps of the launches it
-// stands for), so a time-partitioned solve computes the same bits as the whole.
+// stands for), so a time-partitioned solve computes the same bits as the whole
+// one on the sample windows (the samplers' runs follow the whole horizon too).
 //
 // The whole scan, against chunks stepped through one item of prefetch ahead with
 // depth-4 trees above level 0 and a launch per level and direction: NP = 64,
@@ -504,7 +505,7 @@ template <int NP>
 unsigned chunk_grid(long count)
 {
     constexpr int kPerSm = NP > 32 ? 1 : NP > 16 ? 4 : 8;
-    return (unsigned)std::min<long>((count + kTile - 1) / kTile, 148 * kPerSm);
+    return (unsigned)std::min<long>((count + kTile - 1) / kTile, kSmCount * kPerSm);
 }
 
 // Level 0 of a scan (h: the level's global index) steps through whole chunks.

@@ -343,9 +343,9 @@ __global__ void __launch_bounds__(kThreads) k_expand_level(const double* __restr
 // tasks: the blocks' Z as A fragments in registers, then per 8 rows KS x CT
 // m8n8k4 products and direct stores (a block's 8 rows are 64 consecutive
 // bytes, two per lane).  FP64-tensor bound: RK4 n = 64, m = p = 8, 2^20 steps
-// is 1.88 GFLOP against 67 MB written, 51 us of DMMA; 72 us, the pipe 82 % busy
+// is 1.88 GFLOP against 67 MB written, 51 us of DMMA; 64 us, the pipe 89 % busy
 // while the CTAs run (85 us, 68 %, with 8-byte fragment loads from pitches of
-// 4 mod 16 doubles).  Small tasks (parts > 1) even out the warps of the four
+// 4 mod 16 doubles).  Row tiles in equal parts even out the warps of the four
 // sub-partitions.
 template <int KS>
 struct OutCfg {
@@ -624,7 +624,7 @@ void level_t(const ExpandTables& t, const double* T, double* Z, int imax, long d
     // columns per CTA: one 8-column tile while that leaves CTAs for the whole
     // chip, up to four beyond (the table fragments are loaded once)
     const long tiles = (d + 7) / 8;
-    const int ct = (int)std::max<long>(1, std::min<long>(kLevelTiles, tiles * imax / 148));
+    const int ct = (int)std::max<long>(1, std::min<long>(kLevelTiles, tiles * imax / kSmCount));
     dim3 grid((unsigned)((tiles + ct - 1) / ct), (unsigned)imax);
     launch_dependent(k_expand_level<KS>, grid, dim3(kThreads), 0, s, T, Z, d, t.sh.nblocks, t.sh.NP, ct);
 }

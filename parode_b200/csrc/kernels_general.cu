@@ -43,7 +43,7 @@ namespace {
 // NP = 8 or 16: a warp alone per chunk, M_k's fragments straight from global
 // memory, kAhead steps in flight (more where the chunks are few and a step's
 // load latency is what counts: kDeep chunks and fewer).
-constexpr long kDeep = 148 * 4;
+constexpr long kDeep = kSmCount * 4;
 
 template <int NP, bool kFull, int kAhead>
 __global__ void __launch_bounds__(128) k_scan_up_warp(const double* M, const double* V, int ns, long count, int L,

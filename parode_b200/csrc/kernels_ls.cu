@@ -820,14 +820,14 @@ __global__ void k_to_float(const double* __restrict__ src, float* __restrict__ d
 void launch_to_float(const double* src, float* dst, long n, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_to_float<<<(unsigned)std::min<long>((n / 2 + 255) / 256 + 1, 148L * 16), 256, 0, s>>>(src, dst, n);
+    k_to_float<<<(unsigned)std::min<long>((n / 2 + 255) / 256 + 1, kSmCount * 16), 256, 0, s>>>(src, dst, n);
     PARODE_CUDA(cudaGetLastError());
 }
 
 void launch_split_planes(const double* U, float* hi, float* lo, long n, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_split_planes<<<(unsigned)std::min<long>((n + 255) / 256, 148L * 16), 256, 0, s>>>(U, hi, lo, n);
+    k_split_planes<<<(unsigned)std::min<long>((n + 255) / 256, kSmCount * 16), 256, 0, s>>>(U, hi, lo, n);
     PARODE_CUDA(cudaGetLastError());
 }
 

@@ -10,7 +10,7 @@
 // without that).  Row (j, o) of W_out is zero past the samples that step j
 // reads, so a row tile skips the columns past its last row's limit (on average
 // half the window).  FP64-tensor bound: the outputs of RK4 n = 64, m = p = 8,
-// 2^20 steps are 3.6 GFLOP (97 us) in 0.132 ms; 0.203 ms as 64 x 64 tiles over
+// 2^20 steps are 3.6 GFLOP (97 us) in 0.132 ms, the pipe 79 % busy; 0.203 ms as 64 x 64 tiles over
 // the whole of W (5.5 GFLOP), 0.155 as tiles that skip.  The aggregates have no
 // zeros and stay with the tiles (82 us against 94).
 #include "common.h"

@@ -255,12 +255,17 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         gen_ = false;
         stage_bytes_ = blocked_leaf_stage_bytes(shape_, sys.n, mu_, p_, solver);
         // sampled inputs: the leaf as GEMMs with the block response matrix
-        // (kernels_br.cu), unless the in-block sweeps are forced.  Blocks of 16
-        // steps are at or near the best length of every scan dimension measured
-        // (8 states, 4096 steps FP64: 43 us with 16, 47 with 32, 86 with the
-        // sweeps; 32 states, 3e5 steps mixed, user input: 84 us with 16, 96 with
-        // 64, 340 with the sweeps); 8 steps where a short horizon leaves few
-        // blocks of a 64-state RK4 system (20,000 steps FP64: 76 against 88 us).
+        // (kernels_br.cu), unless the in-block sweeps are forced or W does not fit.
+        // Blocks of 16 steps, 8 for RK4 of 33 to 64 states below 2^15 steps.  FP64,
+        // us with blocks of 4, 8, 16, 32 and 64 steps (m = p inputs and outputs):
+        //   RK4  8 states, m = 2,   4,000 steps: 20 22 21 24 34    m = 8: 23 28 37 33 47
+        //   RK4 24 states, m = 2, 250,000 steps: 62 51 45 48 48    m = 8: 88 83 86 104 143
+        //   RK4 64 states, m = 2,  20,000 steps: 51 43 45 51 62    m = 8: 56 53 62 59 75
+        //   RK4 64 states, m = 2, 250,000 steps: 111 88 72 72 68   m = 8: 145 129 122 138 168
+        //   ABM 16 states, m = 2, 250,000 steps: 107 82 68 64 59   m = 8: 135 116 103 109 117
+        // 16 is at or near the best of long horizons and few inputs; with 8 inputs
+        // and below 2^15 steps 4 or 8 steps are better at every dimension (RK4 8
+        // states, 4,000 steps: 23 against 37), which only the 64-row form takes.
         // The mixed form runs the aggregate and output-window products on the
         // tensor cores (3xTF32) and keeps the initial-state part of the outputs
         // in FP64; at scan dimensions up to 8 it stays in FP64, as ever.

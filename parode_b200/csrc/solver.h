@@ -178,7 +178,7 @@ private:
     BlockedShape shape_;
     long ntiles_ = 0, nblocks_ = 0;
     bool gen_ = false;
-    int sms_ = 148;
+    int sms_ = (int)kSmCount;
     double *dG_ = nullptr, *dWork_ = nullptr, *dCP_ = nullptr, *dCext_ = nullptr;
     size_t stage_bytes_ = 0;
     int precision_used_ = 0;
