@@ -29,14 +29,14 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-METRIC = "state*steps/s (RK4 n=64 T=2^20 solve, mixed 3xTF32 form, rel err <= 1e-6 vs FP64)"
+METRIC = "state*steps/s (RK4 n=64 T=2^20 solve, mixed form, rel err <= 1e-6 vs FP64)"
 UNIT = "state*steps/s"
 WORKLOAD = "cfg2: RK4 n=64 m=8 p=8 h=1e-4 T=2^20, seeded system + sum-of-sinusoids input"
-# DRAM bytes (read + write) of one launch of the dominant kernel at T = 2^20
-# (key: (T, mixed)), from the ncu captures summarised under profiles/.
 # serving: the p99 latency the serving loop is specified to hold (cfg5 requests)
 SERVE_P99_TARGET_MS = 20.0
-DOMINANT_TRAFFIC = {(1 << 20, False): 168.18e6 + 45.27e6, (1 << 20, True): 134.87e6 + 60.82e6}
+# DRAM bytes (read + write) of one launch of the dominant kernel at T = 2^20, from
+# the ncu captures summarised under profiles/.
+DOMINANT_TRAFFIC = {"k_resp_f64": 219.98e6 + 40.49e6, "k_resp_tc": 134.87e6 + 60.82e6, "k_expand_out": 15.49e6 + 10.58e6}
 
 
 def parse():
@@ -252,9 +252,10 @@ def gemm_peak_tflops(torch, dev, dtype, tf32=False):
 def response_flops(case, shape, mixed, phases=False):
     """Algorithmic FLOPs of one solve on the block-response path, per launch
     kind.  shape = (B, K, NP, blocks) from the plan.  The aggregate GEMM
-    costs 2 NP K per block; the output GEMM 2 B p (K + NP) per block (window
-    part 2 B p K, initial-state part 2 B p NP); the carry over blocks 4 NP^2
-    per block (up- and down-sweep).  The dominant launch is the output GEMM
+    costs 2 NP K per block; the output GEMM the window columns that each of a
+    block's steps reads (RK4 (2 j + 1) m, ABM (j + 4) m at step j; the rest of W
+    is zero) and 2 B p NP for the initial-state part; the carry over blocks
+    4 NP^2 per block (up- and down-sweep).  The dominant launch is the output GEMM
     in FP64 and, in the mixed form with sampled inputs, the tensor-core launch
     that computes the aggregates and the output windows together.  With phases
     (the mixed form of sinusoid inputs: K phase columns, kernels_expand.cu) the
@@ -265,7 +266,8 @@ def response_flops(case, shape, mixed, phases=False):
     if phases:
         out, states = 2.0 * B * p * (NP + K) * blocks, 2.0 * NP * (NP + K) * blocks
         return {"dominant": out, "solve": out + states}
-    agg, win, state, carry = 2.0 * NP * K * blocks, 2.0 * B * p * K * blocks, 2.0 * B * p * NP * blocks, \
+    cols = sum(min(K, ((2 * j + 1) if case.solver == 0 else (j + 4)) * case.m) for j in range(B))
+    agg, win, state, carry = 2.0 * NP * K * blocks, 2.0 * p * cols * blocks, 2.0 * B * p * NP * blocks, \
         4.0 * NP * NP * blocks
     dominant = (agg + win) if mixed else (win + state)
     return {"dominant": dominant, "solve": agg + win + state + carry}
@@ -470,9 +472,7 @@ def measure_cfg3(pb, wl, torch, reps=3):
             ts.append(s.elapsed_time(e))
         ms = statistics.median(ts)
         ys[name] = b.output(0)[1]
-        flops = 4.0 * c.scan_dim ** 2 * c.T
-        out[name] = {"ms": ms, "value": b.state_steps / (ms / 1e3), "unit": UNIT,
-                     "sweep_tflops": flops / (ms / 1e3) / 1e12, "launches": b.launch_count}
+        out[name] = {"ms": ms, "value": b.state_steps / (ms / 1e3), "unit": UNIT, "launches": b.launch_count}
         b.close()
     out["mixed_over_fp64"] = out["fp64"]["ms"] / out["mixed"]["ms"]
     out["rel_err_mixed_vs_fp64"] = rel_err(ys["mixed"], ys["fp64"])
@@ -812,11 +812,12 @@ def run_ours(args):
         roofline = {"bound": "tensor",
                     "kernel": ("k_resp_tc: 3xTF32 tcgen05 GEMMs of the block aggregates and output windows"
                                if on_tc else "k_expand_out: FP64 DMMA outputs y = W [X_b; phases of b]" if phases
-                               else "k_level_tiled: FP64 DMMA output GEMM y = W [window; X_b]"),
+                               else "k_resp_f64: FP64 DMMA outputs y = W [window; X_b]"),
                     "stage": stage, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                     "frac": (achieved / peak) if achieved else None, "peak_source": peak_src,
                     "algorithmic_flops_per_launch": fl["dominant"] if fl else None,
-                    "traffic": None if phases else DOMINANT_TRAFFIC.get((case.T, used_mixed)),
+                    "traffic": None if case.T != 1 << 20 else
+                    DOMINANT_TRAFFIC["k_resp_tc" if on_tc else "k_expand_out" if phases else "k_resp_f64"],
                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch (profiles/)",
                     "stages_ms": main["stages_ms"],
                     "whole_solve_tflops": fl["solve"] / (main["ms_per_step"] / 1e3) / 1e12 if fl else None}
