@@ -224,9 +224,14 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         if (opt.path != kPathLevel && can_block) path_ = kPathBlocked;
     }
     if (path_ == kPathBlocked && !choose_expand(opt)) {
-        // sampled inputs: the response leaf where its tables fit, else the sweeps or the levels
+        // sampled inputs: the response leaf where its tables fit, else the sweeps or the levels.
+        // Without B a sample enters its own step's output only, but the leaf's
+        // products would carry one that is not finite into its block's other
+        // outputs and, by the aggregates, into every later state: user functions
+        // (time shards apart, which have no other leaf) then take the sweeps.
+        const bool own_step = sys.zeroB && mu_ > 0 && input_->kind != InputEntry::kSinusoid && opt.shards <= 1 && opt.shard == 0;
         br_ = mu_ > 0 && opt.path != kPathBlockedSweep &&
-              (opt.path == kPathBlockedResponse || block_response_fits(shape_.NP, solver, mu_, p_));
+              (opt.path == kPathBlockedResponse || (!own_step && block_response_fits(shape_.NP, solver, mu_, p_)));
         if (!br_ && !blocked_shape(Ns_, mu_, solver, &shape_)) {
             if (opt.path != kPathAuto) throw Error(kInvalidArgument, "the blocked path: too many inputs for its tiles");
             path_ = kPathLevel;

@@ -54,3 +54,19 @@ def test_ranges_of_a_one_shot_solve(pb):
     for k in (3, 16 * 1015 + 1, 16 * 1016, 100_001):
         t, y = pb.simulate(c.A, c.B, c.C, c.D, c.x0, pb.register_input(GOOD % (KINDS["nan"] % (k * H - 1e-4))), c.t0, c.t_end, c.h)
         assert np.all(np.isfinite(y[:k])) and not np.all(np.isfinite(y[k]))
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+@pytest.mark.parametrize("solver,n,m,p,precision", CASES[:3] + CASES[5:9] + CASES[10:11])
+def test_without_B_only_its_own_step(pb, solver, n, m, p, precision, kind):
+    """Without B a sample enters the output of its own step alone."""
+    T, k = 700, 337
+    c = wl.small(77200 + n, solver, n, m, p, T, h=H)
+    ref = oracle.simulate_affine(oracle.System(c.A, None, c.C, c.D, c.x0), oracle.Input.callable(lambda t, i: np.sin(3.0 * t + i)),
+                                 solver, c.t0, c.t_end, c.h)
+    c.B = None
+    y = _solve(pb, c, GOOD % (KINDS[kind] % (k * H if kind == "one" else k * H - 1e-4)), precision, T)
+    good = np.arange(T) != k if kind == "one" else np.arange(T) < k
+    d = np.max(np.abs(y[good] - ref[good])) / np.max(np.abs(ref))
+    assert d <= (1e-12 if precision == 0 else 1e-6), d
+    assert not np.any(np.isfinite(y[~good]))
