@@ -260,7 +260,7 @@ void Plan::build(int device, const SystemDesc& sys, InputRegistry* inputs, int u
         gen_ = false;
         stage_bytes_ = blocked_leaf_stage_bytes(shape_, sys.n, mu_, p_, solver);
         // sampled inputs: the leaf as GEMMs with the block response matrix
-        // (kernels_br.cu), unless the in-block sweeps are forced or W does not fit.
+        // (kernels_br.cu), unless one of the rules above leaves them to the sweeps.
         // Blocks of 16 steps, 8 for RK4 of 33 to 64 states below 2^15 steps.  FP64,
         // us with blocks of 4, 8, 16, 32 and 64 steps (m = p inputs and outputs):
         //   RK4  8 states, m = 2,   4,000 steps: 20 22 21 24 34    m = 8: 23 28 37 33 47
